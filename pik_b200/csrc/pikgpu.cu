@@ -403,6 +403,7 @@ int UploadTables(pikgpu_ctx* ctx) {
   DevTables t;
   BuildTables(&t);
   CUDA_TRY(ctx, cudaMemcpyToSymbol(c_t, &t, sizeof(t)));
+  CUDA_TRY(ctx, cudaMemcpyToSymbol(g_t, &t, sizeof(t)));
   CUDA_TRY(ctx, cudaFuncSetAttribute(
                     k_epf_box<false, 32>,
                     cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -6,12 +6,17 @@
 // XYB -> linear RGB / sRGB-8. Each kernel names the reference function it
 // implements (paths relative to the google/pik checkout).
 
+#include <type_traits>
+
 #include "kernels.cuh"
 
 
 namespace pikgpu {
 
 __constant__ DevTables c_t;
+// The same tables in global memory, for reads whose index differs between
+// the lanes of a warp (the constant port serves one address at a time).
+__device__ DevTables g_t;
 
 namespace {
 
@@ -169,50 +174,7 @@ __device__ void ReinterpIdct(const float* in, int is, float* out, int os) {
   }
 }
 
-// AcStrategy LLF/LF helpers (pik/ac_strategy.cc:850-1056).
-__device__ void LowestFreqFromDC(int type, const float* dc, int ds, float* llf,
-                                 int ls) {
-  if (type == kDCT16X16) {
-    float t[4];
-    ReinterpDct<16, 2>(dc, ds, t, 2);
-    for (int y = 0; y < 2; ++y)
-      for (int x = 0; x < 2; ++x) llf[y * ls + x] = t[y * 2 + x];
-  } else if (type == kDCT32X32) {
-    float t[16];
-    ReinterpDct<32, 4>(dc, ds, t, 4);
-    for (int y = 0; y < 4; ++y)
-      for (int x = 0; x < 4; ++x) llf[y * ls + x] = t[y * 4 + x];
-  } else {
-    llf[0] = dc[0];
-  }
-}
-
-__device__ void DC2x2FromLowestFreq(int type, const float* llf, int ls,
-                                    float* d, int dstr) {
-  if (type == kDCT || type == kDCT_NOHF || type == kLINES) {
-    ReinterpIdct<8, 1, 2>(llf, 0, d, dstr);
-  } else if (type == kDCT16X16) {
-    float dest[16];
-    for (int i = 0; i < 16; ++i) dest[i] = 0.f;
-    dest[0] = llf[0];
-    dest[1] = llf[1];
-    dest[4] = llf[ls];
-    dest[5] = llf[ls + 1];
-    ReinterpIdct<16, 2, 4>(dest, 4, d, dstr);
-  } else if (type == kDCT32X32) {
-    float dest[64];
-    for (int i = 0; i < 64; ++i) dest[i] = 0.f;
-    for (int iy = 0; iy < 4; ++iy)
-      for (int ix = 0; ix < 4; ++ix) dest[iy * 8 + ix] = llf[iy * ls + ix];
-    ReinterpIdct<32, 4, 8>(dest, 8, d, dstr);
-  } else {
-    d[0] = llf[0];
-    d[1] = llf[0];
-    d[dstr] = llf[0];
-    d[dstr + 1] = llf[0];
-  }
-}
-
+// DC2x2FromLowFrequencies (pik/ac_strategy.cc:850-1056) by one thread.
 // `blk(i)` reads element i of the block's coefficient matrix.
 template <class Blk>
 __device__ void DC2x2FromLowFreq(int type, const Blk& blk, float* d,
@@ -236,33 +198,6 @@ __device__ void DC2x2FromLowFreq(int type, const Blk& blk, float* d,
     d[1] = b00 + b01 - b10 - b11;
     d[dstr] = b00 - b01 + b10 - b11;
     d[dstr + 1] = b00 - b01 - b10 + b11;
-  }
-}
-
-__device__ void LowFreqFromDC2x2(int type, float* d, int dstr) {
-  if (type == kDCT || type == kDCT_NOHF || type == kLINES) {
-    float out[4];
-    ReinterpDct<8, 2>(d, dstr, out, 2);
-    d[0] = out[0];
-    d[1] = out[1];
-    d[dstr] = out[2];
-    d[dstr + 1] = out[3];
-  } else if (type == kDCT16X16) {
-    float out[16];
-    ReinterpDct<16, 4>(d, dstr, out, 4);
-    for (int y = 0; y < 4; ++y)
-      for (int x = 0; x < 4; ++x) d[dstr * y + x] = out[y * 4 + x];
-  } else if (type == kDCT32X32) {
-    float out[64];
-    ReinterpDct<32, 8>(d, dstr, out, 8);
-    for (int y = 0; y < 8; ++y)
-      for (int x = 0; x < 8; ++x) d[dstr * y + x] = out[y * 8 + x];
-  } else {
-    const float b00 = d[0], b01 = d[1], b10 = d[dstr], b11 = d[dstr + 1];
-    d[0] = (b00 + b01 + b10 + b11) * 0.25f;
-    d[1] = (b00 + b01 - b10 - b11) * 0.25f;
-    d[dstr] = (b00 - b01 + b10 - b11) * 0.25f;
-    d[dstr + 1] = (b00 - b01 - b10 + b11) * 0.25f;
   }
 }
 
@@ -630,7 +565,7 @@ __global__ void __launch_bounds__(256) k_dequant_ac(Geo g, DevFrame f,
 // 2 (gxs + 2) x 2 (gys + 2), mirrored at its edges by the blur.
 //
 // A CTA (k_lf_tile) takes one channel of a tile of kLfTile x kLfTile cells
-// of a group and keeps the images it needs in shared memory: the LLF and
+// of a group and keeps the images it needs in shared memory: the DC, LLF and
 // 2x2 images of every block that reaches the tile's blurred range (one
 // cell beyond the tile, and the ring where the tile touches it), so its
 // first cell may lie up to 3 cells before that range (DCT32X32).
@@ -645,23 +580,27 @@ struct LfGroup {
 constexpr int kLfTile = 16;           // cells per tile side
 constexpr int kLfWin = kLfTile + 12;  // shared-memory window, cells
 constexpr int kLfWin2 = 2 * kLfWin;   // the 2x2 images' window, pixels
-constexpr int kLfThreads = 128;
-// Shared memory of k_lf_tile: the LLF image, the 2x2 image before and after
-// LFPredictionBlur, over the window, and the list of the window's first
-// cells (by block size: 8x8-class blocks, then 16x16, then 32x32).
+constexpr int kLfThreads = 256;
+// Shared memory of k_lf_tile: the DC and LLF images, the 2x2 image before
+// and after LFPredictionBlur, over the window, and the list of the window's
+// first cells (by block size: 8x8-class blocks, then 16x16, then 32x32).
 constexpr int kLfList1 = kLfWin * kLfWin;
 constexpr int kLfList2 = (kLfWin / 2 + 1) * (kLfWin / 2 + 1);
 constexpr int kLfList4 = (kLfWin / 4 + 1) * (kLfWin / 4 + 1);
 constexpr size_t kLfSmemBytes =
-    4 * (size_t(kLfWin) * kLfWin + 2 * size_t(kLfWin2) * kLfWin2 + kLfList1 +
-         kLfList2 + kLfList4);
+    4 * (2 * size_t(kLfWin) * kLfWin + 2 * size_t(kLfWin2) * kLfWin2 +
+         kLfList1 + kLfList2 + kLfList4);
 
 // The window of a tile: cell (X, Y) of the group is at (X - ex, Y - ey).
 struct LfWin {
   int ex, ey;
+  float* dc;   // kLfWin x kLfWin
   float* llf;  // kLfWin x kLfWin
   float* tmp;  // kLfWin2 x kLfWin2
   float* lf;   // kLfWin2 x kLfWin2
+  __device__ float* Dc(int X, int Y) const {
+    return dc + (Y - ey) * kLfWin + (X - ex);
+  }
   __device__ float* Llf(int X, int Y) const {
     return llf + (Y - ey) * kLfWin + (X - ex);
   }
@@ -673,18 +612,330 @@ struct LfWin {
   }
 };
 
-__device__ void LlfCell(const Geo& g, const DevFrame& f, const LfGroup& q,
-                        const LfWin& w, int a, int bx, int by) {
-  const int type = a >> 4, cov = Covered(type);
-  float dc[16];
-  for (int iy = 0; iy < cov; ++iy)
-    for (int ix = 0; ix < cov; ++ix)
-      dc[iy * 4 + ix] =
-          f.dc[(size_t(q.c) * g.By + MirrorIdx(q.y0 + by - 1 + iy, g.By)) *
-                   g.Bx +
-               MirrorIdx(q.x0 + bx - 1 + ix, g.Bx)];
-  LowestFreqFromDC(type, dc, 4, w.Llf(bx, by), kLfWin);
-}
+// The per-block LF steps, on a unit of kLanes lanes per block: one lane for
+// the 8x8 classes, a lane per row of the 2 COV x 2 COV low frequencies for
+// 16x16 and 32x32 blocks (4 and 8 lanes). The unit's lanes are consecutive
+// lanes of one warp; every warp step meets at __syncwarp with all lanes
+// (lanes without a block run on the window's first block and store
+// nothing). Each output is ReinterpDct's / ReinterpIdct's sum in their
+// order; products with the zeros of a padded corner, which leave a sum that
+// starts at +0 unchanged, are left out. With one lane per block (the serial
+// 8x8 transforms of a 32x32 block through local memory) the kernel took 1346
+// us on an 8192x8192 frame with a fifth of its area in such blocks, 59 us on
+// a 4K frame of 16x16 blocks and 39 us on a 256x256 frame of every type; with
+// the lanes, 334, 42 and 11 us.
+template <int COV>
+struct LfUnit {
+  static constexpr int N = 2 * COV;                // low frequencies per side
+  static constexpr int kLanes = COV == 1 ? 1 : N;  // lanes per block
+  static constexpr int D = 8 * COV;                // block side
+  static constexpr int sn = SizeIndex(N), sc = SizeIndex(COV),
+                       sd = SizeIndex(D);
+
+  static __device__ __forceinline__ bool DctLike(int type) {
+    return COV > 1 || type == kDCT || type == kDCT_NOHF || type == kLINES;
+  }
+
+  // Row r of a scale table (the tables in global memory: the index differs
+  // between lanes).
+  template <int M>
+  static __device__ __forceinline__ void ScaleRow(const float (*t)[8], int r,
+                                                  float (&v)[M]) {
+#pragma unroll
+    for (int i = 0; i < M; ++i) v[i] = __ldg(&t[r][i]);
+  }
+
+  // ComputeLlf (LowestFrequenciesFromDC) and, with `up`, the block's 2x2
+  // cells from the LLF (DC2x2FromLowestFrequencies).
+  static __device__ __forceinline__ void Llf(const LfWin& w, bool on, int r,
+                                             int type, int X, int Y, bool up) {
+    const float* dc = w.Dc(X, Y);
+    if constexpr (COV == 1) {
+      if (!on) return;
+      float v = dc[0];
+      *w.Llf(X, Y) = v;
+      if (!up) return;
+      float* d = w.Tmp(2 * X, 2 * Y);
+      if (DctLike(type)) {
+        const float* a = IdctMat(2);
+        v = v * c_t.inv_total_scale[sn][0][0] * c_t.total_scale[sd][0][0];
+        // (0.f + x: the sums start at +0)
+        const float t0 = 0.f + v * a[0], t1 = 0.f + v * a[2];
+        *reinterpret_cast<float2*>(d) =
+            make_float2(0.f + a[0] * t0, 0.f + a[2] * t0);
+        *reinterpret_cast<float2*>(d + kLfWin2) =
+            make_float2(0.f + a[0] * t1, 0.f + a[2] * t1);
+      } else {
+        *reinterpret_cast<float2*>(d) = make_float2(v, v);
+        *reinterpret_cast<float2*>(d + kLfWin2) = make_float2(v, v);
+      }
+    } else {
+      // ReinterpDct<D, COV> of the block's DC: the lane takes coefficient
+      // row k = r % COV, whose DCT basis row differs between lanes.
+      const int k = r % COV;
+      float b[COV], ts[COV], its[COV], q[COV], llf[COV];
+#pragma unroll
+      for (int x = 0; x < COV; ++x) {
+        b[x] = __ldg(&g_t.dct[MatOffset(COV) + k * COV + x]);
+      }
+      ScaleRow<COV>(g_t.total_scale[sc], k, ts);
+      ScaleRow<COV>(g_t.inv_total_scale[sd], k, its);
+#pragma unroll
+      for (int y = 0; y < COV; ++y) {
+        float sum = 0.f;
+#pragma unroll
+        for (int x = 0; x < COV; ++x) sum += b[x] * dc[y * kLfWin + x];
+        q[y] = sum;
+      }
+      constexpr float scale = 1.0f / float(COV * COV);
+#pragma unroll
+      for (int l = 0; l < COV; ++l) {
+        float sum = 0.f;
+#pragma unroll
+        for (int y = 0; y < COV; ++y) {
+          sum += q[y] * c_t.dct[MatOffset(COV) + l * COV + y];
+        }
+        llf[l] = sum * scale * ts[l] * its[l];
+      }
+      if (on && r < COV) {
+#pragma unroll
+        for (int l = 0; l < COV; ++l) w.Llf(X, Y + k)[l] = llf[l];
+      }
+      __syncwarp();
+      if (!up) return;
+      // ReinterpIdct<D, COV, N>: the lane takes column v = r of the first
+      // pass and row r of the result.
+      float a[COV], t[COV];
+#pragma unroll
+      for (int l = 0; l < COV; ++l) {
+        a[l] = __ldg(&g_t.idct[MatOffset(N) + r * N + l]);
+      }
+      const float* in = w.Llf(X, Y);
+#pragma unroll
+      for (int kk = 0; kk < COV; ++kk) {
+        float sum = 0.f;
+#pragma unroll
+        for (int l = 0; l < COV; ++l) {
+          const float v = in[kk * kLfWin + l] *
+                          c_t.inv_total_scale[sn][kk][l] *
+                          c_t.total_scale[sd][kk][l];
+          sum += v * a[l];
+        }
+        t[kk] = sum;
+      }
+      float o[N];
+#pragma unroll
+      for (int u = 0; u < N; ++u) {
+        float sum = 0.f;
+#pragma unroll
+        for (int kk = 0; kk < COV; ++kk) {
+          sum += c_t.idct[MatOffset(N) + u * N + kk] * t[kk];
+        }
+        o[u] = sum;
+      }
+      if (on) {
+        float2* d = reinterpret_cast<float2*>(w.Tmp(2 * X, 2 * Y + r));
+#pragma unroll
+        for (int u = 0; u < N; u += 2) d[u / 2] = make_float2(o[u], o[u + 1]);
+      }
+    }
+  }
+
+  // LowFrequenciesFromDC2x2 of the block's cells of the blurred 2x2 image,
+  // in place.
+  static __device__ __forceinline__ void Forward(const LfWin& w, bool on,
+                                                 int r, int type, int X,
+                                                 int Y) {
+    float* base = w.Lf(2 * X, 2 * Y);
+    if constexpr (COV == 1) {
+      if (!on) return;
+      const float2 p0 = *reinterpret_cast<const float2*>(base);
+      const float2 p1 = *reinterpret_cast<const float2*>(base + kLfWin2);
+      const float in[4] = {p0.x, p0.y, p1.x, p1.y};
+      float o[4];
+      if (DctLike(type)) {
+        ReinterpDct<D, N>(in, N, o, N);
+      } else {
+        o[0] = (in[0] + in[1] + in[2] + in[3]) * 0.25f;
+        o[1] = (in[0] + in[1] - in[2] - in[3]) * 0.25f;
+        o[2] = (in[0] - in[1] + in[2] - in[3]) * 0.25f;
+        o[3] = (in[0] - in[1] - in[2] + in[3]) * 0.25f;
+      }
+      *reinterpret_cast<float2*>(base) = make_float2(o[0], o[1]);
+      *reinterpret_cast<float2*>(base + kLfWin2) = make_float2(o[2], o[3]);
+    } else {
+      float q[N];
+      if constexpr (COV == 2) {
+        // The lane forms its row of the first pass from the whole block.
+        float b[N];
+#pragma unroll
+        for (int x = 0; x < N; ++x) {
+          b[x] = __ldg(&g_t.dct[MatOffset(N) + r * N + x]);
+        }
+#pragma unroll
+        for (int y = 0; y < N; ++y) {
+          float sum = 0.f;
+#pragma unroll
+          for (int x = 0; x < N; ++x) sum += b[x] * base[y * kLfWin2 + x];
+          q[y] = sum;
+        }
+      } else {
+        // First pass on the lane's row, transposed through the window.
+        float p[N], t[N];
+        LoadRow(base + r * kLfWin2, p);
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+          float sum = 0.f;
+#pragma unroll
+          for (int x = 0; x < N; ++x) {
+            sum += c_t.dct[MatOffset(N) + k * N + x] * p[x];
+          }
+          t[k] = sum;
+        }
+        __syncwarp();
+        if (on) {
+#pragma unroll
+          for (int k = 0; k < N; ++k) base[k * kLfWin2 + r] = t[k];
+        }
+        __syncwarp();
+        LoadRow(base + r * kLfWin2, q);
+      }
+      float ts[N], its[N], o[N];
+      ScaleRow<N>(g_t.total_scale[sn], r, ts);
+      ScaleRow<N>(g_t.inv_total_scale[sd], r, its);
+      constexpr float scale = 1.0f / float(N * N);
+#pragma unroll
+      for (int l = 0; l < N; ++l) {
+        float sum = 0.f;
+#pragma unroll
+        for (int y = 0; y < N; ++y) {
+          sum += q[y] * c_t.dct[MatOffset(N) + l * N + y];
+        }
+        o[l] = sum * scale * ts[l] * its[l];
+      }
+      __syncwarp();
+      if (on) StoreRow(base + r * kLfWin2, o);
+      __syncwarp();
+    }
+  }
+
+  // UpdateLfForDecoder in place on the dequantised AC: the LLF from DC into
+  // the block's corner, the LF prediction added to the LF coefficients, and
+  // the block's pred2x2 cells from the updated corner. The corner's rows are
+  // contiguous in the frame layout's first cell row.
+  static __device__ __forceinline__ void Update(
+      const Geo& g, const DevFrame& f, const LfGroup& q, const LfWin& w,
+      bool on, int r, int type, int X, int Y, int predict_lf,
+      int predict_hf) {
+    float* base = f.ac + size_t(q.c) * g.ac_stride * g.By +
+                  size_t(q.y0 + Y - 1) * g.ac_stride +
+                  size_t(q.x0 + X - 1) * 64;
+    float* pred = f.pred2x2_g + q.gi * kG2GroupFloats + q.c * kG2 * kG2 +
+                  2 * Y * kG2 + 2 * X;
+    if constexpr (COV == 1) {
+      if (!on) return;
+      float b[4];
+      const float2 a0 = *reinterpret_cast<const float2*>(base);
+      const float2 a1 = *reinterpret_cast<const float2*>(base + 8);
+      b[0] = *w.Llf(X, Y), b[1] = a0.y, b[2] = a1.x, b[3] = a1.y;
+      if (predict_lf) {
+        const float* l = w.Lf(2 * X, 2 * Y);
+        b[1] += l[1], b[2] += l[kLfWin2], b[3] += l[kLfWin2 + 1];
+      }
+      *reinterpret_cast<float2*>(base) = make_float2(b[0], b[1]);
+      *reinterpret_cast<float2*>(base + 8) = make_float2(b[2], b[3]);
+      if (predict_hf) {
+        float o[4];
+        if (DctLike(type)) {
+          ReinterpIdct<D, N, N>(b, N, o, N);
+        } else {
+          o[0] = b[0] + b[1] + b[2] + b[3];
+          o[1] = b[0] + b[1] - b[2] - b[3];
+          o[2] = b[0] - b[1] + b[2] - b[3];
+          o[3] = b[0] - b[1] - b[2] + b[3];
+        }
+        *reinterpret_cast<float2*>(pred) = make_float2(o[0], o[1]);
+        *reinterpret_cast<float2*>(pred + kG2) = make_float2(o[2], o[3]);
+      }
+    } else {
+      float* row = base + r * D;
+      float v[N];
+#pragma unroll
+      for (int x = 0; x < N; x += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(row + x);
+        v[x] = a.x, v[x + 1] = a.y, v[x + 2] = a.z, v[x + 3] = a.w;
+      }
+      float* lf = w.Lf(2 * X, 2 * Y + r);
+      if (predict_lf) {
+        float l[N];
+        LoadRow(lf, l);
+#pragma unroll
+        for (int x = 0; x < N; ++x) v[x] += l[x];
+      }
+      if (r < COV) {
+#pragma unroll
+        for (int x = 0; x < COV; ++x) v[x] = w.Llf(X, Y + r)[x];
+      }
+      if (on) {
+#pragma unroll
+        for (int x = 0; x < N; x += 4) {
+          *reinterpret_cast<float4*>(row + x) =
+              make_float4(v[x], v[x + 1], v[x + 2], v[x + 3]);
+        }
+      }
+      if (!predict_hf) return;
+      // ReinterpIdct<D, N, N>, transposed through the block's cells of the
+      // window (which only this unit still reads).
+      float its[N], ts[N], t[N], o[N];
+      ScaleRow<N>(g_t.inv_total_scale[sn], r, its);
+      ScaleRow<N>(g_t.total_scale[sd], r, ts);
+#pragma unroll
+      for (int l = 0; l < N; ++l) v[l] = v[l] * its[l] * ts[l];
+#pragma unroll
+      for (int u = 0; u < N; ++u) {
+        float sum = 0.f;
+#pragma unroll
+        for (int l = 0; l < N; ++l) {
+          sum += v[l] * c_t.idct[MatOffset(N) + u * N + l];
+        }
+        t[u] = sum;
+      }
+      __syncwarp();
+      if (on) StoreRow(lf, t);
+      __syncwarp();
+      const float* col = w.Lf(2 * X + r, 2 * Y);
+#pragma unroll
+      for (int k = 0; k < N; ++k) t[k] = col[k * kLfWin2];
+#pragma unroll
+      for (int u = 0; u < N; ++u) {
+        float sum = 0.f;
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+          sum += c_t.idct[MatOffset(N) + u * N + k] * t[k];
+        }
+        o[u] = sum;
+      }
+      if (on) StoreRow(pred + r * kG2, o);
+    }
+  }
+
+  // N values of a row of a 2x2 image (8-byte aligned).
+  static __device__ __forceinline__ void LoadRow(const float* p,
+                                                 float (&v)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+      const float2 a = *reinterpret_cast<const float2*>(p + i);
+      v[i] = a.x, v[i + 1] = a.y;
+    }
+  }
+  static __device__ __forceinline__ void StoreRow(float* p,
+                                                  const float (&v)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+      *reinterpret_cast<float2*>(p + i) = make_float2(v[i], v[i + 1]);
+    }
+  }
+};
 
 // LFPredictionBlur over the group's 2x2 image (ConvolveT<Symmetric3>,
 // mirrored at the image's edges) for the run of up to 8 pixels x0 ..
@@ -725,61 +976,62 @@ __device__ void PredBorderCell(const DevFrame& f, const LfGroup& q,
                                const LfWin& w, int x, int y,
                                int predict_lf) {
   float* pred = f.pred2x2_g + q.gi * kG2GroupFloats + q.c * kG2 * kG2;
+  float* d = pred + 2 * y * kG2 + 2 * x;
   if (predict_lf) {
-    float blk[10];
-    blk[0] = *w.Llf(x, y);
-    blk[1] = *w.Lf(2 * x + 1, 2 * y);
-    blk[8] = *w.Lf(2 * x, 2 * y + 1);
-    blk[9] = *w.Lf(2 * x + 1, 2 * y + 1);
-    DC2x2FromLowFreq(kDCT, [&](int k) { return blk[k]; },
-                     pred + 2 * y * kG2 + 2 * x, kG2);
+    const float in[4] = {*w.Llf(x, y), *w.Lf(2 * x + 1, 2 * y),
+                         *w.Lf(2 * x, 2 * y + 1), *w.Lf(2 * x + 1, 2 * y + 1)};
+    ReinterpIdct<8, 2, 2>(in, 2, d, kG2);
   } else {
-    DC2x2FromLowestFreq(kDCT, w.Llf(x, y), kLfWin,
-                        pred + 2 * y * kG2 + 2 * x, kG2);
+    ReinterpIdct<8, 1, 2>(w.Llf(x, y), 0, d, kG2);
   }
 }
 
-// UpdateLfForDecoder for the first block at group cell (X, Y), in place on
-// the dequantised AC: the LLF from DC into the block's corner, the LF
-// prediction added to the LF coefficients, and the block's pred2x2 cells
-// from the updated corner.
-__device__ void LfUpdateBlock(const Geo& g, const DevFrame& f,
-                              const LfGroup& q, const LfWin& w, int type,
-                              int X, int Y, int predict_lf, int predict_hf) {
-  const int bx = q.x0 + X - 1, by = q.y0 + Y - 1, c = q.c;
-  const int cov = Covered(type);
-  float* base = f.ac + size_t(c) * g.ac_stride * g.By +
-                size_t(by) * g.ac_stride + size_t(bx) * 64;
-  const int chunk = 64 * cov;
-  auto at = [&](int i) -> float& {
-    return base[(i / chunk) * size_t(g.ac_stride) + i % chunk];
+// Runs fn(cov, on, r, entry) for the first n[k] blocks of each list (32x32
+// blocks first, whose steps are the longest), warp by warp: a warp step
+// takes 32 / LfUnit<cov>::kLanes blocks of one size. Entries past own[k]
+// stand at the list's back.
+template <typename Fn>
+__device__ __forceinline__ void ForLfUnits(int* const* lists, const int* own,
+                                           const int* n, Fn&& fn) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int kWarps = kLfThreads / 32;
+  const int w4 = (n[2] + 3) / 4, w2 = w4 + (n[1] + 7) / 8,
+            w1 = w2 + (n[0] + 31) / 32;
+  auto entry = [&](int k, int cap, bool on, int u) {
+    if (!on) u = 0;
+    return lists[k][u < own[k] ? u : cap - 1 - (u - own[k])];
   };
-  for (int y = 0; y < cov; ++y)
-    for (int x = 0; x < cov; ++x) at(cov * 8 * y + x) = *w.Llf(X + x, Y + y);
-  if (predict_lf) {
-    for (int y = 0; y < 2 * cov; ++y) {
-      const int start = y < cov ? cov : 0;
-      for (int x = start; x < 2 * cov; ++x) {
-        at(y * cov * 8 + x) += *w.Lf(2 * X + x, 2 * Y + y);
-      }
+  for (int i = warp; i < w1; i += kWarps) {
+    if (i < w4) {
+      const int u = 4 * i + lane / 8;
+      const bool on = u < n[2];
+      fn(std::integral_constant<int, 4>(), on, lane % 8,
+         entry(2, kLfList4, on, u));
+    } else if (i < w2) {
+      const int u = 8 * (i - w4) + lane / 4;
+      const bool on = u < n[1];
+      fn(std::integral_constant<int, 2>(), on, lane % 4,
+         entry(1, kLfList2, on, u));
+    } else {
+      const int u = 32 * (i - w2) + lane;
+      const bool on = u < n[0];
+      fn(std::integral_constant<int, 1>(), on, 0, entry(0, kLfList1, on, u));
     }
-  }
-  if (predict_hf) {
-    float* pred = f.pred2x2_g + q.gi * kG2GroupFloats + c * kG2 * kG2;
-    DC2x2FromLowFreq(type, [&](int i) { return at(i); },
-                     pred + 2 * Y * kG2 + 2 * X, kG2);
   }
 }
 
 // One channel of one tile: blockIdx.x = tile, blockIdx.y = group,
-// blockIdx.z = channel. Phases (a barrier between them): LLF and the 2x2
-// image of every block whose first cell is in [lo - 4, hi + 1) (the blur
-// reads cells lo - 1 .. hi), then the blur and LowFrequenciesFromDC2x2 over
-// [lo, hi) -- the tile plus the ring cells beside it -- then the ring's
-// pred2x2 and the update of the tile's blocks.
+// blockIdx.z = channel. Phases (a barrier between them): the window's DC and
+// the list of its blocks; LLF and the 2x2 image of every block whose first
+// cell is in [lo - 4, hi + 1) (the blur reads cells lo - 1 .. hi), then the
+// blur and LowFrequenciesFromDC2x2 over [lo, hi) -- the tile plus the ring
+// cells beside it -- then the ring's pred2x2 and the update of the tile's
+// blocks. Bound by the latency of the phases' chains: four CTAs per SM (64
+// registers, some spills) took 334 us at 8192x8192, three (80 registers) 340
+// and two 382.
 __global__ void __launch_bounds__(kLfThreads, 4)
     k_lf_tile(Geo g, DevFrame f, int predict_lf, int predict_hf) {
-  extern __shared__ float lf_smem[];
+  extern __shared__ __align__(16) float lf_smem[];
   LfGroup q;
   q.gi = blockIdx.y;
   q.c = blockIdx.z;
@@ -795,47 +1047,55 @@ __global__ void __launch_bounds__(kLfThreads, 4)
   LfWin w;
   w.ex = lx - 4;
   w.ey = ly - 4;
-  w.llf = lf_smem;
-  w.tmp = w.llf + kLfWin * kLfWin;
+  w.tmp = lf_smem;
   w.lf = w.tmp + kLfWin2 * kLfWin2;
+  w.llf = w.lf + kLfWin2 * kLfWin2;
+  w.dc = w.llf + kLfWin * kLfWin;
   // The first cells of the blocks reaching cells lx - 1 .. hx (clipped to
-  // the group's ring), listed as X | Y << 10 | strategy byte << 20, so that
-  // the per-block phases below give every lane a block (a cell-per-lane
-  // loop leaves the lanes of the other cells of multi-block transforms
-  // idle). One list per block size, read as one after the other, so that a
-  // warp's lanes mostly take the same transform sizes (the 32x32 blocks'
-  // LF transforms are far longer than the others').
-  __shared__ int s_n[3];
-  int* lists[3];
-  lists[0] = reinterpret_cast<int*>(w.lf + kLfWin2 * kLfWin2);
-  lists[1] = lists[0] + kLfList1;
-  lists[2] = lists[1] + kLfList2;
-  if (threadIdx.x < 3) s_n[threadIdx.x] = 0;
+  // the group's ring), listed as X | Y << 10 | strategy byte << 20, one list
+  // per block size, so that the per-block phases give every lane work of
+  // its own size. A list holds the tile's own blocks (the only ones to
+  // update) from its front and the others from its back.
+  __shared__ int s_own[3], s_far[3];
+  int* const lists[3] = {
+      reinterpret_cast<int*>(w.dc + kLfWin * kLfWin),
+      reinterpret_cast<int*>(w.dc + kLfWin * kLfWin) + kLfList1,
+      reinterpret_cast<int*>(w.dc + kLfWin * kLfWin) + kLfList1 + kLfList2};
+  if (threadIdx.x < 3) s_own[threadIdx.x] = s_far[threadIdx.x] = 0;
   __syncthreads();
-  const int sx = max(lx - 4, 0), sy = max(ly - 4, 0);
-  const int nx = min(hx + 1, q.gxs + 2) - sx, ny = min(hy + 1, q.gys + 2) - sy;
-  for (int i = threadIdx.x; i < nx * ny; i += kLfThreads) {
-    const int X = sx + i % nx, Y = sy + i / nx;
+  const float* dc = f.dc + size_t(q.c) * g.By * g.Bx;
+  for (int i = threadIdx.x; i < kLfWin * kLfWin; i += kLfThreads) {
+    const int X = w.ex + i % kLfWin, Y = w.ey + i / kLfWin;
+    if (X < 0 || Y < 0 || X > q.gxs + 1 || Y > q.gys + 1) continue;
+    w.dc[i] = dc[size_t(MirrorIdx(q.y0 + Y - 1, g.By)) * g.Bx +
+                 MirrorIdx(q.x0 + X - 1, g.Bx)];
+    if (X > hx || Y > hy) continue;
     const int a = q.Acs(g, f, X, Y);
     if (a & 0xF) continue;
     const int cov = Covered(a >> 4), k = cov == 1 ? 0 : cov == 2 ? 1 : 2;
-    lists[k][atomicAdd(&s_n[k], 1)] = X | (Y << 10) | (a << 20);
-  }
-  __syncthreads();
-  const int n0 = s_n[0], n01 = n0 + s_n[1], nfirst = n01 + s_n[2];
-  auto first_at = [&](int i) {
-    return i < n0 ? lists[0][i] : i < n01 ? lists[1][i - n0]
-                                          : lists[2][i - n01];
-  };
-  for (int i = threadIdx.x; i < nfirst; i += kLfThreads) {
-    const int e = first_at(i);
-    const int X = e & 1023, Y = (e >> 10) & 1023, a = e >> 20;
-    LlfCell(g, f, q, w, a, X, Y);
-    if (predict_lf) {
-      DC2x2FromLowestFreq(a >> 4, w.Llf(X, Y), kLfWin, w.Tmp(2 * X, 2 * Y),
-                          kLfWin2);
+    const int e = X | (Y << 10) | (a << 20);
+    const int cap = k == 0 ? kLfList1 : k == 1 ? kLfList2 : kLfList4;
+    if (X >= X0 && X < X1 && Y >= Y0 && Y < Y1) {
+      lists[k][atomicAdd(&s_own[k], 1)] = e;
+      // The update's lines of the dequantised AC, two phases ahead.
+      const float* row = f.ac + size_t(q.c) * g.ac_stride * g.By +
+                         size_t(q.y0 + Y - 1) * g.ac_stride +
+                         size_t(q.x0 + X - 1) * 64;
+      for (int r = 0; r < (cov == 1 ? 1 : 2 * cov); r += 2) {
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(row + 8 * cov * r));
+      }
+    } else {
+      lists[k][cap - 1 - atomicAdd(&s_far[k], 1)] = e;
     }
   }
+  __syncthreads();
+  int own[3], all[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) own[k] = s_own[k], all[k] = own[k] + s_far[k];
+  ForLfUnits(lists, own, all, [&](auto cov, bool on, int r, int e) {
+    LfUnit<cov.value>::Llf(w, on, r, e >> 24, e & 1023, (e >> 10) & 1023,
+                           predict_lf);
+  });
   __syncthreads();
   if (predict_lf) {
     // Runs of 8 pixels of the blurred range's rows.
@@ -846,12 +1106,11 @@ __global__ void __launch_bounds__(kLfThreads, 4)
       LfBlurRun(q, w, 2 * lx + 8 * r, y, min(8, w2 - 8 * r));
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < nfirst; i += kLfThreads) {
-      const int e = first_at(i);
-      const int X = e & 1023, Y = (e >> 10) & 1023, a = e >> 20;
-      if (X < lx || X >= hx || Y < ly || Y >= hy) continue;
-      LowFreqFromDC2x2(a >> 4, w.Lf(2 * X, 2 * Y), kLfWin2);
-    }
+    ForLfUnits(lists, own, all, [&](auto cov, bool on, int r, int e) {
+      const int X = e & 1023, Y = (e >> 10) & 1023;
+      on = on && X >= lx && X < hx && Y >= ly && Y < hy;
+      LfUnit<cov.value>::Forward(w, on, r, e >> 24, X, Y);
+    });
     __syncthreads();
   }
   if (predict_hf) {
@@ -874,12 +1133,10 @@ __global__ void __launch_bounds__(kLfThreads, 4)
       PredBorderCell(f, q, w, X, Y, predict_lf);
     }
   }
-  for (int i = threadIdx.x; i < nfirst; i += kLfThreads) {
-    const int e = first_at(i);
-    const int X = e & 1023, Y = (e >> 10) & 1023, a = e >> 20;
-    if (X < X0 || X >= X1 || Y < Y0 || Y >= Y1) continue;
-    LfUpdateBlock(g, f, q, w, a >> 4, X, Y, predict_lf, predict_hf);
-  }
+  ForLfUnits(lists, own, own, [&](auto cov, bool on, int r, int e) {
+    LfUnit<cov.value>::Update(g, f, q, w, on, r, e >> 24, e & 1023,
+                              (e >> 10) & 1023, predict_lf, predict_hf);
+  });
 }
 
 // ---------------------------------------------------------------------------
