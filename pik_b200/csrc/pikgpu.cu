@@ -783,8 +783,7 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
       ch(k_square_idct_tc1<32, 3>, grid, tc::kThreads, 0, g, f, L[kC32],
          n[kC32], s.predict_hf, counters + kWorkIdct32, P<int>(ctx->tc_err));
     } else if (n[kC32]) {
-      // One 256-thread CTA per block.
-      ch(k_square_idct<32>, n[kC32], 256, 0, g, f, L[kC32], n[kC32],
+      ch(k_square32_idct, 3 * n[kC32], kSquareThreads, 0, g, f, L[kC32],
          s.predict_hf);
     }
     if (n[kC16] && ctx->form != PIKGPU_FORM_FP32) {
@@ -903,7 +902,7 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
          g, f, s, P<uint32_t>(ctx->active[kC32]), counters + kC32,
          counters + kWorkAr32, P<int>(ctx->tc_err));
     } else if (n[kC32]) {
-      ch(k_square_ar<32>, n[kC32], 256, 0, g, f, s,
+      ch(k_square32_ar, n[kC32], square32::kArThreads, 0, g, f, s,
          P<uint32_t>(ctx->active[kC32]), counters + kC32);
     }
     if (n[kC16] && ctx->form != PIKGPU_FORM_FP32) {

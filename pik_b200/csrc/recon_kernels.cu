@@ -16,7 +16,7 @@ namespace pikgpu {
 __constant__ DevTables c_t;
 // The same tables in global memory, for reads whose index differs between
 // the lanes of a warp (the constant port serves one address at a time).
-__device__ DevTables g_t;
+__device__ __align__(16) DevTables g_t;
 
 namespace {
 
@@ -1140,57 +1140,12 @@ __global__ void __launch_bounds__(kLfThreads, 4)
 }
 
 // ---------------------------------------------------------------------------
-// Cooperative batched transforms in shared memory. `nb` blocks of n x n,
-// contiguous in smem; T threads; every thread calls __syncthreads.
-__device__ void CoopTsIdct(int n, int nb, const float* a, const float* in,
-                           float* tmp, float* out) {
-  const int nn = n * n;
-  for (int i = threadIdx.x; i < nb * nn; i += blockDim.x) {
-    const int b = i / nn, r = i % nn, k = r / n, v = r % n;
-    const float* src = in + b * nn + k * n;
-    float s = 0.f;
-    for (int l = 0; l < n; ++l) s += src[l] * a[v * n + l];
-    tmp[b * nn + k * n + v] = s;
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < nb * nn; i += blockDim.x) {
-    const int b = i / nn, r = i % nn, v = r / n, u = r % n;
-    const float* t = tmp + b * nn;
-    float s = 0.f;
-    for (int k = 0; k < n; ++k) s += a[u * n + k] * t[k * n + v];
-    out[b * nn + v * n + u] = s;
-  }
-  __syncthreads();
-}
-
-__device__ void CoopTsDct(int n, int nb, const float* bm, const float* in,
-                          float* tmp, float* out) {
-  const int nn = n * n;
-  for (int i = threadIdx.x; i < nb * nn; i += blockDim.x) {
-    const int b = i / nn, r = i % nn, k = r / n, y = r % n;
-    const float* src = in + b * nn + y * n;
-    float s = 0.f;
-    for (int x = 0; x < n; ++x) s += bm[k * n + x] * src[x];
-    tmp[b * nn + k * n + y] = s;
-  }
-  __syncthreads();
-  const float scale = 1.0f / float(nn);
-  for (int i = threadIdx.x; i < nb * nn; i += blockDim.x) {
-    const int b = i / nn, r = i % nn, k = r / n, l = r % n;
-    const float* t = tmp + b * nn + k * n;
-    float s = 0.f;
-    for (int y = 0; y < n; ++y) s += t[y] * bm[l * n + y];
-    out[b * nn + k * n + l] = s * scale;
-  }
-  __syncthreads();
-}
-
-// The same two transforms with the matrix given transposed (aT[l n + v] =
-// A[v][l], bT[x n + k] = B[k][x]) and the first DCT pass mapped with k
-// fastest: consecutive threads then read consecutive shared-memory words of
-// the matrix (the plain forms read it with a stride of n words, an n-way
-// bank conflict at n = 32). Every output is the same sum of the same
-// products in the same order, so the results are bit-identical.
+// Cooperative batched transforms in shared memory (the adjoint's). `nb`
+// blocks of n x n, contiguous in smem; every thread of the CTA takes part
+// and calls __syncthreads. The matrix is given transposed (aT[l n + v] =
+// A[v][l], bT[x n + k] = B[k][x]) and the first DCT pass is mapped with k
+// fastest, so that consecutive threads read consecutive words of it. Every
+// output is TsIdct1's / TsDct1's sum in its order.
 __device__ void CoopTsIdctT(int n, int nb, const float* aT, const float* in,
                             float* tmp, float* out) {
   const int nn = n * n;
@@ -1277,74 +1232,6 @@ __device__ __forceinline__ void UpsampleRow(const float* pred, int X0, int Y,
   }
 }
 
-// Square DCT blocks (DCT8, DCT_NOHF, DCT16, DCT32): HF prediction (if the
-// type predicts HF) + AddBlockExceptLFAndLLFTo + InverseIntegralTransform
-// (pik/compressed_image.cc:869-934). One CTA handles `nb` blocks of n x n.
-template <int N>
-__global__ void __launch_bounds__(256)
-    k_square_idct(Geo g, DevFrame f, const uint32_t* list, int count,
-                  int predict_hf) {
-  PdlLaunchDependents();
-  PdlTail pdl_tail;
-  constexpr int NN = N * N;
-  constexpr int NB = NN >= 256 ? 1 : 256 / NN;
-  __shared__ float s_a[NN], s_b[NN];
-  __shared__ float s_c[NB * NN], s_t[NB * NN], s_p[NB * NN];
-  for (int i = threadIdx.x; i < NN; i += blockDim.x) {  // transposed
-    s_a[i] = c_t.idct[MatOffset(N) + (i % N) * N + i / N];
-    s_b[i] = c_t.dct[MatOffset(N) + (i % N) * N + i / N];
-  }
-  const int first = blockIdx.x * NB;
-  const int nb = min(NB, count - first);
-  constexpr int cov = N / 8, chunk = 64 * cov;
-  const size_t plane_ac = size_t(g.ac_stride) * g.By;
-  const size_t plane_px = size_t(g.PW) * g.PH;
-  __syncthreads();
-  for (int c = 0; c < 3; ++c) {
-    // Load coefficients and, if predicting HF, the upsampled pixels.
-    for (int i = threadIdx.x; i < nb * NN; i += blockDim.x) {
-      const int b = i / NN, e = i % NN;
-      const uint32_t pk = list[first + b];
-      const int bx = pk & 0xFFFF, by = pk >> 16;
-      const float* base = f.ac + c * plane_ac + size_t(by) * g.ac_stride +
-                          size_t(bx) * 64;
-      s_c[i] = base[(e / chunk) * size_t(g.ac_stride) + e % chunk];
-      // DCT_NOHF shares this kernel with DCT but takes no HF prediction.
-      if (predict_hf && !PredictHFOf(f.acs[by * g.Bx + bx] >> 4)) {
-        s_p[i] = 0.f;
-      } else if (predict_hf) {
-        const int gi = (by >> 6) * g.Gx + (bx >> 6);
-        const float* pred = f.pred2x2_g + gi * kG2GroupFloats + c * kG2 * kG2;
-        const int X = (bx & 63) * 8 + e % N, Y = (by & 63) * 8 + e / N;
-        s_p[i] = Upsample(pred, X, Y);
-      }
-    }
-    __syncthreads();
-    if (predict_hf) {
-      CoopTsDctT(N, nb, s_b, s_p, s_t, s_p);
-      for (int i = threadIdx.x; i < nb * NN; i += blockDim.x) {
-        const int e = i % NN, y = e / N, x = e % N;
-        if (y < 2 * cov && x < 2 * cov) continue;
-        const uint32_t pk = list[first + i / NN];
-        if (!PredictHFOf(f.acs[(pk >> 16) * g.Bx + (pk & 0xFFFF)] >> 4)) {
-          continue;
-        }
-        s_c[i] += s_p[i];
-      }
-      __syncthreads();
-    }
-    CoopTsIdctT(N, nb, s_a, s_c, s_t, s_p);
-    for (int i = threadIdx.x; i < nb * NN; i += blockDim.x) {
-      const int b = i / NN, e = i % NN;
-      const uint32_t pk = list[first + b];
-      const int bx = pk & 0xFFFF, by = pk >> 16;
-      f.idct[c * plane_px + size_t(by * 8 + e / N) * g.PW + bx * 8 + e % N] =
-          s_p[i];
-    }
-    __syncthreads();
-  }
-}
-
 // DCT4X4 (and _NOHF): four 4x4 transforms with interleaved coefficients
 // (AcStrategy::TransformFromPixels/ToPixels, pik/ac_strategy.cc:604-629,
 // 762-790), with the HF prediction (UpSample4x4BlurDCT,
@@ -1354,8 +1241,7 @@ __global__ void __launch_bounds__(256)
 // (sy, 0) and (sy, 1) (columns sx + 2 l), and in the pixel domain pixel
 // row 4 sy + k. The 4x4 transforms' second passes need the other rows of a
 // sub-block: they go through a small shared-memory transpose per unit.
-// Every sum has the operation order of TsIdct / TsDct (CoopTsIdct,
-// CoopTsDct), so the result is bit-identical to the CTA-wide form.
+// Every sum has the operation order of TsIdct1 / TsDct1.
 constexpr int kDct4Threads = 128;
 __global__ void __launch_bounds__(kDct4Threads)
     k_dct4_idct(Geo g, DevFrame f, const uint32_t* list, int count,
@@ -1964,97 +1850,14 @@ __device__ __forceinline__ float LlfScale(int type, int x, int y) {
   return 1.0f;
 }
 
-// One CTA of 256 threads per DCT32 block (the rows form's one warp per
-// block leaves most SMs idle at a few hundred blocks). `count` is read from
-// device memory (the compacted list of k_active_blocks); the grid covers the
-// class's whole list.
-template <int N>
-__global__ void __launch_bounds__(256)
-    k_square_ar(Geo g, DevFrame f, FrameScalars s, const uint32_t* list,
-                const int* count_ptr) {
-  PdlLaunchDependents();
-  PdlTail pdl_tail;
-  constexpr int NN = N * N;
-  constexpr int NB = NN >= 256 ? 1 : 256 / NN;
-  constexpr int cov = N / 8;
-  const int count = *count_ptr;
-  if (int(blockIdx.x) * NB >= count) return;  // whole CTA
-  __shared__ float s_a[NN], s_b[NN];
-  __shared__ float s_blk[3][NB * NN];
-  __shared__ float s_r[NB * NN], s_t[NB * NN], s_p[NB * NN];
-  for (int i = threadIdx.x; i < NN; i += blockDim.x) {  // transposed
-    s_a[i] = c_t.idct[MatOffset(N) + (i % N) * N + i / N];
-    s_b[i] = c_t.dct[MatOffset(N) + (i % N) * N + i / N];
-  }
-  const int first = blockIdx.x * NB;
-  const int nb = min(NB, count - first);
-  const size_t plane = size_t(g.PW) * g.PH;
-  __syncthreads();
-  for (int c = 0; c < 3; ++c) {
-    for (int i = threadIdx.x; i < nb * NN; i += blockDim.x) {
-      const int b = i / NN, e = i % NN;
-      const uint32_t pk = list[first + b];
-      const int bx = pk & 0xFFFF, by = pk >> 16;
-      const size_t o = c * plane + size_t(by * 8 + e / N) * g.PW + bx * 8 + e % N;
-      s_p[i] = f.filt[o] - f.idct[o];
-    }
-    __syncthreads();
-    CoopTsDctT(N, nb, s_b, s_p, s_t, s_blk[c]);
-  }
-  for (int i = threadIdx.x; i < nb * NN; i += blockDim.x) {
-    const int b = i / NN, e = i % NN, y = e / N, x = e % N;
-    const uint32_t pk = list[first + b];
-    const int bx = pk & 0xFFFF, by = pk >> 16;
-    const int type = f.acs[by * g.Bx + bx] >> 4;
-    const ArBlockInfo info = ArInfo(g, f, s, bx, by, type);
-    float mr = 1.0f, rt[3];
-    int arg = -1;
-    for (int c = 0; c < 3; ++c) {
-      const float interval =
-          (y < cov && x < cov)
-              ? LlfScale(type, x, y) * s.mul_dc[c]
-              : info.dm[c][e] * info.inv_quant_ac;
-      rt[c] = ClampRatio(s_blk[c][i], interval);
-      if (rt[c] < mr) mr = rt[c], arg = c;
-    }
-    if (f.clamp_tape || f.clamp_tape_in) {
-      const size_t to = CoefOffset(g, bx, by, cov, e);
-      uint8_t code = arg < 0 ? 0 : mr == 0.0f ? 4 : uint8_t(arg + 1);
-      if (f.clamp_tape_in) {
-        code = f.clamp_tape_in[to];
-        mr = TapeRatio(code, rt[0], rt[1], rt[2]);
-      }
-      if (f.clamp_tape) f.clamp_tape[to] = code;
-    }
-    s_r[i] = mr;
-  }
-  __syncthreads();
-  for (int c = 0; c < 3; ++c) {
-    for (int i = threadIdx.x; i < nb * NN; i += blockDim.x) {
-      s_blk[c][i] = s_blk[c][i] * s_r[i];
-    }
-    __syncthreads();
-    CoopTsIdctT(N, nb, s_a, s_blk[c], s_t, s_p);
-    for (int i = threadIdx.x; i < nb * NN; i += blockDim.x) {
-      const int b = i / NN, e = i % NN;
-      const uint32_t pk = list[first + b];
-      const int bx = pk & 0xFFFF, by = pk >> 16;
-      const size_t o = c * plane + size_t(by * 8 + e / N) * g.PW + bx * 8 + e % N;
-      f.filt[o] = s_p[i] + f.idct[o];
-    }
-    __syncthreads();
-  }
-}
-
 // Clamp for DCT4X4 blocks: one warp per block, lanes 8 c + j (c < 3) on
 // channel c. Lane j = 4 sy + k of a channel holds pixel row 4 sy + k of the
 // correction (filtered - original) and, after the forward 4x4 transforms,
 // coefficient row sy + 2 k; the minimum ratio over the channels is read
 // from the lanes j, j + 8, j + 16 of the other channels. The second pass
 // of each 4x4 transform reads the other rows of its sub-block through a
-// shared-memory transpose. Every sum has the operation order of TsDct /
-// TsIdct (CoopTsDct, CoopTsIdct). Lanes 24..31 repeat channel 2 and store
-// nothing.
+// shared-memory transpose. Every sum has the operation order of TsDct1 /
+// TsIdct1. Lanes 24..31 repeat channel 2 and store nothing.
 constexpr int kDct4ArThreads = 128;
 __global__ void __launch_bounds__(kDct4ArThreads)
     k_dct4_ar(Geo g, DevFrame f, FrameScalars s, const uint32_t* list,
@@ -2456,8 +2259,6 @@ template __global__ void k_square_idct_rows<8>(Geo, DevFrame, const uint32_t*,
                                                int, int);
 template __global__ void k_square_idct_rows<16>(Geo, DevFrame,
                                                 const uint32_t*, int, int);
-template __global__ void k_square_idct_rows<32>(Geo, DevFrame,
-                                                const uint32_t*, int, int);
 template __global__ void k_square_idct_tc1<16, 2>(Geo, DevFrame,
                                                   const uint32_t*, int, int,
                                                   int*, int*);
@@ -2479,8 +2280,6 @@ template __global__ void k_square_ar_tc<32, 3>(Geo, DevFrame, FrameScalars,
 template __global__ void k_square_ar_rows<8>(Geo, DevFrame, FrameScalars,
                                              const uint32_t*, const int*);
 template __global__ void k_square_ar_rows<16>(Geo, DevFrame, FrameScalars,
-                                              const uint32_t*, const int*);
-template __global__ void k_square_ar_rows<32>(Geo, DevFrame, FrameScalars,
                                               const uint32_t*, const int*);
 
 }  // namespace pikgpu

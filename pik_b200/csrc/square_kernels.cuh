@@ -1,4 +1,4 @@
-// Square DCT blocks (8x8, 16x16, 32x32) with one thread per row of the
+// Square DCT blocks (8x8, 16x16) with one thread per row of the
 // N x N block: a "unit" of N lanes holds one block (and channel) in
 // registers, the transform matrices are compile-time operands from
 // __constant__ memory, and the transpose between the two separable passes
@@ -302,6 +302,230 @@ __global__ void __launch_bounds__(kSquareThreads)
       }
     }
   }
+}
+
+// ---------------------------------------------------------------------------
+// DCT32X32 in the plain FP32 form. Four warps take one block and channel:
+// lane r of every warp holds row r (or column r) of the 32 x 32 matrix in
+// registers and warp w forms the pass's outputs 8 w .. 8 w + 7 of it, with
+// the transform matrix read as 16-byte broadcasts from shared memory (fully
+// unrolled rows with constant operands, as for 16x16, would be 130 KB of
+// code). The transposes between the passes go through two padded tiles, each
+// written again only after the barrier that follows its last reads. Every
+// output is the sequential sum (index 0..31, separate multiply and add) of
+// the row-major formulation, so results are bit-identical to it.
+//
+// Bound by the FP32 pipe and the issue slots of the row and matrix reads: at
+// 3001x2003 with 89% of the area in such blocks the inverse's 8192 rounded
+// operations per lane, block and channel take 0.11 ms at one per clock. A CTA
+// per block with both operands of every product in shared memory took 0.565
+// ms there (clamp 0.544); this split takes 0.241 (0.319), and 9 us instead of
+// 49 on a 256x256 frame of mixed blocks. One warp per item, or per two items,
+// without barriers: 0.248 and 0.223 ms there, but 18 and 31 us on small
+// frames, and 72 instead of 46 us at 1000x1000, where its longer turns leave
+// the last wave empty.
+namespace square32 {
+
+constexpr int kN = 32;
+constexpr int kStride = kN + 1;
+constexpr int kTile = kN * kStride;
+constexpr int kOut = 8;  // outputs per lane and pass
+constexpr int kArThreads = 3 * kSquareThreads;
+
+// The forward or inverse matrix of the tables, row-major.
+__device__ __forceinline__ void LoadMat(float* m, const float* table) {
+  const float4* src = reinterpret_cast<const float4*>(table + MatOffset(kN));
+  for (int i = threadIdx.x; i < kN * kN / 4; i += blockDim.x) {
+    reinterpret_cast<float4*>(m)[i] = src[i];
+  }
+}
+
+// Rows 8 w .. 8 w + 7 of the matrix times the lane's vector.
+__device__ __forceinline__ void Pass(const float* m, int w,
+                                     const float (&v)[kN], float (&o)[kOut]) {
+#pragma unroll
+  for (int h = 0; h < kOut; h += 4) {
+    const float* row = m + (kOut * w + h) * kN;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) o[h + u] = 0.f;
+#pragma unroll
+    for (int i = 0; i < kN; i += 4) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float4 c = *reinterpret_cast<const float4*>(row + u * kN + i);
+        o[h + u] += v[i] * c.x;
+        o[h + u] += v[i + 1] * c.y;
+        o[h + u] += v[i + 2] * c.z;
+        o[h + u] += v[i + 3] * c.w;
+      }
+    }
+  }
+}
+
+__device__ __forceinline__ void Row(const float* t, int r, float (&v)[kN]) {
+#pragma unroll
+  for (int i = 0; i < kN; ++i) v[i] = t[r * kStride + i];
+}
+__device__ __forceinline__ void Col(const float* t, int r, float (&v)[kN]) {
+#pragma unroll
+  for (int i = 0; i < kN; ++i) v[i] = t[i * kStride + r];
+}
+__device__ __forceinline__ void PutRow(float* t, int r, int w,
+                                       const float (&o)[kOut]) {
+#pragma unroll
+  for (int i = 0; i < kOut; ++i) t[r * kStride + kOut * w + i] = o[i];
+}
+__device__ __forceinline__ void PutCol(float* t, int r, int w,
+                                       const float (&o)[kOut]) {
+#pragma unroll
+  for (int i = 0; i < kOut; ++i) t[(kOut * w + i) * kStride + r] = o[i];
+}
+// Eight floats at a 16-byte aligned address.
+__device__ __forceinline__ void Load(const float* p, float (&v)[kOut]) {
+  const float4 a = *reinterpret_cast<const float4*>(p);
+  const float4 b = *reinterpret_cast<const float4*>(p + 4);
+  v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+  v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+}
+__device__ __forceinline__ void Store(float* p, const float (&v)[kOut]) {
+  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
+}
+
+// tsDCT of the pixel rows in t0: coefficients (r, 8 w ..) in `o`.
+__device__ __forceinline__ void Forward(const float* b, const float* t0,
+                                        float* t1, int r, int w,
+                                        float (&o)[kOut]) {
+  float v[kN];
+  __syncthreads();
+  Row(t0, r, v);
+  Pass(b, w, v, o);
+  PutCol(t1, r, w, o);
+  __syncthreads();
+  Row(t1, r, v);
+  Pass(b, w, v, o);
+#pragma unroll
+  for (int i = 0; i < kOut; ++i) o[i] = o[i] * (1.0f / float(kN * kN));
+}
+// tsIDCT of the coefficient rows in t0: pixels (r, 8 w ..) in `o`.
+__device__ __forceinline__ void Inverse(const float* a, const float* t0,
+                                        float* t1, int r, int w,
+                                        float (&o)[kOut]) {
+  float v[kN];
+  __syncthreads();
+  Row(t0, r, v);
+  Pass(a, w, v, o);
+  PutRow(t1, r, w, o);
+  __syncthreads();
+  Col(t1, r, v);
+  Pass(a, w, v, o);
+}
+
+}  // namespace square32
+
+// HF prediction + AddBlockExceptLFAndLLFTo + IDCT, a CTA per (block, channel).
+__global__ void __launch_bounds__(kSquareThreads)
+    k_square32_idct(Geo g, DevFrame f, const uint32_t* list, int predict_hf) {
+  PdlLaunchDependents();
+  PdlTail pdl_tail;
+  using namespace square32;
+  __shared__ __align__(16) float a[kN * kN], b[kN * kN];
+  __shared__ float t0[kTile], t1[kTile];
+  const int r = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int c = blockIdx.x % 3;
+  const uint32_t pk = list[blockIdx.x / 3];
+  const int bx = pk & 0xFFFF, by = pk >> 16;
+  float x[kOut], o[kOut];
+  Load(f.ac + c * size_t(g.ac_stride) * g.By +
+           square::CoefRowOffset(g, bx, by, kN, r) + kOut * w,
+       x);
+  LoadMat(a, g_t.idct);
+  if (predict_hf) {
+    LoadMat(b, g_t.dct);
+    const int gi = (by >> 6) * g.Gx + (bx >> 6);
+    const float* pred = f.pred2x2_g + gi * kG2GroupFloats + c * kG2 * kG2;
+    UpsampleRow<kOut>(pred, (bx & 63) * 8 + kOut * w, (by & 63) * 8 + r, o);
+    PutRow(t0, r, w, o);
+    Forward(b, t0, t1, r, w, o);
+    if (r >= 8 || w >= 1) {  // all but the 8 x 8 low frequencies
+#pragma unroll
+      for (int i = 0; i < kOut; ++i) x[i] += o[i];
+    }
+  }
+  PutRow(t0, r, w, x);
+  Inverse(a, t0, t1, r, w, o);
+  Store(f.idct + c * size_t(g.PW) * g.PH + size_t(by * 8 + r) * g.PW + bx * 8 +
+            kOut * w,
+        o);
+}
+
+// AdaptiveReconstruction clamp of DCT32X32 blocks
+// (pik/adaptive_reconstruction.cc:128-244, 334-471): a CTA per block, four
+// warps per channel; the channels' ratios meet in shared memory. `count` is
+// read from device memory (k_active_blocks).
+__global__ void __launch_bounds__(square32::kArThreads, 3)
+    k_square32_ar(Geo g, DevFrame f, FrameScalars s, const uint32_t* list,
+                  const int* count_ptr) {
+  PdlLaunchDependents();
+  PdlTail pdl_tail;
+  using namespace square32;
+  constexpr int cov = kN / 8;
+  __shared__ __align__(16) float a[kN * kN], b[kN * kN];
+  __shared__ float t0[3][kTile], t1[3][kTile];
+  if (int(blockIdx.x) >= *count_ptr) return;  // whole CTA
+  const int r = threadIdx.x & 31, w = (threadIdx.x >> 5) & 3;
+  const int c = threadIdx.x / kSquareThreads;
+  const uint32_t pk = list[blockIdx.x];
+  const int bx = pk & 0xFFFF, by = pk >> 16;
+  const size_t row = c * size_t(g.PW) * g.PH + size_t(by * 8 + r) * g.PW +
+                     bx * 8 + kOut * w;
+  float x[kOut], y[kOut], o[kOut];
+  Load(f.filt + row, y);
+  Load(f.idct + row, x);
+  LoadMat(a, g_t.idct);
+  LoadMat(b, g_t.dct);
+  const ArBlockInfo info = ArInfo(g, f, s, bx, by, kDCT32X32);
+  const float* dm = c == 0 ? info.dm[0] : c == 1 ? info.dm[1] : info.dm[2];
+  const int e0 = r * kN + kOut * w;
+#pragma unroll
+  for (int i = 0; i < kOut; ++i) y[i] = y[i] - x[i];
+  PutRow(t0[c], r, w, y);
+  Forward(b, t0[c], t1[c], r, w, y);
+  // This channel's ratios, then the minimum over the channels.
+#pragma unroll
+  for (int i = 0; i < kOut; ++i) {
+    const bool llf = r < cov && kOut * w + i < cov;
+    const float interval = llf ? c_t.ar_llf32[r & 3][i & 3] * s.mul_dc[c]
+                               : dm[e0 + i] * info.inv_quant_ac;
+    o[i] = ClampRatio(y[i], interval);
+  }
+  PutRow(t0[c], r, w, o);
+  __syncthreads();
+  const size_t to = CoefOffset(g, bx, by, cov, e0);
+#pragma unroll
+  for (int i = 0; i < kOut; ++i) {
+    const int p = r * kStride + kOut * w + i;
+    const float r0 = t0[0][p], r1 = t0[1][p], r2 = t0[2][p];
+    float mr = 1.0f;
+    int arg = -1;
+    if (r0 < mr) mr = r0, arg = 0;
+    if (r1 < mr) mr = r1, arg = 1;
+    if (r2 < mr) mr = r2, arg = 2;
+    if (f.clamp_tape || f.clamp_tape_in) {
+      uint8_t code = arg < 0 ? 0 : mr == 0.0f ? 4 : uint8_t(arg + 1);
+      if (f.clamp_tape_in) {
+        code = f.clamp_tape_in[to + i];
+        mr = TapeRatio(code, r0, r1, r2);
+      }
+      if (f.clamp_tape && c == 0) f.clamp_tape[to + i] = code;
+    }
+    y[i] = y[i] * mr;
+  }
+  PutRow(t1[c], r, w, y);
+  Inverse(a, t1[c], t0[c], r, w, o);
+#pragma unroll
+  for (int i = 0; i < kOut; ++i) o[i] = o[i] + x[i];
+  Store(f.filt + row, o);
 }
 
 }  // namespace pikgpu
