@@ -868,13 +868,9 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
       }
     }
     br.Fork(2, 1);
-    auto rows_grid = [](int items, int nn) {
-      const int upw = 32 / nn;
-      const int warps = (items + upw - 1) / upw;
-      return (warps * 32 + kSquareThreads - 1) / kSquareThreads;
-    };
     if (n[kC8]) {
-      k_square_ar_rows<8><<<rows_grid(n[kC8], 8), kSquareThreads, 0, st>>>(
+      k_square_ar_rows<8><<<Blocks(n[kC8], SquareArBlocks<8>()),
+                            kSquareArThreads, 0, st>>>(
           g, f, s, P<uint32_t>(ctx->active[kC8]), counters + kC8);
       ++ctx->launches;
     }
@@ -918,8 +914,9 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
            counters + kWorkAr, P<int>(ctx->tc_err));
       }
     } else if (n[kC16]) {
-      ch(k_square_ar_rows<16>, rows_grid(n[kC16], 16), kSquareThreads, 0, g,
-         f, s, P<uint32_t>(ctx->active[kC16]), counters + kC16);
+      ch(k_square_ar_rows<16>, Blocks(n[kC16], SquareArBlocks<16>()),
+         kSquareArThreads, 0, g, f, s, P<uint32_t>(ctx->active[kC16]),
+         counters + kC16);
     }
     CUDA_TRY(ctx, ch.err);
     br.Join(2, 1);

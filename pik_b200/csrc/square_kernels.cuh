@@ -197,80 +197,103 @@ __global__ void k_active_blocks(Geo g, const int32_t* sigma,
   }
 }
 
-// AdaptiveReconstruction clamp for square DCT blocks, one unit per block
-// (pik/adaptive_reconstruction.cc:128-244, 334-471). `count` is read from
-// device memory (the compacted list of k_active_blocks).
+// Clamp intervals of N consecutive coefficients from the dequantisation
+// matrix at `dm` (16-byte loads where its place in the table allows them).
 template <int N>
-__global__ void __launch_bounds__(kSquareThreads)
+__device__ __forceinline__ void LoadIntervals(const float* dm, float scale,
+                                              float (&v)[N]) {
+  if ((reinterpret_cast<uintptr_t>(dm) & 15) == 0) {
+#pragma unroll
+    for (int i = 0; i < N; i += 4) {
+      const float4 q = *reinterpret_cast<const float4*>(dm + i);
+      v[i] = q.x * scale, v[i + 1] = q.y * scale;
+      v[i + 2] = q.z * scale, v[i + 3] = q.w * scale;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = dm[i] * scale;
+  }
+}
+
+// AdaptiveReconstruction clamp for square DCT blocks
+// (pik/adaptive_reconstruction.cc:128-244, 334-471): a warp per channel of
+// 32 / N blocks, the channels' ratios meeting in shared memory. With the
+// three channels in one warp instead (three times the registers and a third
+// of the warps) the clamp of a 256x256 frame of 16x16 blocks took 27 us
+// against 9, of a 3840x2160 one 103 against 65. `count` is read from device
+// memory (the compacted list of k_active_blocks).
+constexpr int kSquareArGroups = 2;  // warps per channel in a CTA
+constexpr int kSquareArThreads = 96 * kSquareArGroups;
+template <int N>
+__host__ __device__ constexpr int SquareArBlocks() {  // blocks per CTA
+  return kSquareArGroups * 32 / N;
+}
+template <int N>
+__global__ void __launch_bounds__(kSquareArThreads)
     k_square_ar_rows(Geo g, DevFrame f, FrameScalars s, const uint32_t* list,
                      const int* count_ptr) {
   PdlLaunchDependents();
   PdlTail pdl_tail;
   using namespace square;
   constexpr int UPW = 32 / N;
-  constexpr int cov = N / 8;
-  __shared__ float s_tile[kSquareThreads / N][N * (N + 1)];
+  constexpr int cov = N / 8, tile_size = N * (N + 1);
+  __shared__ float s_tile[kSquareArGroups][3][UPW][tile_size];
+  __shared__ float s_ratio[kSquareArGroups][3][UPW][tile_size];
   const int count = *count_ptr;
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (int(blockIdx.x) * SquareArBlocks<N>() >= count) return;  // whole CTA
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = warp % 3, grp = warp / 3;
   const int unit = lane / N, r = lane % N;
-  const int item = warp * UPW + unit;
-  if (warp * UPW >= count) return;  // warp-uniform
+  const int item = (blockIdx.x * kSquareArGroups + grp) * UPW + unit;
   const bool active = item < count;
-  float* tile = s_tile[threadIdx.x / N];
+  float* tile = s_tile[grp][c][unit];
   const uint32_t pk = list[active ? item : 0];
   const int bx = pk & 0xFFFF, by = pk >> 16;
-  const int type = f.acs[by * g.Bx + bx] >> 4;
-  const size_t plane = size_t(g.PW) * g.PH;
-  const size_t row0 = size_t(by * 8 + r) * g.PW + bx * 8;
-  float Y[3][N];
+  const size_t row = c * size_t(g.PW) * g.PH + size_t(by * 8 + r) * g.PW +
+                     bx * 8;
+  float X[N], D[N], Y[N];
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    float D[N], T[N];
-#pragma unroll
-    for (int x = 0; x < N; x += 4) {
-      const float4 a =
-          *reinterpret_cast<const float4*>(f.filt + c * plane + row0 + x);
-      const float4 o =
-          *reinterpret_cast<const float4*>(f.idct + c * plane + row0 + x);
-      D[x] = a.x - o.x, D[x + 1] = a.y - o.y;
-      D[x + 2] = a.z - o.z, D[x + 3] = a.w - o.w;
-    }
-    DctRow<N>(D, T);
-    PutCol<N>(tile, r, T);
-    __syncwarp();
-    GetRow<N>(tile, r, D);
-    DctCol<N>(D, Y[c]);
-    __syncwarp();
+  for (int x = 0; x < N; x += 4) {
+    const float4 a = *reinterpret_cast<const float4*>(f.filt + row + x);
+    const float4 o = *reinterpret_cast<const float4*>(f.idct + row + x);
+    X[x] = o.x, X[x + 1] = o.y, X[x + 2] = o.z, X[x + 3] = o.w;
+    D[x] = a.x - o.x, D[x + 1] = a.y - o.y;
+    D[x + 2] = a.z - o.z, D[x + 3] = a.w - o.w;
   }
-  // Clamp ratios of coefficient row k = r, minimum over the channels.
-  const int qac = f.qf[by * g.Bx + bx];
-  const float inv_quant_ac =
-      ClampInvQuantAc(g, f, s.inv_global_scale, bx, by, qac);
-  const int cf = f.dq_cf[(by >> 3) * g.Tx + (bx >> 3)];
-  const int table = f.dq_map[cf * 256 + (qac - 1)];
-  const int kind = QuantKindOf(type);
-  const float* dm0 = f.table + f.offsets[(table * 7 + kind) * 3 + 0] + r * N;
-  const float* dm1 = f.table + f.offsets[(table * 7 + kind) * 3 + 1] + r * N;
-  const float* dm2 = f.table + f.offsets[(table * 7 + kind) * 3 + 2] + r * N;
+  const int type = f.acs[by * g.Bx + bx] >> 4;
+  const ArBlockInfo info = ArInfo(g, f, s, bx, by, type);
+  const float* dm = c == 0 ? info.dm[0] : c == 1 ? info.dm[1] : info.dm[2];
+  DctRow<N>(D, Y);
+  PutCol<N>(tile, r, Y);
+  __syncwarp();
+  GetRow<N>(tile, r, D);
+  DctCol<N>(D, Y);
+  __syncwarp();
+  // This channel's clamp ratios of coefficient row k = r.
+  float* ratio = s_ratio[grp][0][unit] + r * (N + 1);
+  constexpr int channel = UPW * tile_size;
+  LoadIntervals<N>(dm + r * N, info.inv_quant_ac, D);
+  if (r < cov) {
+#pragma unroll
+    for (int l = 0; l < cov; ++l) D[l] = LlfScale(type, l, r) * s.mul_dc[c];
+  }
+#pragma unroll
+  for (int l = 0; l < N; ++l) ratio[c * channel + l] = ClampRatio(Y[l], D[l]);
+  __syncthreads();
   const size_t tape_row = CoefOffset(g, bx, by, cov, r * N);
-  uint8_t* tape = f.clamp_tape && active ? f.clamp_tape + tape_row : nullptr;
+  uint8_t* tape =
+      f.clamp_tape && active && c == 0 ? f.clamp_tape + tape_row : nullptr;
   const uint8_t* tin =
       f.clamp_tape_in && active ? f.clamp_tape_in + tape_row : nullptr;
 #pragma unroll
   for (int l = 0; l < N; ++l) {
-    const bool llf = r < cov && l < cov;
-    const float ls = llf ? LlfScale(type, l, r) : 0.f;
+    // The minimum over the channels.
+    const float rt0 = ratio[l], rt1 = ratio[channel + l],
+                rt2 = ratio[2 * channel + l];
     float mr = 1.0f;
     int arg = -1;
-    const float rt0 =
-        ClampRatio(Y[0][l], llf ? ls * s.mul_dc[0] : dm0[l] * inv_quant_ac);
     if (rt0 < mr) mr = rt0, arg = 0;
-    const float rt1 =
-        ClampRatio(Y[1][l], llf ? ls * s.mul_dc[1] : dm1[l] * inv_quant_ac);
     if (rt1 < mr) mr = rt1, arg = 1;
-    const float rt2 =
-        ClampRatio(Y[2][l], llf ? ls * s.mul_dc[2] : dm2[l] * inv_quant_ac);
     if (rt2 < mr) mr = rt2, arg = 2;
     uint8_t code = arg < 0 ? 0 : mr == 0.0f ? 4 : uint8_t(arg + 1);
     if (tin) {
@@ -278,28 +301,19 @@ __global__ void __launch_bounds__(kSquareThreads)
       mr = TapeRatio(code, rt0, rt1, rt2);
     }
     if (tape) tape[l] = code;
-    Y[0][l] = Y[0][l] * mr;
-    Y[1][l] = Y[1][l] * mr;
-    Y[2][l] = Y[2][l] * mr;
+    Y[l] = Y[l] * mr;
   }
+  IdctRow<N>(Y, D);
+  PutRow<N>(tile, r, D);
+  __syncwarp();
+  GetCol<N>(tile, r, Y);
+  IdctCol<N>(Y, D);
+  if (active) {
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    float T[N], U[N];
-    IdctRow<N>(Y[c], T);
-    PutRow<N>(tile, r, T);
-    __syncwarp();
-    GetCol<N>(tile, r, U);
-    IdctCol<N>(U, T);
-    __syncwarp();
-    if (active) {
-#pragma unroll
-      for (int x = 0; x < N; x += 4) {
-        const float4 o =
-            *reinterpret_cast<const float4*>(f.idct + c * plane + row0 + x);
-        *reinterpret_cast<float4*>(f.filt + c * plane + row0 + x) =
-            make_float4(T[x] + o.x, T[x + 1] + o.y, T[x + 2] + o.z,
-                        T[x + 3] + o.w);
-      }
+    for (int x = 0; x < N; x += 4) {
+      *reinterpret_cast<float4*>(f.filt + row + x) =
+          make_float4(D[x] + X[x], D[x + 1] + X[x + 1], D[x + 2] + X[x + 2],
+                      D[x + 3] + X[x + 3]);
     }
   }
 }
@@ -319,7 +333,7 @@ __global__ void __launch_bounds__(kSquareThreads)
 // 3001x2003 with 89% of the area in such blocks the inverse's 8192 rounded
 // operations per lane, block and channel take 0.11 ms at one per clock. A CTA
 // per block with both operands of every product in shared memory took 0.565
-// ms there (clamp 0.544); this split takes 0.241 (0.319), and 9 us instead of
+// ms there (clamp 0.544); this split takes 0.241 (0.290), and 9 us instead of
 // 49 on a 256x256 frame of mixed blocks. One warp per item, or per two items,
 // without barriers: 0.248 and 0.223 ms there, but 18 and 31 us on small
 // frames, and 72 instead of 46 us at 1000x1000, where its longer turns leave
@@ -492,13 +506,13 @@ __global__ void __launch_bounds__(square32::kArThreads, 3)
   PutRow(t0[c], r, w, y);
   Forward(b, t0[c], t1[c], r, w, y);
   // This channel's ratios, then the minimum over the channels.
+  LoadIntervals<kOut>(dm + e0, info.inv_quant_ac, o);
+  if (r < cov && w == 0) {
 #pragma unroll
-  for (int i = 0; i < kOut; ++i) {
-    const bool llf = r < cov && kOut * w + i < cov;
-    const float interval = llf ? c_t.ar_llf32[r & 3][i & 3] * s.mul_dc[c]
-                               : dm[e0 + i] * info.inv_quant_ac;
-    o[i] = ClampRatio(y[i], interval);
+    for (int i = 0; i < cov; ++i) o[i] = c_t.ar_llf32[r][i] * s.mul_dc[c];
   }
+#pragma unroll
+  for (int i = 0; i < kOut; ++i) o[i] = ClampRatio(y[i], o[i]);
   PutRow(t0[c], r, w, o);
   __syncthreads();
   const size_t to = CoefOffset(g, bx, by, cov, e0);
