@@ -23,12 +23,11 @@
 //    at most kNoAllocMaxBlocks x kNoAllocMaxBlocks, so images up to
 //    4096 x 4096 pixels. Larger sizes are rejected with PIKGPU_ERR_INVALID_ARG
 //    before any work is queued.
-//  * The scratch holds the padded DC image (3 x 512 x 512 floats), 4096
-//    per-block sigmas and the guide min/max words, about 3.02 MiB of static
-//    device memory per device.
+//  * The scratch holds the padded DC image (3 x 512 x 512 floats) and the
+//    guide min/max words, about 3 MiB of static device memory per device.
 //  * No part of the scratch has to start at zero. Every call first resets
 //    the min/max words with a kernel, then fully writes the padded image
-//    and the sigmas before it reads them.
+//    before it reads it.
 //  * The first call on a device does the set-up, with that device current:
 //    it uploads the constant tables, sets the EPF kernel's shared-memory
 //    limit, reads the SM count and looks up the scratch address. Make
@@ -43,10 +42,8 @@ namespace {
 
 constexpr int kNoAllocMaxBlocks = 512;
 constexpr size_t kNoAllocPlane = size_t(kNoAllocMaxBlocks) * kNoAllocMaxBlocks;
-constexpr size_t kNoAllocSigmas = kNoAllocPlane / 64;  // 8x8-block EPF cells
 constexpr size_t kNoAllocPadOff = 0;                  // 3 padded DC planes
-constexpr size_t kNoAllocSigOff = 3 * kNoAllocPlane;  // int32 sigma / cell
-constexpr size_t kNoAllocMmOff = kNoAllocSigOff + kNoAllocSigmas;  // 16 words
+constexpr size_t kNoAllocMmOff = 3 * kNoAllocPlane;   // 16 words
 constexpr size_t kNoAllocWords = kNoAllocMmOff + 64;
 
 struct NoAllocDevice {
@@ -164,22 +161,17 @@ int DcNoAlloc(pikgpu_ctx* ctx, const int16_t* quantized_dc, uint32_t bx,
   f.dc = dc;
 
   float* dcpad = reinterpret_cast<float*>(scratch + kNoAllocPadOff);
-  int32_t* sig = reinterpret_cast<int32_t*>(scratch + kNoAllocSigOff);
   uint32_t* mm = scratch + kNoAllocMmOff;
   const int dpw = (g.Bx + 7) / 8 * 8, dph = (g.By + 7) / 8 * 8;
 
   // The FP32 form's DC stage of LaunchAll: min/max reset, dequantisation
   // with the padded copy and its min/max, then the EPF clamping into `dc`.
-  k_frame_init<<<1, 32, 0, st>>>(mm, nullptr, 0);
+  k_frame_init<<<1, 32, 0, st>>>(mm, nullptr, 0, nullptr, 0);
   k_dc_prep<<<dim3(Blocks(dpw, 32), Blocks(dph, 8)), 256, 0, st>>>(
       g, f, s, dcpad, dpw, dph, mm + 8);
-  EpfSigma sgs{};
-  sgs.const_qf = s.quant_dc / 2;
-  sgs.fixed = -1;
-  sgs.out = sig;
   const EpfDc dco{dc, g.Bx, g.By, half_step[0], half_step[1], half_step[2]};
   EpfLaunch(st, num_sms, PIKGPU_FORM_FP32, dcpad, dcpad, 0, dpw, dph, mm + 8,
-            sgs, nullptr, nullptr, dco, /*err=*/nullptr);
+            DcEpfWork(s), nullptr, nullptr, dco, /*err=*/nullptr);
   CUDA_TRY(ctx, cudaGetLastError());
   return PIKGPU_OK;
 }

@@ -56,7 +56,6 @@ constexpr size_t EpfSmemBytes(int th) {
 __host__ __device__ constexpr uint32_t EpfTileBytes(int th) {
   return uint32_t(3 * (th + 10) * kEpfTW * 4);
 }
-constexpr size_t kEpfSmemBytes = EpfSmemBytes(kEpfH);
 
 // WeightFast (pik/epf_target.cc:304-428) as 4 integer operations:
 // ((int16(min(sad, 507) << 6) * mul) >> 16 + (127 << 7)) in the high half of
@@ -122,23 +121,22 @@ __device__ __forceinline__ void PatchSads4(const uint32_t* rf,
   }
 }
 
-// Where the per-block sigma comes from. It is computed in the kernel from
-// the guide's stretch (SigmaFromQuant, pik/epf_target.cc:1072-1111):
-// `ovr` (the verification override) if set; else `fixed` if >= 0 (the
-// fixed-sigma EPF, pik/epf_target.cc:1342-1386); else from qf, strategy
-// and LUT per block; or, qf NULL (the DC image), from the constant
-// `const_qf` with a DCT strategy and LUT 0 (AdaptiveDCReconstruction,
-// pik/adaptive_reconstruction.cc:300-318). The sigma used is written to
-// `out` (NULL: not written) by one lane per block.
-struct EpfSigma {
-  const int32_t* ovr;
-  const int32_t* qf;
-  const uint8_t* acs;
-  const uint8_t* lut;
-  int const_qf;
-  int fixed;
-  int32_t* out;
+// The frame EPF's work list, made by k_epf_plan: the regions of kEpfW x
+// kEpfRegionH pixels that hold a filtered block. The output of the others is
+// the input, and is not written: their readers take the input there
+// (k_final_direct; the clamp only visits filtered blocks, and no block
+// crosses regions). `sigma` is the blocks' sigma. The DC image's tiles are
+// all taken; its blocks share one sigma (SigmaFromQuant of the constant
+// `dc_qf` with a DCT strategy and LUT 0, AdaptiveDCReconstruction,
+// pik/adaptive_reconstruction.cc:300-318).
+struct EpfWork {
+  const uint32_t* list;
+  const int* count;
+  const int32_t* sigma;
+  int dc_qf;
 };
+constexpr int kEpfRegionH = kRegionH;  // every tile height divides it
+static_assert(kEpfW == kRegionW, "a region is as wide as a tile");
 
 // The DC image's output: instead of storing the filtered value, the clamp
 // of AdaptiveDCReconstruction (pik/adaptive_reconstruction.cc:319-331),
@@ -149,37 +147,6 @@ struct EpfDc {
   int w, h;
   float hs0, hs1, hs2;
 };
-
-// Sigma of this thread's block in the tile at (x0, y0); 0 outside the image.
-// Sigma of the block holding pixel (px, py0) (0 outside the image); `store`:
-// also write it to s.out.
-__device__ __forceinline__ int EpfBlockSigma(const EpfSigma& s, float stretch,
-                                             int w, int h, int px, int py0,
-                                             bool store) {
-  if (px >= w || py0 >= h) return 0;
-  const int bi = (py0 >> 3) * (w / 8) + (px >> 3);
-  int sg;
-  if (s.ovr) {
-    sg = s.ovr[bi];
-  } else if (s.fixed >= 0) {
-    sg = s.fixed;
-  } else if (s.qf) {
-    sg = SigmaFromQuant(float(s.qf[bi]), ARQuantScaleOf(s.acs[bi] >> 4),
-                        s.lut[bi], stretch);
-  } else {
-    sg = SigmaFromQuant(float(s.const_qf), 1.0f, 0, stretch);
-  }
-  if (s.out && store) s.out[bi] = sg;
-  return sg;
-}
-
-__device__ __forceinline__ int EpfLaneSigma(const EpfSigma& s, float stretch,
-                                            int w, int h, int x0, int y0) {
-  const int t = threadIdx.x;
-  const int px = x0 + (t & 31) + 32 * ((t >> 5) & 1), py0 = y0 + 4 * (t >> 6);
-  return EpfBlockSigma(s, stretch, w, h, px, py0,
-                       (px & 7) == 0 && (py0 & 7) == 0);
-}
 
 // Stores the value of channel c at pixel (px, y) of the tile's output.
 __device__ __forceinline__ void EpfStore(float* out, const EpfDc& dco,
@@ -548,7 +515,7 @@ __device__ __forceinline__ void EpfFilterCore(
 // Filters the staged tile at (x0, y0) into `out` (or, for the DC image,
 // into dco's clamp), with every thread of the CTA: the guide, then the
 // filter. The tile's copies are complete in every thread (the first
-// barrier below publishes them); `sig` is EpfLaneSigma of this thread;
+// barrier below publishes them); `sig` is the sigma of this thread's block;
 // (amin, mul) quantise the guide (GuideParams). `sa` holds the aligned
 // guide words while the guide is built.
 //
@@ -585,9 +552,15 @@ __device__ __forceinline__ void EpfFilterTile(
   EpfFilterCore<kFma, TH>(tid, sig, out, dco, w, h, sg, tile, x0, y0);
 }
 
-// One CTA per 64 x TH tile (1-D grid, row-major tile order). More CTAs
-// than resident slots balance the uneven tiles (copies, border tiles)
-// better than CTAs that loop over tiles.
+// One CTA per 64 x TH tile (1-D grid). More CTAs than resident slots balance
+// the uneven tiles (copies, border tiles) better than CTAs that loop over
+// tiles. kList: the tiles of the regions in the work list; the grid has a CTA
+// for every tile that the list may hold, and those past its end leave at
+// once. Against a CTA per tile that reads, and where nothing is filtered
+// copies, every tile: 426 -> 76 us at 8192x8192 with 4% of the blocks
+// filtered, 218 -> 188 at 4K with a third, and 402 -> 404 at 3001x2003 with
+// all of them. CTAs that loop over the list's tiles took 105, 211 and 439: a
+// new CTA's list entry and copy overlap the filtering of its neighbours.
 //
 // Interior tiles are staged by the Tensor Memory Accelerator when `tmap`
 // is valid (use_tma): one thread issues a 3-D tiled bulk copy
@@ -599,13 +572,13 @@ __device__ __forceinline__ void EpfFilterTile(
 // multiple of 64), as the copy requires. The wait is bounded (`polls`, the
 // context's PIKGPU_OPT_TC_WAIT_POLLS): if it runs out, the kernel sets
 // *err = 2 (the host reports the frame as failed) and waits once more,
-// bounded, so that no copy is in flight when the CTA exits. Border tiles, and all tiles without a tensor map, are staged with
-// cp.async (EpfStage).
-template <bool kFma, int TH>
+// bounded, so that no copy is in flight when the CTA exits. Border tiles,
+// and all tiles without a tensor map, are staged with cp.async (EpfStage).
+template <bool kFma, int TH, bool kList>
 __global__ void __launch_bounds__(16 * TH, TH == 16 ? 3 : 2)
     k_epf_box(const float* in, const float* guide_src,
               const uint8_t* guide_ovr, int gab, int w, int h,
-              const uint32_t* mm, EpfSigma sgs, float* out, EpfDc dco,
+              const uint32_t* mm, EpfWork work, float* out, EpfDc dco,
               const __grid_constant__ CUtensorMap tmap, int use_tma,
               int* err, uint32_t polls) {
   extern __shared__ __align__(128) uint32_t epf_smem[];
@@ -614,15 +587,27 @@ __global__ void __launch_bounds__(16 * TH, TH == 16 ? 3 : 2)
       epf_smem + 3 * (TH + 8) * kEpfGRow);
   uint32_t* sa = epf_smem + 3 * (TH + 8) * kEpfGRow + 3 * (TH + 10) * kEpfTS;
   uint64_t* mbar = reinterpret_cast<uint64_t*>(sa + 3 * (TH + 8) * kEpfAligned);
-  PdlLaunchDependents();  // the active-block pass may start on free SMs
+  PdlLaunchDependents();
   const int tiles_x = (w + kEpfW - 1) / kEpfW;
-  const int x0 = (blockIdx.x % tiles_x) * kEpfW;
-  const int y0 = (blockIdx.x / tiles_x) * TH;
   const uint32_t tile_s = tc::SmemU32(tile), mbar_s = tc::SmemU32(mbar);
+  const int tid = threadIdx.x, lane = tid & 31;
+  int x0, y0;
+  if (kList) {
+    constexpr int kSub = kEpfRegionH / TH;  // tiles per region
+    PdlWait();  // the list is the output of the kernel before this one
+    const int region = int(work.list[blockIdx.x / kSub]);
+    if (int(blockIdx.x) >= *work.count * kSub) return;
+    x0 = (region % tiles_x) * kEpfW;
+    y0 = (region / tiles_x) * kEpfRegionH + (blockIdx.x % kSub) * TH;
+    if (y0 >= h) return;
+  } else {
+    x0 = (blockIdx.x % tiles_x) * kEpfW;
+    y0 = (blockIdx.x / tiles_x) * TH;
+  }
   const bool tma = use_tma && EpfInterior<TH>(w, h, x0, y0) &&
                    (tile_s & 127u) == 0;
   if (tma) {
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar_s)
                    : "memory");
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -639,19 +624,21 @@ __global__ void __launch_bounds__(16 * TH, TH == 16 ? 3 : 2)
           : "memory");
     }
   } else {
-    EpfStage<TH>(in, w, h, x0, y0, tile, threadIdx.x);
+    EpfStage<TH>(in, w, h, x0, y0, tile, tid);
   }
-  // The input is complete before the min/max pass starts; the guide range
-  // in `mm` is that pass's output (the previous kernel on the stream, under
-  // a programmatic dependent launch still running until here).
-  PdlWait();
   float amin, mul, stretch;
   GuideParams(mm, &amin, &mul, &stretch);
-  const int sig = EpfLaneSigma(sgs, stretch, w, h, x0, y0);
+  int sig = 0;
+  const int px = x0 + lane + 32 * ((tid >> 5) & 1), py = y0 + 4 * (tid >> 6);
+  if (px < w && py < h) {
+    sig = kList ? work.sigma[(py >> 3) * (w / 8) + (px >> 3)]
+                : ScaledSigma(UnscaledSigma(float(work.dc_qf), 1.0f, 0),
+                              stretch);
+  }
   if (tma) {
     __syncthreads();  // the mbarrier is initialised before anyone waits
     // (tc::WaitMma is the bounded mbarrier wait of the tensor-core kernels)
-    if (!tc::WaitMma(mbar_s, 0, polls) && threadIdx.x == 0) {
+    if (!tc::WaitMma(mbar_s, 0, polls) && tid == 0) {
       atomicExch(err, 2);
     }
   } else {

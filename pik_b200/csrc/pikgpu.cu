@@ -36,7 +36,8 @@ enum Class { kC8 = 0, kC16, kC32, kC4, kCSmall, kNumClasses };
 // transform and clamp kernels.
 constexpr int kWorkIdct = kNumClasses, kWorkAr = kNumClasses + 1;
 constexpr int kWorkIdct32 = kNumClasses + 2, kWorkAr32 = kNumClasses + 3;
-constexpr int kNumCounters = kNumClasses + 4;
+constexpr int kEpfRegions = kNumClasses + 4;  // regions in the EPF's list
+constexpr int kNumCounters = kNumClasses + 5;
 // Up to this many small-transform blocks per SM, the small classes run one
 // CTA per block (short latency: one or two waves); above it, one thread per
 // block and channel (throughput).
@@ -105,7 +106,9 @@ struct pikgpu_ctx {
   // device buffers
   DevBuf acs, qf, lut, dq_cf, dq_map, ytox, ytob, table, offsets;
   DevBuf qdc, qac, dc, dcpad, ac, pred2x2_g;
-  DevBuf idct, smoothed, filt, mm, sigma, dc_sigma, list[kNumClasses];
+  DevBuf idct, smoothed, filt, mm, sigma, list[kNumClasses];
+  // Which regions of `filt` the EPF wrote, and their list (k_epf_plan).
+  DevBuf region, region_list;
   DevBuf out_lin, out_rgb8, dbg_dequant, dbg_epf, dbg_pre, guide_ovr, pnm;
   // Linear planes of the last reconstruction (device; NULL if it wrote
   // none), for pikgpu_encode_pnm.
@@ -404,22 +407,19 @@ int UploadTables(pikgpu_ctx* ctx) {
   BuildTables(&t);
   CUDA_TRY(ctx, cudaMemcpyToSymbol(c_t, &t, sizeof(t)));
   CUDA_TRY(ctx, cudaMemcpyToSymbol(g_t, &t, sizeof(t)));
-  CUDA_TRY(ctx, cudaFuncSetAttribute(
-                    k_epf_box<false, 32>,
-                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                    int(EpfSmemBytes(32))));
-  CUDA_TRY(ctx, cudaFuncSetAttribute(
-                    k_epf_box<false, 8>,
-                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                    int(EpfSmemBytes(8))));
-  CUDA_TRY(ctx, cudaFuncSetAttribute(
-                    k_epf_box<true, 16>,
-                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                    int(EpfSmemBytes(16))));
-  CUDA_TRY(ctx, cudaFuncSetAttribute(
-                    k_epf_box<true, 8>,
-                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                    int(EpfSmemBytes(8))));
+  auto epf_smem = [](auto kernel, int th) {
+    return cudaFuncSetAttribute(kernel,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                int(EpfSmemBytes(th)));
+  };
+  CUDA_TRY(ctx, epf_smem(k_epf_box<false, kEpfH, true>, kEpfH));
+  CUDA_TRY(ctx, epf_smem(k_epf_box<false, kEpfH, false>, kEpfH));
+  CUDA_TRY(ctx, epf_smem(k_epf_box<false, 8, true>, 8));
+  CUDA_TRY(ctx, epf_smem(k_epf_box<false, 8, false>, 8));
+  CUDA_TRY(ctx, epf_smem(k_epf_box<true, 16, true>, 16));
+  CUDA_TRY(ctx, epf_smem(k_epf_box<true, 16, false>, 16));
+  CUDA_TRY(ctx, epf_smem(k_epf_box<true, 8, true>, 8));
+  CUDA_TRY(ctx, epf_smem(k_epf_box<true, 8, false>, 8));
   CUDA_TRY(ctx, cudaFuncSetAttribute(
                     k_lf_tile, cudaFuncAttributeMaxDynamicSharedMemorySize,
                     int(kLfSmemBytes)));
@@ -440,6 +440,9 @@ int UploadTables(pikgpu_ctx* ctx) {
 }
 
 inline int Blocks(size_t n, int t) { return int((n + t - 1) / t); }
+inline size_t NumRegions(const Geo& g) {
+  return size_t(Blocks(g.PW, kRegionW)) * Blocks(g.PH, kRegionH);
+}
 
 
 // Writes the smoothed frame (gaborish #1 of the IDCT output) for the stage
@@ -486,8 +489,8 @@ cudaError_t LaunchPdl(bool pdl, void (*kernel)(KArgs...), int grid, int block,
 }
 
 // The frame EPF or the DC EPF: the min/max of the guide source is expected
-// in `mm` already. `sgs`: where the per-block sigma comes from (computed in
-// the kernel); `dco`: the DC image's clamped output instead of `out`.
+// in `mm` already. `work`: the tiles and the blocks' sigma (EpfWork); `dco`:
+// the DC image's clamped output instead of `out`.
 // `gab` > 0: the guide is gaborish (that strength) of `in`, computed inside
 // the kernel.
 // The wait that ran out, from the context's timeout flag: 1 from the
@@ -539,43 +542,43 @@ bool EpfTileMap(CUtensorMap* m, const float* in, int w, int h, int th) {
 // `polls` the first wait's limit; err NULL: no TMA staging.
 void EpfLaunch(cudaStream_t st, int num_sms, int form, const float* in,
                const float* guide_src, int gab, int w, int h,
-               const uint32_t* mm, const EpfSigma& sgs, float* out,
+               const uint32_t* mm, const EpfWork& work, float* out,
                const uint8_t* guide_ovr, const EpfDc& dco, int* err,
                uint32_t polls = tc::kMaxPolls, bool pdl = false) {
   // Images that fill fewer than two CTAs per SM with 32-row tiles (the DC
   // image) take 8-row tiles: four times the CTAs, a quarter of the latency.
   const bool small = Blocks(w, kEpfW) * Blocks(h, kEpfH) < 2 * num_sms;
   const bool fma = form != PIKGPU_FORM_FP32;
-  // One CTA per 64 x th tile.
-  auto grid = [&](int th) { return Blocks(w, kEpfW) * Blocks(h, th); };
   const int th = small ? 8 : fma ? 16 : kEpfH;
   CUtensorMap map;
   memset(&map, 0, sizeof(map));
   const int tma = err && EpfTileMap(&map, in, w, h, th) ? 1 : 0;
+  // A CTA per 64 x th tile (of the frame: as many as the work list may hold).
+  const int grid = Blocks(w, kEpfW) *
+                   (work.list ? Blocks(h, kEpfRegionH) * (kEpfRegionH / th)
+                              : Blocks(h, th));
   // Errors of the launch surface through cudaGetLastError.
-  if (small) {
-    if (fma) {
-      LaunchPdl(pdl, k_epf_box<true, 8>, grid(8), 16 * 8, EpfSmemBytes(8), st,
-                in, guide_src, guide_ovr, gab, w, h, mm, sgs, out, dco, map,
-                tma, err, polls);
-    } else {
-      LaunchPdl(pdl, k_epf_box<false, 8>, grid(8), 16 * 8, EpfSmemBytes(8),
-                st, in, guide_src, guide_ovr, gab, w, h, mm, sgs, out, dco,
-                map, tma, err, polls);
-    }
+  auto launch = [&](auto kernel) {
+    LaunchPdl(pdl, kernel, grid, 16 * th, EpfSmemBytes(th), st, in, guide_src,
+              guide_ovr, gab, w, h, mm, work, out, dco, map, tma, err, polls);
+  };
+  if (work.list) {
+    // 16-row tiles of 256 threads, three CTAs per SM, in the tensor-core
+    // forms: their cx-major loop needs ~85 registers.
+    small ? launch(fma ? k_epf_box<true, 8, true> : k_epf_box<false, 8, true>)
+    : fma ? launch(k_epf_box<true, 16, true>)
+          : launch(k_epf_box<false, kEpfH, true>);
   } else {
-    if (fma) {
-      // 16-row tiles of 256 threads, three CTAs per SM: the cx-major loop
-      // of these forms needs ~85 registers.
-      LaunchPdl(pdl, k_epf_box<true, 16>, grid(16), 16 * 16,
-                EpfSmemBytes(16), st, in, guide_src, guide_ovr, gab, w, h, mm,
-                sgs, out, dco, map, tma, err, polls);
-    } else {
-      LaunchPdl(pdl, k_epf_box<false, kEpfH>, grid(kEpfH), kEpfThreads,
-                kEpfSmemBytes, st, in, guide_src, guide_ovr, gab, w, h, mm,
-                sgs, out, dco, map, tma, err, polls);
-    }
+    small ? launch(fma ? k_epf_box<true, 8, false> : k_epf_box<false, 8, false>)
+    : fma ? launch(k_epf_box<true, 16, false>)
+          : launch(k_epf_box<false, kEpfH, false>);
   }
+}
+
+EpfWork DcEpfWork(const FrameScalars& s) {
+  EpfWork work{};
+  work.dc_qf = s.quant_dc / 2;
+  return work;
 }
 
 // Concurrent branches of the launch sequence. Fork(i, n) makes side streams
@@ -640,7 +643,7 @@ struct ClassChain {
 //   main:   the DCT8 inverse transforms, beside
 //   side 0: the other classes' inverse transforms (ClassChain; the classes'
 //           blocks are disjoint)
-//   main:   gaborish minmax, sigma, EPF
+//   main:   gaborish minmax, the plan (sigma, work lists), EPF
 //   main + side 0: the clamp, split the same way
 //   main:   gaborish #2, opsin, outputs
 //
@@ -692,7 +695,10 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
   ctx->smoothed_valid = false;
   // Both min/max sets and the clamp's block counters start empty.
   int* counters = P<int>(ctx->counters);
-  k_frame_init<<<1, 32, 0, st>>>(mm, counters, kNumCounters); ++ctx->launches;
+  const int nr = s.have_ar ? int(NumRegions(g)) : 0;
+  k_frame_init<<<Blocks(std::max(nr, 32), 256), 256, 0, st>>>(
+      mm, counters, kNumCounters, P<uint32_t>(ctx->region), nr);
+  ++ctx->launches;
   br.Fork(0, 1);
   Mark(ctx, kTDc);
   // DC (side stream 0): dequantisation, the 8-padded copy and its min/max;
@@ -704,14 +710,10 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
   {
     k_dc_prep<<<dim3(Blocks(dpw, 32), Blocks(dph, 8)), 256, 0, sd>>>(
         g, f, s, dcpad, dpw, dph, mm_dc); ++ctx->launches;
-    EpfSigma sgs{};
-    sgs.const_qf = s.quant_dc / 2;
-    sgs.fixed = -1;
-    sgs.out = P<int32_t>(ctx->dc_sigma);
     const EpfDc dco{f.dc, g.Bx, g.By, ctx->dc_half_step[0],
                     ctx->dc_half_step[1], ctx->dc_half_step[2]};
     EpfLaunch(sd, ctx->num_sms, ctx->form, dcpad, dcpad, 0, dpw, dph, mm_dc,
-              sgs, nullptr, nullptr, dco, P<int>(ctx->tc_err), ctx->tc_polls);
+              DcEpfWork(s), nullptr, nullptr, dco, P<int>(ctx->tc_err), ctx->tc_polls);
     ++ctx->launches;
   }
   Mark(ctx, kTDequant);
@@ -809,6 +811,7 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
   }
   br.Join(1, 1);
   const float* final_in = f.idct;
+  const uint32_t* final_region = nullptr;
   Mark(ctx, kTGab1);
   if (s.have_ar) {
     const size_t npx = size_t(g.PW) * g.PH;
@@ -818,9 +821,9 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
     const int gab = s.use_sharpened ? 0 : s.gaborish;
     // The clamp tape starts empty (written by the clamp kernels only).
     if (f.clamp_tape) cudaMemsetAsync(f.clamp_tape, 0, nac, st);
-    // The EPF, and after it the active-block pass, as programmatic
-    // dependents of the kernel before each (LaunchPdl) when nothing else
-    // lies between them on the stream (no per-group events, no stage copy).
+    // The plan, and after it the EPF, as programmatic dependents of the kernel
+    // before each (LaunchPdl) when nothing else lies between them on the
+    // stream (no per-group events).
     const bool pdl = !ctx->profile && !ctx->keep_stages;
     if (gab) {
       const int warps = Blocks(g.PW, 128) * Blocks(g.PH, kGmmRows);
@@ -831,16 +834,33 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
                                                                mm); ++ctx->launches;
     }
     Mark(ctx, kTEpf);
-    int32_t* sig = P<int32_t>(ctx->sigma);
-    EpfSigma sgs{};
-    sgs.ovr = ctx->use_sigma_ovr ? P<int32_t>(ctx->sigma_ovr) : nullptr;
-    sgs.qf = f.qf;
-    sgs.acs = f.acs;
-    sgs.lut = f.lut;
-    sgs.fixed = s.epf_fixed_sigma;
-    sgs.out = sig;
+    // Every cell's sigma, the blocks to clamp per class and the regions to
+    // filter; then the EPF on those regions.
+    EpfPlan plan{};
+    plan.ovr = ctx->use_sigma_ovr ? P<int32_t>(ctx->sigma_ovr) : nullptr;
+    plan.fixed = s.epf_fixed_sigma;
+    plan.keep_all = ctx->keep_stages;
+    plan.sigma = P<int32_t>(ctx->sigma);
+    plan.region = P<uint32_t>(ctx->region);
+    plan.region_list = P<uint32_t>(ctx->region_list);
+    plan.region_count = counters + kEpfRegions;
+    ClassLists cl{};
+    int total = 0;
+    for (int k = 0; k < kNumClasses; ++k) {
+      cl.list[k] = L[k];
+      cl.n[k] = n[k];
+      cl.active[k] = P<uint32_t>(ctx->active[k]);
+      total += n[k];
+    }
+    CUDA_TRY(ctx, LaunchPdl(pdl, k_epf_plan, Blocks(total, 256), 256, 0, st,
+                            g, f, mm, plan, cl, counters));
+    ++ctx->launches;
+    EpfWork work{};
+    work.list = plan.region_list;
+    work.count = plan.region_count;
+    work.sigma = plan.sigma;
     EpfLaunch(st, ctx->num_sms, ctx->form, f.idct, f.idct, gab, g.PW, g.PH,
-              mm, sgs, f.filt,
+              mm, work, f.filt,
               ctx->use_guide_ovr ? P<uint8_t>(ctx->guide_ovr) : nullptr,
               EpfDc{}, P<int>(ctx->tc_err), ctx->tc_polls, pdl);
     ++ctx->launches;
@@ -849,24 +869,8 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
                       cudaMemcpyDeviceToDevice, st);
     }
     Mark(ctx, kTAr);
-    // Only blocks the EPF filtered need the clamp (see k_active_blocks).
-    // Every class's filtered blocks in one pass (main stream), then the
-    // classes' clamps, the ones with few blocks first (see the transforms).
-    {
-      ClassLists cl{};
-      int total = 0;
-      for (int k = 0; k < kNumClasses; ++k) {
-        cl.list[k] = L[k];
-        cl.n[k] = n[k];
-        cl.active[k] = P<uint32_t>(ctx->active[k]);
-        total += n[k];
-      }
-      if (total) {
-        CUDA_TRY(ctx, LaunchPdl(pdl, k_active_blocks, Blocks(total, 256), 256,
-                                0, st, g, sig, f.acs, cl, counters));
-        ++ctx->launches;
-      }
-    }
+    // Only blocks the EPF filtered need the clamp: the classes' clamps, the
+    // ones with few blocks first (see the transforms).
     br.Fork(2, 1);
     if (n[kC8]) {
       k_square_ar_rows<8><<<Blocks(n[kC8], SquareArBlocks<8>()),
@@ -921,6 +925,7 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
     CUDA_TRY(ctx, ch.err);
     br.Join(2, 1);
     final_in = f.filt;
+    final_region = P<uint32_t>(ctx->region);
   } else {
     Mark(ctx, kTEpf);
     Mark(ctx, kTAr);
@@ -933,12 +938,12 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
     float* pre = ctx->keep_stages ? P<float>(ctx->dbg_pre) : nullptr;
     if (s.gaborish) {
       k_final_direct<true><<<Blocks(warps, 8), 256, 0, st>>>(
-          final_in, g.PW, g.PH, g.W, g.H, s.gaborish, pre, lin, lin_stride,
-          vec_lin, rgb8, rgb8_stride);
+          final_in, f.idct, final_region, g.PW, g.PH, g.W, g.H, s.gaborish,
+          pre, lin, lin_stride, vec_lin, rgb8, rgb8_stride);
     } else {
       k_final_direct<false><<<Blocks(warps, 8), 256, 0, st>>>(
-          final_in, g.PW, g.PH, g.W, g.H, 0, pre, lin, lin_stride, vec_lin,
-          rgb8, rgb8_stride);
+          final_in, f.idct, final_region, g.PW, g.PH, g.W, g.H, 0, pre, lin,
+          lin_stride, vec_lin, rgb8, rgb8_stride);
     }
     ++ctx->launches;
   }
@@ -1088,8 +1093,9 @@ int pikgpu_ctx_destroy(pikgpu_ctx* ctx) {
                     &ctx->qdc,     &ctx->qac,       &ctx->dc,
                     &ctx->dcpad,   &ctx->ac,
                     &ctx->pred2x2_g, &ctx->idct,    &ctx->smoothed,
-                    &ctx->filt,    &ctx->mm,        &ctx->sigma,
-                    &ctx->dc_sigma, &ctx->out_lin,  &ctx->out_rgb8,
+                    &ctx->filt,    &ctx->region,    &ctx->region_list, &ctx->mm,
+                    &ctx->sigma,
+                    &ctx->out_lin,  &ctx->out_rgb8,
                     &ctx->dbg_dequant, &ctx->dbg_epf, &ctx->dbg_pre,
                     &ctx->guide_ovr, &ctx->sigma_ovr, &ctx->dq_ovr,
                     &ctx->clamp_scale, &ctx->adj_a,  &ctx->adj_b,
@@ -1236,9 +1242,10 @@ int pikgpu_frame_begin(pikgpu_ctx* ctx, const pikgpu_frame_params* p) {
       {&ctx->pred2x2_g, 4 * kG2GroupFloats * ng},
       {&ctx->idct, 4 * 3 * npx},
       {&ctx->filt, 4 * 3 * npx},
+      {&ctx->region, 4 * NumRegions(g)},
+      {&ctx->region_list, 4 * NumRegions(g)},
       {&ctx->mm, 64},
       {&ctx->sigma, 4 * nb},
-      {&ctx->dc_sigma, 4 * size_t(dpw / 8) * (dph / 8)},
   };
   for (auto& a : allocs) {
     rc = Ensure(ctx, a.b, a.bytes);
@@ -1594,6 +1601,13 @@ int pikgpu_get_stage(pikgpu_ctx* ctx, int stage, float* const planes[3],
       break;
     case PIKGPU_STAGE_AR:
       src = P<float>(ctx->filt), w = g.PW, h = g.PH;
+      if (ctx->s.have_ar) {
+        k_fill_regions<<<Blocks(3 * w * h, 4 * 256), 256, 0, ctx->stream>>>(
+            P<float>(ctx->idct), P<uint32_t>(ctx->region), g.PW, g.PH,
+            P<float>(ctx->filt));
+        CUDA_TRY(ctx, cudaGetLastError());
+        CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+      }
       break;
     case PIKGPU_STAGE_PRE_OPSIN:
       src = P<float>(ctx->dbg_pre), w = g.W, h = g.H;

@@ -230,12 +230,19 @@ __host__ __device__ inline float FromOrderedBits(uint32_t u) {
 #endif
 }
 
+// The regions that the EPF's work is listed in: a region without a filtered
+// block is left out (k_epf_plan, k_epf_box).
+constexpr int kRegionW = 64, kRegionH = 32;
+
 // Start of a frame: the two min/max sets (the frame EPF's at mm[0..5], the
-// DC EPF's at mm[8..13]) reset to empty, and `n` counters to 0.
-__global__ void k_frame_init(uint32_t* mm, int* counters, int n) {
-  const int t = threadIdx.x;
+// DC EPF's at mm[8..13]) reset to empty, and `n` counters and `nr` region
+// flags to 0.
+__global__ void k_frame_init(uint32_t* mm, int* counters, int n,
+                             uint32_t* region, int nr) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < 16) mm[t] = (t & 7) < 3 ? 0xFFFFFFFFu : 0u;
   if (t < n) counters[t] = 0;
+  if (t < nr) region[t] = 0;
 }
 
 __global__ void __launch_bounds__(256)
@@ -334,22 +341,20 @@ __device__ __forceinline__ void GuideParams(const uint32_t* mm, float* all_min,
 }
 
 // SigmaFromQuant (pik/epf_target.cc:1072-1111) of one 8x8 block with raw
-// quant field ac_q, strategy scale (ARQuantScale) and LUT `lut_id`.
-__device__ __forceinline__ int SigmaFromQuant(float ac_q, float scale,
-                                              int lut_id, float stretch) {
+// quant field ac_q, strategy scale (ARQuantScale) and LUT `lut_id`, in two
+// steps: what does not depend on the frame's stretch, and the rest.
+__device__ __forceinline__ float UnscaledSigma(float ac_q, float scale,
+                                               int lut_id) {
   const float quant = ac_q * scale * 0.039324273f;
-  float unscaled;
   const float* l = c_t.sigma_lut[lut_id];
-  if (quant <= 0.022156f) {
-    unscaled = l[0];
-  } else if (quant >= 0.531738f) {
-    unscaled = l[15];
-  } else {
-    const float pos = (quant - 0.022156f) * 29.435892f;
-    const int trunc = int(pos);
-    const float frac = pos - float(trunc);
-    unscaled = frac * l[trunc + 1] + (1.0f - frac) * l[trunc];
-  }
+  if (quant <= 0.022156f) return l[0];
+  if (quant >= 0.531738f) return l[15];
+  const float pos = (quant - 0.022156f) * 29.435892f;
+  const int trunc = int(pos);
+  const float frac = pos - float(trunc);
+  return frac * l[trunc + 1] + (1.0f - frac) * l[trunc];
+}
+__device__ __forceinline__ int ScaledSigma(float unscaled, float stretch) {
   const int sg = int(unscaled * stretch + 0.5182760822018414f);
   return min(sg, kMaxSigma);
 }

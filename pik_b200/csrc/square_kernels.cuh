@@ -160,26 +160,71 @@ __global__ void __launch_bounds__(kSquareThreads)
   }
 }
 
-// Keeps the blocks of each class's list that the EPF filtered (some cell
-// has sigma >= kMinSigma) in that class's active list (counter k); for the
-// others the clamp stage is an exact no-op because the filtered block
-// equals the original. One thread per block of all the classes.
-__global__ void k_active_blocks(Geo g, const int32_t* sigma,
-                                const uint8_t* acs, ClassLists cl,
-                                int* counters) {
-  PdlWait();  // the EPF's sigma
+// What the EPF and the clamp have to do, once the guide's range is known.
+// One thread per block of all the classes:
+//  * the sigma of its cells (SigmaFromQuant): `ovr` (the verification
+//    override) if set; else `fixed` if >= 0 (the fixed-sigma EPF,
+//    pik/epf_target.cc:1342-1386); else from the cell's quant field, strategy
+//    and LUT;
+//  * the block into its class's active list (counter k) if some cell is
+//    filtered (sigma >= kMinSigma); for the others the clamp stage is an
+//    exact no-op because the filtered block equals the original;
+//  * its region (kRegionW x kRegionH pixels; no block crosses one) into the
+//    EPF's list, once, if it is active or every region is kept.
+struct EpfPlan {
+  const int32_t* ovr;
+  int fixed;
+  int keep_all;
+  int32_t* sigma;
+  uint32_t* region;       // 0 / 1 per region
+  uint32_t* region_list;  // the regions set, *region_count of them
+  int* region_count;
+};
+__global__ void __launch_bounds__(256)
+    k_epf_plan(Geo g, DevFrame f, const uint32_t* mm, EpfPlan p,
+               ClassLists cl, int* counters) {
+  PdlLaunchDependents();  // the EPF may start on free SMs
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   int k = 0;
   while (k < kMaxClasses && i >= cl.n[k]) i -= cl.n[k++];
-  bool any = false;
+  const bool on = k < kMaxClasses;
   uint32_t pk = 0;
-  if (k < kMaxClasses) {
+  int cov = 0, cell0 = 0;
+  float scale = 1.0f, most = 0.f;
+  if (on) {
+    // The inputs do not wait for the guide's range, and a sigma grows with
+    // its unscaled value: the largest tells whether the block is filtered.
     pk = cl.list[k][i];
-    const int bx = pk & 0xFFFF, by = pk >> 16;
-    const int cov = Covered(acs[by * g.Bx + bx] >> 4);
+    cell0 = int(pk >> 16) * g.Bx + int(pk & 0xFFFF);
+    const int type = f.acs[cell0] >> 4;
+    cov = Covered(type);
+    scale = ARQuantScaleOf(type);
+    for (int y = 0; y < cov; ++y) {
+      for (int x = 0; x < cov; ++x) {
+        const int cell = cell0 + y * g.Bx + x;
+        most = fmaxf(most,
+                     UnscaledSigma(float(f.qf[cell]), scale, f.lut[cell]));
+      }
+    }
+  }
+  PdlWait();  // the min/max pass
+  float amin, mul, stretch;
+  GuideParams(mm, &amin, &mul, &stretch);
+  bool any = on && (p.fixed >= 0 ? p.fixed : ScaledSigma(most, stretch)) >=
+                       kMinSigma;
+  if (p.ovr) {
+    any = false;
     for (int y = 0; y < cov; ++y)
       for (int x = 0; x < cov; ++x)
-        any |= sigma[(by + y) * g.Bx + bx + x] >= kMinSigma;
+        any |= p.ovr[cell0 + y * g.Bx + x] >= kMinSigma;
+  }
+  const int bx = pk & 0xFFFF, by = pk >> 16;
+  if (on && (any || p.keep_all)) {
+    const int rw = (g.PW + kRegionW - 1) / kRegionW;
+    const int r = by / (kRegionH / 8) * rw + bx / (kRegionW / 8);
+    if (p.region[r] == 0 && atomicExch(&p.region[r], 1u) == 0u) {
+      p.region_list[atomicAdd(p.region_count, 1)] = r;
+    }
   }
   // One atomic per warp and class: the lanes of a class take consecutive
   // slots after the first of them reserves them all.
@@ -193,6 +238,17 @@ __global__ void k_active_blocks(Geo g, const int32_t* sigma,
     base = __shfl_sync(0xFFFFFFFFu, base, leader);
     if (any && k == kk) {
       cl.active[kk][base + __popc(m & ((1u << lane) - 1))] = pk;
+    }
+  }
+  for (int y = 0; y < cov; ++y) {
+    for (int x = 0; x < cov; ++x) {
+      const int cell = cell0 + y * g.Bx + x;
+      p.sigma[cell] =
+          p.ovr          ? p.ovr[cell]
+          : p.fixed >= 0 ? p.fixed
+                         : ScaledSigma(UnscaledSigma(float(f.qf[cell]), scale,
+                                                     f.lut[cell]),
+                                       stretch);
     }
   }
 }
@@ -221,7 +277,7 @@ __device__ __forceinline__ void LoadIntervals(const float* dm, float scale,
 // three channels in one warp instead (three times the registers and a third
 // of the warps) the clamp of a 256x256 frame of 16x16 blocks took 27 us
 // against 9, of a 3840x2160 one 103 against 65. `count` is read from device
-// memory (the compacted list of k_active_blocks).
+// memory (the compacted list of k_epf_plan).
 constexpr int kSquareArGroups = 2;  // warps per channel in a CTA
 constexpr int kSquareArThreads = 96 * kSquareArGroups;
 template <int N>
@@ -476,7 +532,7 @@ __global__ void __launch_bounds__(kSquareThreads)
 // AdaptiveReconstruction clamp of DCT32X32 blocks
 // (pik/adaptive_reconstruction.cc:128-244, 334-471): a CTA per block, four
 // warps per channel; the channels' ratios meet in shared memory. `count` is
-// read from device memory (k_active_blocks).
+// read from device memory (k_epf_plan).
 __global__ void __launch_bounds__(square32::kArThreads, 3)
     k_square32_ar(Geo g, DevFrame f, FrameScalars s, const uint32_t* list,
                   const int* count_ptr) {

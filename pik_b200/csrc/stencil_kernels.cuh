@@ -282,14 +282,28 @@ __device__ __forceinline__ void XybToRgb(float x, float y, float b, float* r,
 // 16-byte loads up front;
 // horizontal neighbours come from the adjacent lanes, lane 0's and the
 // row's last lane's by scalar loads. Coordinates mirror at the padded
-// plane's border (pw x ph). `vec_lin`: the linear outputs may be written as
+// plane's border (pw x ph). `region` (NULL: always `in`): the EPF's region
+// flags; where a region's flag is 0 its pixels are read from `alt` (the
+// EPF's input). `vec_lin`: the linear outputs may be written as
 // float4 (width, stride and base all multiples of 4 floats / 16 bytes).
 // Grid: warps / 8.
 constexpr int kFinRows = 2;
+// Completes the EPF's output planes for the stage export: regions that it
+// left out get its input. One thread per 4 pixels of a plane.
+__global__ void k_fill_regions(const float* in, const uint32_t* region, int w,
+                               int h, float* out) {
+  const size_t o = 4 * (blockIdx.x * size_t(blockDim.x) + threadIdx.x);
+  if (o >= 3 * size_t(w) * h) return;
+  const int x = int(o % w), y = int(o / w % h);
+  const int rw = (w + kRegionW - 1) / kRegionW;
+  if (region[(y / kRegionH) * rw + x / kRegionW]) return;
+  *reinterpret_cast<float4*>(out + o) =
+      *reinterpret_cast<const float4*>(in + o);
+}
 template <bool kGab>
 __global__ void __launch_bounds__(256)
-    k_final_direct(const float* in, int pw, int ph, int w, int h,
-                   int strength, float* pre, float* lin, size_t lin_stride,
+    k_final_direct(const float* in, const float* alt, const uint32_t* region,
+                   int pw, int ph, int w, int h, int strength, float* pre, float* lin, size_t lin_stride,
                    int vec_lin, uint8_t* rgb8, size_t rgb8_stride) {
   constexpr int R = kFinRows, NR = kGab ? R + 2 : R;
   const int lane = threadIdx.x & 31;
@@ -302,21 +316,30 @@ __global__ void __launch_bounds__(256)
   const bool xv = x < pw;
   const bool own_right = lane == 31 || x + 4 >= pw;
   const int xl = MirrorIdx(x0 - 1, pw), xr = MirrorIdx(x + 4, pw);
+  const int rw = (pw + kRegionW - 1) / kRegionW;
   float4 q[3][NR];
   float el[3][NR], er[3][NR];
 #pragma unroll
-  for (int c = 0; c < 3; ++c)
+  for (int r = 0; r < NR; ++r) {
+    const int y = MirrorIdx(kGab ? y0 - 1 + r : y0 + r, ph);
+    // The source planes of column xx.
+    auto src = [&](int xx) {
+      return !region || region[(y / kRegionH) * rw + xx / kRegionW] ? in : alt;
+    };
+    const float* own = (xv ? src(x) : in) + size_t(y) * pw;
+    const float* left = (kGab && lane == 0 ? src(xl) : in) + size_t(y) * pw;
+    const float* right =
+        (kGab && own_right && xv ? src(xr) : in) + size_t(y) * pw;
 #pragma unroll
-    for (int r = 0; r < NR; ++r) {
-      const int y = kGab ? y0 - 1 + r : y0 + r;
-      const float* row = in + c * plane + size_t(MirrorIdx(y, ph)) * pw;
-      q[c][r] = xv ? *reinterpret_cast<const float4*>(row + x)
+    for (int c = 0; c < 3; ++c) {
+      q[c][r] = xv ? *reinterpret_cast<const float4*>(own + c * plane + x)
                    : make_float4(0.f, 0.f, 0.f, 0.f);
       if (kGab) {
-        el[c][r] = lane == 0 ? row[xl] : 0.f;
-        er[c][r] = own_right && xv ? row[xr] : 0.f;
+        el[c][r] = lane == 0 ? left[c * plane + xl] : 0.f;
+        er[c][r] = own_right && xv ? right[c * plane + xr] : 0.f;
       }
     }
+  }
   const float* wt = c_t.gaborish[strength];
   const float w0 = wt[0], w1 = wt[1], w2 = wt[2];
   auto row6 = [&](int c, int r, float v[6]) {

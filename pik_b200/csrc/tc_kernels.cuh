@@ -342,7 +342,7 @@ __device__ __forceinline__ bool Pass1(Smem1<N, S>& s, int j, bool a_mn,
 // 128-244, 334-471): DCT of (filtered - original) for the three channels,
 // the clamp ratio of each coefficient (minimum over X, Y, B) in registers,
 // then the IDCT of the scaled correction added to the original. `count` is
-// read from device memory (the compacted list of k_active_blocks).
+// read from device memory (the compacted list of k_epf_plan).
 // Dynamic shared memory of k_square_ar_tc: its Smem and room to align it
 // to 128 bytes.
 template <int N, int S>
