@@ -170,7 +170,7 @@ int DcNoAlloc(pikgpu_ctx* ctx, const int16_t* quantized_dc, uint32_t bx,
   k_dc_prep<<<dim3(Blocks(dpw, 32), Blocks(dph, 8)), 256, 0, st>>>(
       g, f, s, dcpad, dpw, dph, mm + 8);
   const EpfDc dco{dc, g.Bx, g.By, half_step[0], half_step[1], half_step[2]};
-  EpfLaunch(st, num_sms, PIKGPU_FORM_FP32, dcpad, dcpad, 0, dpw, dph, mm + 8,
+  EpfLaunch(st, num_sms, PIKGPU_FORM_FP32, dcpad, 0, dpw, dph, mm + 8,
             DcEpfWork(s), nullptr, nullptr, dco, /*err=*/nullptr);
   CUDA_TRY(ctx, cudaGetLastError());
   return PIKGPU_OK;

@@ -1,10 +1,10 @@
 // Edge-preserving filter (AdaptiveFilter + WeightedSum,
 // pik/epf_target.cc:526-801, 1113-1278) on packed guide bytes.
 //
-// A CTA filters 64 x TH pixel tiles with 2 TH / 4 warps. Lane l of warp w
-// owns the pixels (x0 + 32 (w mod 2) + l, y0 + 4 (w / 2) + j), j = 0..3: one
-// column (the 32 lanes of a warp read 32 consecutive values of every
-// shared-memory row), four rows inside one 8x8 block row.
+// A CTA filters a 64 x TH pixel tile, a thread ROWS rows of one column: lane
+// l of warp w owns the pixels (x0 + 32 (w mod 2) + l, y0 + ROWS (w / 2) + j),
+// j < ROWS (the 32 lanes of a warp read 32 consecutive values of every
+// shared-memory row; the rows lie inside one 8x8 block row).
 //
 // The u8 guide is staged in shared memory as one 32-bit word per byte
 // offset: word o of a row holds the guide bytes o .. o + 3. The 4 guide bytes
@@ -12,26 +12,28 @@
 // loads of 32 consecutive offsets hit 32 consecutive words, free of bank
 // conflicts), and the sum of absolute differences against the centre
 // pixel's patch row is one __vsadu4. For every displacement (cy, cx) of the 7 x 8 neighbourhood and
-// every channel, a lane forms the 6 patch-row SADs of each of its columns and
-// sums them vertically into the 3 x 4 patch SADs of its 4 rows; the SAD is
+// every channel, a lane forms ROWS + 2 patch-row SADs of its column and
+// sums them vertically into the 3 x 4 patch SADs of its rows; the SAD is
 // the maximum over the channels. The SADs are exact integers; the weights
 // (WeightFast's bit construction) and the weighted sums follow the
 // reference's neighbour order (cy = -3..3, cx = -3..4) with separately
 // rounded products and sums, so the output equals the per-pixel formulation
 // bit for bit.
 //
-// The guide is quantised from one of three sources: the verification
-// override (bytes), a plane (`guide_src`: the sharpened guide, a frame
-// without gaborish, the DC image), or -- the common case -- gaborish of
-// `in` computed here from the staged input tile (the smoothed plane is then
-// never written to memory; `gab` > 0 selects it and its strength).
+// The guide is quantised from the verification override (bytes), or from the
+// staged input tile: its values (the sharpened guide, a frame without
+// gaborish, the DC image) or -- the common case -- gaborish of them (the
+// smoothed plane is then never written to memory; `gab` > 0 selects it and
+// its strength). Border tiles hold mirrored values and take the same steps:
+// 402 -> 380 us at 3001x2003, 22 -> 14 on the DC image of a 256x256 frame,
+// against mirroring every guide byte's coordinates.
 // Included by recon_kernels.cu.
 #pragma once
 
 namespace pikgpu {
 
 constexpr int kEpfW = 64, kEpfH = 32;   // output tile (TH = kEpfH)
-constexpr int kEpfThreads = 16 * kEpfH;  // two warps per 4-row band
+constexpr int kEpfThreads = 16 * kEpfH;  // four rows per thread
 constexpr int kEpfGH = kEpfH + 8;       // guide rows: y0 - 4 .. y0 + 35
 constexpr int kEpfGBytes = 80;          // guide bytes x0 - 8 .. x0 + 71
 constexpr int kEpfGRow = kEpfGBytes;    // words per guide row (one per byte)
@@ -98,27 +100,36 @@ __device__ __forceinline__ uint32_t Sad4(uint32_t a, uint32_t b, uint32_t c) {
   return d;
 }
 
-// The 3-row patch SADs of 4 pixel rows from 6 patch-row pairs (centre row
-// r against window row r): six byte-SADs (rows 1 + 2 and 3 + 4 accumulated
-// onto rows 2 and 3, rows 0 and 5 onto those pairs) and two adds, which
-// need not run on the integer ALU. c0: the first channel (no maximum).
-template <bool c0>
-__device__ __forceinline__ void PatchSads4(const uint32_t* rf,
-                                           const uint32_t* wd, uint32_t* sad) {
-  const uint32_t h2 = Sad4(rf[2], wd[2], 0u);
-  const uint32_t h3 = Sad4(rf[3], wd[3], 0u);
-  const uint32_t p12 = Sad4(rf[1], wd[1], h2);
-  const uint32_t p34 = Sad4(rf[4], wd[4], h3);
-  const uint32_t s0 = Sad4(rf[0], wd[0], p12);
-  const uint32_t s1 = p12 + h3;
-  const uint32_t s2 = p34 + h2;
-  const uint32_t s3 = Sad4(rf[5], wd[5], p34);
-  if (c0) {
-    sad[0] = s0, sad[1] = s1, sad[2] = s2, sad[3] = s3;
+// The 3-row patch SADs of R = 4, 2 or 1 pixel rows from R + 2 patch-row
+// pairs (centre row r against window row r): for four rows six byte-SADs
+// (rows 1 + 2 and 3 + 4 accumulated onto rows 2 and 3, rows 0 and 5 onto
+// those pairs) and two adds, which need not run on the integer ALU. c0: the
+// first channel (no maximum).
+template <bool c0, int R>
+__device__ __forceinline__ void PatchSads(const uint32_t* rf,
+                                          const uint32_t* wd, uint32_t* sad) {
+  uint32_t s[R];
+  if constexpr (R == 4) {
+    const uint32_t h2 = Sad4(rf[2], wd[2], 0u);
+    const uint32_t h3 = Sad4(rf[3], wd[3], 0u);
+    const uint32_t p12 = Sad4(rf[1], wd[1], h2);
+    const uint32_t p34 = Sad4(rf[4], wd[4], h3);
+    s[0] = Sad4(rf[0], wd[0], p12);
+    s[1] = p12 + h3;
+    s[2] = p34 + h2;
+    s[3] = Sad4(rf[5], wd[5], p34);
   } else {
-    sad[0] = max(sad[0], s0), sad[1] = max(sad[1], s1);
-    sad[2] = max(sad[2], s2), sad[3] = max(sad[3], s3);
+    uint32_t p = 0u;  // the rows that all R patches share
+#pragma unroll
+    for (int i = R - 1; i < 3; ++i) p = Sad4(rf[i], wd[i], p);
+    s[0] = p;
+    if constexpr (R == 2) {
+      s[0] = Sad4(rf[0], wd[0], p);
+      s[1] = Sad4(rf[3], wd[3], p);
+    }
   }
+#pragma unroll
+  for (int j = 0; j < R; ++j) sad[j] = c0 ? s[j] : max(sad[j], s[j]);
 }
 
 // The frame EPF's work list, made by k_epf_plan: the regions of kEpfW x
@@ -176,7 +187,7 @@ __device__ __forceinline__ bool EpfInterior(int w, int h, int x0, int y0) {
 // the three planes into `tile` by asynchronous copies: 16 bytes each for
 // interior tiles, 4 bytes per mirrored coordinate at the image border. The
 // caller commits them and waits.
-template <int TH, int NT = 16 * TH>
+template <int TH, int NT>
 __device__ __forceinline__ void EpfStage(const float* in, int w, int h, int x0,
                                          int y0,
                                          float (*tile)[TH + 10][kEpfTS],
@@ -192,62 +203,55 @@ __device__ __forceinline__ void EpfStage(const float* in, int w, int h, int x0,
                 in + c * plane + size_t(y0 - 5 + r) * w + x0 - 12 + 4 * q);
     }
   } else {
-    for (int i = tid; i < 3 * kTH * kEpfTW; i += kThreads) {
-      const int c = i / (kTH * kEpfTW);
-      const int r = (i / kEpfTW) % kTH, col = i % kEpfTW;
-      const int gx = x0 - 12 + col, gy = y0 - 5 + r;
-      CpAsync4(&tile[c][r][col],
-               in + c * plane + size_t(MirrorIdx(gy, h)) * w + MirrorIdx(gx, w));
+    // A row per warp and turn; a lane's columns mirror once.
+    const int lane = tid & 31;
+    int gx[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) gx[i] = MirrorIdx(x0 - 12 + lane + 32 * i, w);
+    for (int cr = tid >> 5; cr < 3 * kTH; cr += kThreads / 32) {
+      const int c = cr / kTH, r = cr - c * kTH;
+      const float* row = in + c * plane + size_t(MirrorIdx(y0 - 5 + r, h)) * w;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const int col = lane + 32 * i;
+        if (col < kEpfTW) CpAsync4(&tile[c][r][col], row + gx[i]);
+      }
     }
   }
 }
 
 // Builds the tile's u8 guide (MakeGuide, pik/epf_target.cc:1009-1070) in
-// shared memory: the aligned words into `sa`, then one word per byte offset
-// into `sg`. NT threads take part (this thread is `tid` of them), and
-// `sync` is their barrier; the tile's copies are complete and published.
-// Returns after the last barrier.
+// shared memory: the aligned words (bytes 4 wd .. 4 wd + 3 of a row) into
+// `sa` (row-major, kEpfAligned words per channel and guide row), then one
+// word per byte offset into `sg`. NT threads take part (this thread is `tid`
+// of them), and `sync` is their barrier; the tile's copies are complete and
+// published. Returns after the last barrier.
+//
+// The guide's position (gy, gx) is the tile's (gy - (y0 - 5), gx - (x0 - 12)),
+// beyond the image's border too, where the tile holds the mirrored values:
+// the smoothed value at a mirrored position has the same pairs of neighbours,
+// and Sym3 adds each pair first.
 template <int TH, int NT, typename Sync>
 __device__ __forceinline__ void EpfBuildGuide(
-    int tid, Sync sync, const float* guide_src, const uint8_t* guide_ovr,
-    int gab, int w, int h, float amin, float mul, uint32_t* sg, uint32_t* sa,
+    int tid, Sync sync, const uint8_t* guide_ovr, int gab, int w, int h,
+    float amin, float mul, uint32_t* sg, uint32_t* sa,
     float (*tile)[TH + 10][kEpfTS], int x0, int y0) {
-  constexpr int kGH = TH + 8, kTH = TH + 10;
-  const size_t plane = size_t(w) * h;
-  const bool interior = EpfInterior<TH>(w, h, x0, y0);
+  constexpr int kGH = TH + 8;
+  constexpr int kAligned = kEpfAligned;
   const float* gw = c_t.gaborish[gab];
   auto quant = [&](float v) {
     return uint32_t(uint8_t(uint32_t(__float2int_rz((v - amin) * mul))));
   };
-  // Gaborish (Sym3 order) at tile position (ly, lx) from the tile.
-  auto smooth = [&](int c, int ly, int lx) {
-    const float* t = &tile[c][ly - 1][lx];
-    const float* m = &tile[c][ly][lx];
-    const float* bt = &tile[c][ly + 1][lx];
-    const float sum_tb = t[0] + bt[0];
-    const float mul0 = m[0] * gw[0];
-    const float sum_lr = m[-1] + m[1];
-    const float x1 = sum_tb + sum_lr;
-    const float mul1 = x1 * gw[1] + mul0;
-    const float sum_t2 = t[-1] + t[1];
-    const float sum_b2 = bt[-1] + bt[1];
-    const float x2 = sum_t2 + sum_b2;
-    return x2 * gw[2] + mul1;
-  };
-  // u8 guide (MakeGuide, pik/epf_target.cc:1009-1070): the aligned words
-  // (bytes 4 wd .. 4 wd + 3 of a row) first, into `sa` (row-major, one
-  // row of kEpfAligned words per channel and guide row).
-  constexpr int kAligned = kEpfAligned;
-  // Interior tiles with the smoothed guide: each thread takes a vertical
-  // strip of kStrip words of one channel and column, with its three input
-  // rows rolling down the strip, so that each input row is loaded once and
-  // its pair sums v[i] + v[i + 2] (Sym3's left/right and corner sums) are
-  // formed once for the three output rows that use them. The arithmetic of
-  // each value is Sym3Rows', in its order.
+  // The smoothed guide: each thread takes a vertical strip of kStrip words of
+  // one channel and column, with its three input rows rolling down the strip,
+  // so that each input row is loaded once and its pair sums v[i] + v[i + 2]
+  // (Sym3's left/right and corner sums) are formed once for the three output
+  // rows that use them. The arithmetic of each value is Sym3Rows', in its
+  // order.
   constexpr int kStrip = (3 * kGH * kAligned + NT - 1) / NT;
   static_assert(kGH % kStrip == 0, "whole strips");
   constexpr int kStrips = kGH / kStrip;
-  const bool strips = interior && !guide_ovr && gab;
+  const bool strips = !guide_ovr && gab;
   if (strips && tid < 3 * kAligned * kStrips) {
     const int wd = tid % kAligned, c = (tid / kAligned) % 3;
     const int r0 = (tid / (3 * kAligned)) * kStrip;
@@ -287,56 +291,22 @@ __device__ __forceinline__ void EpfBuildGuide(
   for (int i = tid; i < 3 * kGH * kAligned && !strips; i += NT) {
     const int cr = i / kAligned, wd = i - cr * kAligned;
     const int c = cr / kGH, r = cr - c * kGH;
-    const int gy = y0 - 4 + r;
     uint32_t word = 0;
-    if (interior && !guide_ovr) {
-      if (gab) {
-        // Four smoothed values from float4 row segments: tile row r + 1,
-        // cols 4 wd + 4 .. 4 wd + 7 (gx = x0 - 8 + 4 wd ..).
-        const int lx = 4 * wd + 4;
-        float v[3][6];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          const float* row = &tile[c][r + k][lx];
-          const float4 q = *reinterpret_cast<const float4*>(row);
-          v[k][0] = row[-1];
-          v[k][1] = q.x, v[k][2] = q.y, v[k][3] = q.z, v[k][4] = q.w;
-          v[k][5] = row[4];
-        }
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          word |= quant(Sym3Rows(v[0], v[1], v[2], b, gw[0], gw[1], gw[2]))
-                  << (8 * b);
-        }
-      } else {
-        const float4 q = *reinterpret_cast<const float4*>(
-            guide_src + c * plane + size_t(gy) * w + x0 - 8 + 4 * wd);
-        word = quant(q.x) | quant(q.y) << 8 | quant(q.z) << 16 |
-               quant(q.w) << 24;
-      }
-    } else {
+    if (guide_ovr) {
+      const int gy = y0 - 4 + r;
       for (int b = 0; b < 4; ++b) {
         const int gx = x0 - 8 + 4 * wd + b;
-        uint32_t v = 0;
-        if (guide_ovr) {
-          const bool ok = gx >= -6 && gx < w + 6 && gy >= -6 && gy < h + 6;
-          v = ok ? guide_ovr[(size_t(c) * (h + 12) + gy + 6) * (w + 12) +
-                             gx + 6]
-                 : 0u;
-        } else if (gab) {
-          // Smoothed value at the mirrored position, from the tile;
-          // positions whose mirror leaves the tile are never read.
-          const int ly = MirrorIdx(gy, h) - (y0 - 5);
-          const int lx = MirrorIdx(gx, w) - (x0 - 12);
-          if (ly >= 1 && ly < kTH - 1 && lx >= 1 && lx < kEpfTW - 1) {
-            v = quant(smooth(c, ly, lx));
-          }
-        } else {
-          v = quant(guide_src[c * plane + size_t(MirrorIdx(gy, h)) * w +
-                              MirrorIdx(gx, w)]);
-        }
+        const bool ok = gx >= -6 && gx < w + 6 && gy >= -6 && gy < h + 6;
+        const uint32_t v =
+            ok ? guide_ovr[(size_t(c) * (h + 12) + gy + 6) * (w + 12) + gx + 6]
+               : 0u;
         word |= v << (8 * b);
       }
+    } else {
+      const float4 q =
+          *reinterpret_cast<const float4*>(&tile[c][r + 1][4 * wd + 4]);
+      word = quant(q.x) | quant(q.y) << 8 | quant(q.z) << 16 |
+             quant(q.w) << 24;
     }
     sa[i] = word;
   }
@@ -352,27 +322,31 @@ __device__ __forceinline__ void EpfBuildGuide(
                    __funnelshift_r(lo, hi, 24));
   }
   sync();
-
 }
 
-// Filters the tile from its staged input and guide (this thread's pixels:
-// `tid` < 16 TH of the tile's filtering threads), with `sig` the sigma of
+// Threads of a 64 x TH tile whose threads own R rows of a column each.
+template <int TH, int R>
+__host__ __device__ constexpr int EpfThreads() {
+  return kEpfW * TH / R;
+}
+
+// Filters the tile from its staged input and guide, with `sig` the sigma of
 // this thread's block, and stores the result. No CTA barrier.
-template <bool kFma, int TH>
+template <bool kFma, int TH, int ROWS>
 __device__ __forceinline__ void EpfFilterCore(
     int tid, int sig, float* out, const EpfDc& dco, int w, int h,
     const uint32_t* sg, float (*tile)[TH + 10][kEpfTS], int x0, int y0) {
   constexpr int kGH = TH + 8;
   constexpr int kGPlane = kGH * kEpfGRow;
   const int lane = tid & 31, wp = tid >> 5;
-  // 4-row band of the warp and its first column (tile-local).
-  const int band = wp >> 1, col0 = 32 * (wp & 1);
+  // The warp's rows and its first column (tile-local).
+  const int row0 = ROWS * (wp >> 1), col0 = 32 * (wp & 1);
   const size_t plane = size_t(w) * h;
-  const int px = x0 + lane + col0, py0 = y0 + 4 * band;
+  const int px = x0 + lane + col0, py0 = y0 + row0;
   const bool inside = px < w && py0 < h;  // w and h are multiples of 8
   const bool filtered = sig >= kMinSigma;
   // Tile position of the pixel (px, py0).
-  const int tr0 = 4 * band + 3 + kEpfTRow0, tc0 = lane + col0 + 3 + kEpfTCol0;
+  const int tr0 = row0 + 3 + kEpfTRow0, tc0 = lane + col0 + 3 + kEpfTCol0;
 
   // Warps (half a block row of 8 blocks) without filtered blocks copy.
   if (!__any_sync(0xFFFFFFFFu, filtered)) {
@@ -380,7 +354,7 @@ __device__ __forceinline__ void EpfFilterCore(
 #pragma unroll
       for (int c = 0; c < 3; ++c)
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < ROWS; ++j)
           EpfStore(out, dco, plane, w, c, px, py0 + j, tile[c][tr0 + j][tc0]);
     }
     return;
@@ -388,66 +362,66 @@ __device__ __forceinline__ void EpfFilterCore(
   const int m64 = c_t.mul_table[filtered ? sig : kMinSigma] * 64;
   const EpfCut cut = EpfCutOf(filtered ? sig : kMinSigma, m64);
 
-  // Centre patch rows: guide rows py0 - 1 .. py0 + 4, bytes px - 1 .. px + 2
+  // Centre patch rows: guide rows py0 - 1 .. py0 + ROWS, bytes px - 1 .. px + 2
   // (byte offset of px - 1 from x0 - 8).
-  const int gr0 = 4 * band + 3;  // guide smem row of py0 - 1
+  const int gr0 = row0 + 3;  // guide smem row of py0 - 1
   const int gc0 = lane + col0 + 7;
-  float ws[3][4], sw[4];
+  float ws[3][ROWS], sw[ROWS];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
+  for (int j = 0; j < ROWS; ++j) {
     ws[0][j] = ws[1][j] = ws[2][j] = 0.f;
     sw[j] = 0.f;
   }
   if constexpr (kFma) {
     // Tensor-core forms: cx outermost. For one cx the 7 vertical offsets
-    // read 12 distinct guide rows per channel (one load each), and each
-    // staged input row serves every pixel of the lane it reaches: about
-    // 84 shared-memory loads per cx and lane instead of 210. Each pixel's
+    // read ROWS + 8 distinct guide rows per channel (one load each), and
+    // each staged input row serves every pixel of the lane it reaches: for
+    // four rows about 84 shared-memory loads per cx and lane instead of 210. Each pixel's
     // sums run cx-major, not in the reference's cy-major order (these
     // forms are not bound to its rounding).
 #pragma unroll 1
     for (int cx = -3; cx <= 4; ++cx) {
       const uint32_t* g = sg + (gr0 - 3) * kEpfGRow + gc0 + cx;
-      uint32_t sad[7][4];
+      uint32_t sad[7][ROWS];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        uint32_t wd[12];  // guide rows gr0 - 3 .. gr0 + 8 at this cx
+        uint32_t wd[ROWS + 8];  // guide rows gr0 - 3 .. at this cx
 #pragma unroll
-        for (int t = 0; t < 12; ++t) wd[t] = g[c * kGPlane + t * kEpfGRow];
+        for (int t = 0; t < ROWS + 8; ++t) wd[t] = g[c * kGPlane + t * kEpfGRow];
         // The centre patch words again from shared memory (registers are
         // the limit).
-        uint32_t rf[6];
+        uint32_t rf[ROWS + 2];
 #pragma unroll
-        for (int r = 0; r < 6; ++r) {
+        for (int r = 0; r < ROWS + 2; ++r) {
           rf[r] = sg[c * kGPlane + (gr0 + r) * kEpfGRow + gc0];
         }
 #pragma unroll
-        for (int k = 0; k < 7; ++k) {  // cy = k - 3: rows k .. k + 5
+        for (int k = 0; k < 7; ++k) {  // cy = k - 3: rows k ..
           if (c == 0) {
-            PatchSads4<true>(rf, wd + k, sad[k]);
+            PatchSads<true, ROWS>(rf, wd + k, sad[k]);
           } else {
-            PatchSads4<false>(rf, wd + k, sad[k]);
+            PatchSads<false, ROWS>(rf, wd + k, sad[k]);
           }
         }
       }
-      float wt[4][7];
+      float wt[ROWS][7];
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
+      for (int j = 0; j < ROWS; ++j)
 #pragma unroll
         for (int k = 0; k < 7; ++k) {
           const float wgt = EpfCutWeight(m64, cut, sad[k][j]);
           wt[j][k] = wgt;
           sw[j] += wgt;
         }
-      // Input rows band + R - 3 (R = j + cy + 3 = 0..9) at column px + cx.
+      // Input rows R - 3 (R = j + cy + 3) at column px + cx.
       const int col = tc0 + cx;
 #pragma unroll
-      for (int R = 0; R < 10; ++R) {
+      for (int R = 0; R < ROWS + 6; ++R) {
         const int ir = tr0 - 3 + R;
         const float v0 = tile[0][ir][col], v1 = tile[1][ir][col],
                     v2 = tile[2][ir][col];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < ROWS; ++j) {
           const int k = R - j;  // cy + 3
           if (k < 0 || k > 6) continue;
           ws[0][j] = fmaf(v0, wt[j][k], ws[0][j]);
@@ -458,33 +432,33 @@ __device__ __forceinline__ void EpfFilterCore(
     }
   } else {
     // The reference's order: cy-major, products and sums rounded separately.
-    uint32_t ref[3][6];
+    uint32_t ref[3][ROWS + 2];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
-      for (int r = 0; r < 6; ++r)
+      for (int r = 0; r < ROWS + 2; ++r)
         ref[c][r] = sg[c * kGPlane + (gr0 + r) * kEpfGRow + gc0];
 #pragma unroll 1
     for (int cy = -3; cy <= 3; ++cy) {
-#pragma unroll 1
+#pragma unroll(ROWS == 4 ? 1 : 4)
       for (int cx = -3; cx <= 4; ++cx) {
         // Window byte offset: the patch start moved by cx.
         const uint32_t* g = sg + (gr0 + cy) * kEpfGRow + gc0 + cx;
-        uint32_t sad[4];
+        uint32_t sad[ROWS];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          uint32_t wd[6];
+          uint32_t wd[ROWS + 2];
 #pragma unroll
-          for (int r = 0; r < 6; ++r) wd[r] = g[c * kGPlane + r * kEpfGRow];
+          for (int r = 0; r < ROWS + 2; ++r) wd[r] = g[c * kGPlane + r * kEpfGRow];
           if (c == 0) {
-            PatchSads4<true>(ref[c], wd, sad);
+            PatchSads<true, ROWS>(ref[c], wd, sad);
           } else {
-            PatchSads4<false>(ref[c], wd, sad);
+            PatchSads<false, ROWS>(ref[c], wd, sad);
           }
         }
         const int col = tc0 + cx;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < ROWS; ++j) {
           const int ir = tr0 + j + cy;
           const float wgt = EpfCutWeight(m64, cut, sad[j]);
           ws[0][j] += tile[0][ir][col] * wgt;
@@ -499,13 +473,13 @@ __device__ __forceinline__ void EpfFilterCore(
   // The normalisation: an IEEE division in the FP32 form (the reference's
   // rounding); in the tensor-core forms one reciprocal per row (the weight
   // sum is in [1, 56]) and a multiply per channel, within 2 ulp.
-  float inv[4];
+  float inv[ROWS];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) inv[j] = kFma ? __frcp_rn(sw[j]) : 0.f;
+  for (int j = 0; j < ROWS; ++j) inv[j] = kFma ? __frcp_rn(sw[j]) : 0.f;
 #pragma unroll
   for (int c = 0; c < 3; ++c)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < ROWS; ++j) {
       const float v = kFma ? ws[c][j] * inv[j] : ws[c][j] / sw[j];
       EpfStore(out, dco, plane, w, c, px, py0 + j,
                filtered ? v : tile[c][tr0 + j][tc0]);
@@ -522,34 +496,20 @@ __device__ __forceinline__ void EpfFilterCore(
 // kFma: the weighted sums with fused multiply-adds (the tensor-core forms,
 // which are not bound to the reference's rounding); otherwise every product
 // and sum is rounded separately, as the reference does.
-template <bool kFma, int TH>
+template <bool kFma, int TH, int ROWS>
 __device__ __forceinline__ void EpfFilterTile(
-    const float* guide_src, const uint8_t* guide_ovr, int gab, int w, int h,
-    float amin, float mul, int sig, float* out, const EpfDc& dco,
-    uint32_t* sg, uint32_t* sa, float (*tile)[TH + 10][kEpfTS], int x0,
-    int y0) {
+    const uint8_t* guide_ovr, int gab, int w, int h, float amin, float mul,
+    int sig, float* out, const EpfDc& dco, uint32_t* sg, uint32_t* sa,
+    float (*tile)[TH + 10][kEpfTS], int x0, int y0) {
   const int tid = threadIdx.x;
-  // Tiles without filtered blocks are copies (CopyOriginalBlock).
-  if (!__syncthreads_or(sig >= kMinSigma)) {
-    const int lane = tid & 31, wp = tid >> 5;
-    const int band = wp >> 1, col0 = 32 * (wp & 1);
-    const size_t plane = size_t(w) * h;
-    const int px = x0 + lane + col0, py0 = y0 + 4 * band;
-    const int tr0 = 4 * band + 3 + kEpfTRow0;
-    const int tc0 = lane + col0 + 3 + kEpfTCol0;
-    if (px < w && py0 < h) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          EpfStore(out, dco, plane, w, c, px, py0 + j, tile[c][tr0 + j][tc0]);
-    }
-    return;
+  // Tiles without filtered blocks are copies (CopyOriginalBlock): every warp
+  // copies, and no guide is needed.
+  if (__syncthreads_or(sig >= kMinSigma)) {
+    EpfBuildGuide<TH, EpfThreads<TH, ROWS>()>(tid, [] { __syncthreads(); },
+                                              guide_ovr, gab, w, h, amin, mul,
+                                              sg, sa, tile, x0, y0);
   }
-  EpfBuildGuide<TH, 16 * TH>(tid, [] { __syncthreads(); }, guide_src,
-                             guide_ovr, gab, w, h, amin, mul, sg, sa, tile,
-                             x0, y0);
-  EpfFilterCore<kFma, TH>(tid, sig, out, dco, w, h, sg, tile, x0, y0);
+  EpfFilterCore<kFma, TH, ROWS>(tid, sig, out, dco, w, h, sg, tile, x0, y0);
 }
 
 // One CTA per 64 x TH tile (1-D grid). More CTAs than resident slots balance
@@ -574,10 +534,9 @@ __device__ __forceinline__ void EpfFilterTile(
 // *err = 2 (the host reports the frame as failed) and waits once more,
 // bounded, so that no copy is in flight when the CTA exits. Border tiles,
 // and all tiles without a tensor map, are staged with cp.async (EpfStage).
-template <bool kFma, int TH, bool kList>
-__global__ void __launch_bounds__(16 * TH, TH == 16 ? 3 : 2)
-    k_epf_box(const float* in, const float* guide_src,
-              const uint8_t* guide_ovr, int gab, int w, int h,
+template <bool kFma, int TH, int ROWS, bool kList>
+__global__ void __launch_bounds__(EpfThreads<TH, ROWS>(), TH == 16 ? 3 : 2)
+    k_epf_box(const float* in, const uint8_t* guide_ovr, int gab, int w, int h,
               const uint32_t* mm, EpfWork work, float* out, EpfDc dco,
               const __grid_constant__ CUtensorMap tmap, int use_tma,
               int* err, uint32_t polls) {
@@ -624,12 +583,13 @@ __global__ void __launch_bounds__(16 * TH, TH == 16 ? 3 : 2)
           : "memory");
     }
   } else {
-    EpfStage<TH>(in, w, h, x0, y0, tile, tid);
+    EpfStage<TH, EpfThreads<TH, ROWS>()>(in, w, h, x0, y0, tile, tid);
   }
   float amin, mul, stretch;
   GuideParams(mm, &amin, &mul, &stretch);
   int sig = 0;
-  const int px = x0 + lane + 32 * ((tid >> 5) & 1), py = y0 + 4 * (tid >> 6);
+  const int px = x0 + lane + 32 * ((tid >> 5) & 1);
+  const int py = y0 + ROWS * (tid >> 6);
   if (px < w && py < h) {
     sig = kList ? work.sigma[(py >> 3) * (w / 8) + (px >> 3)]
                 : ScaledSigma(UnscaledSigma(float(work.dc_qf), 1.0f, 0),
@@ -644,8 +604,8 @@ __global__ void __launch_bounds__(16 * TH, TH == 16 ? 3 : 2)
   } else {
     CpAsyncWaitAll();
   }
-  EpfFilterTile<kFma, TH>(guide_src, guide_ovr, gab, w, h, amin, mul, sig,
-                          out, dco, sg, sa, tile, x0, y0);
+  EpfFilterTile<kFma, TH, ROWS>(guide_ovr, gab, w, h, amin, mul, sig, out, dco,
+                                sg, sa, tile, x0, y0);
 }
 
 }  // namespace pikgpu

@@ -400,6 +400,32 @@ void ComputeScalars(const pikgpu_frame_params* p, FrameScalars* s) {
   s->epf_fixed_sigma = p->epf_enable_adaptive ? -1 : int(p->epf_sigma);
 }
 
+// Calls fn with the EPF kernel of a form, tile height, rows per thread and
+// kind of work. The tensor-core forms' 16-row tiles have 256 threads, three
+// CTAs per SM: their cx-major loop needs ~85 registers.
+template <typename Fn>
+void ForEpfKernel(bool fma, int th, int rows, bool list, Fn&& fn) {
+  auto pick = [&](auto r) {
+    constexpr int R = decltype(r)::value;
+    if (list) {
+      fma ? fn(k_epf_box<true, 8, R, true>) : fn(k_epf_box<false, 8, R, true>);
+    } else {
+      fma ? fn(k_epf_box<true, 8, R, false>)
+          : fn(k_epf_box<false, 8, R, false>);
+    }
+  };
+  if (th == 8) {
+    rows == 1 ? pick(std::integral_constant<int, 1>())
+              : pick(std::integral_constant<int, 2>());
+  } else if (list) {
+    fma ? fn(k_epf_box<true, 16, 4, true>)
+        : fn(k_epf_box<false, kEpfH, 4, true>);
+  } else {
+    fma ? fn(k_epf_box<true, 16, 4, false>)
+        : fn(k_epf_box<false, kEpfH, 4, false>);
+  }
+}
+
 int UploadTables(pikgpu_ctx* ctx) {
   std::lock_guard<std::mutex> lock(g_table_mutex);
   if (ctx->device < 64 && g_tables_uploaded[ctx->device]) return PIKGPU_OK;
@@ -407,19 +433,18 @@ int UploadTables(pikgpu_ctx* ctx) {
   BuildTables(&t);
   CUDA_TRY(ctx, cudaMemcpyToSymbol(c_t, &t, sizeof(t)));
   CUDA_TRY(ctx, cudaMemcpyToSymbol(g_t, &t, sizeof(t)));
-  auto epf_smem = [](auto kernel, int th) {
-    return cudaFuncSetAttribute(kernel,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                int(EpfSmemBytes(th)));
-  };
-  CUDA_TRY(ctx, epf_smem(k_epf_box<false, kEpfH, true>, kEpfH));
-  CUDA_TRY(ctx, epf_smem(k_epf_box<false, kEpfH, false>, kEpfH));
-  CUDA_TRY(ctx, epf_smem(k_epf_box<false, 8, true>, 8));
-  CUDA_TRY(ctx, epf_smem(k_epf_box<false, 8, false>, 8));
-  CUDA_TRY(ctx, epf_smem(k_epf_box<true, 16, true>, 16));
-  CUDA_TRY(ctx, epf_smem(k_epf_box<true, 16, false>, 16));
-  CUDA_TRY(ctx, epf_smem(k_epf_box<true, 8, true>, 8));
-  CUDA_TRY(ctx, epf_smem(k_epf_box<true, 8, false>, 8));
+  for (int i = 0; i < 12; ++i) {  // every EPF kernel
+    const bool fma = i & 1, list = i & 2;
+    const int rows = i < 4 ? 1 : i < 8 ? 2 : 4;
+    const int th = rows < 4 ? 8 : fma ? 16 : kEpfH;
+    cudaError_t e = cudaSuccess;
+    ForEpfKernel(fma, th, rows, list, [&](auto kernel) {
+      e = cudaFuncSetAttribute(kernel,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               int(EpfSmemBytes(th)));
+    });
+    CUDA_TRY(ctx, e);
+  }
   CUDA_TRY(ctx, cudaFuncSetAttribute(
                     k_lf_tile, cudaFuncAttributeMaxDynamicSharedMemorySize,
                     int(kLfSmemBytes)));
@@ -541,14 +566,19 @@ bool EpfTileMap(CUtensorMap* m, const float* in, int w, int h, int th) {
 // `err`: the context's wait-timeout flag (k_epf_box's TMA wait sets 2),
 // `polls` the first wait's limit; err NULL: no TMA staging.
 void EpfLaunch(cudaStream_t st, int num_sms, int form, const float* in,
-               const float* guide_src, int gab, int w, int h,
-               const uint32_t* mm, const EpfWork& work, float* out,
+               int gab, int w, int h, const uint32_t* mm, const EpfWork& work, float* out,
                const uint8_t* guide_ovr, const EpfDc& dco, int* err,
                uint32_t polls = tc::kMaxPolls, bool pdl = false) {
   // Images that fill fewer than two CTAs per SM with 32-row tiles (the DC
-  // image) take 8-row tiles: four times the CTAs, a quarter of the latency.
-  const bool small = Blocks(w, kEpfW) * Blocks(h, kEpfH) < 2 * num_sms;
+  // image, small frames) take 8-row tiles with fewer rows per thread: more
+  // CTAs and threads, a shorter chain in each. With 8-row tiles of four rows
+  // per thread the DC EPF of a 4K frame took 33 us (FP32; 29 split-BF16),
+  // with one row 19 (16); on a 1030x530 frame two rows took 25 us, four 31,
+  // one 29; up to 5 CTAs per SM instead of 2 made 1600x900 5% slower.
   const bool fma = form != PIKGPU_FORM_FP32;
+  const bool small = Blocks(w, kEpfW) * Blocks(h, kEpfH) < 2 * num_sms;
+  const int tiles8 = Blocks(w, kEpfW) * Blocks(h, 8);
+  const int rows = !small ? 4 : tiles8 <= 2 * num_sms ? 1 : 2;
   const int th = small ? 8 : fma ? 16 : kEpfH;
   CUtensorMap map;
   memset(&map, 0, sizeof(map));
@@ -558,21 +588,10 @@ void EpfLaunch(cudaStream_t st, int num_sms, int form, const float* in,
                    (work.list ? Blocks(h, kEpfRegionH) * (kEpfRegionH / th)
                               : Blocks(h, th));
   // Errors of the launch surface through cudaGetLastError.
-  auto launch = [&](auto kernel) {
-    LaunchPdl(pdl, kernel, grid, 16 * th, EpfSmemBytes(th), st, in, guide_src,
+  ForEpfKernel(fma, th, rows, work.list != nullptr, [&](auto kernel) {
+    LaunchPdl(pdl, kernel, grid, kEpfW * th / rows, EpfSmemBytes(th), st, in,
               guide_ovr, gab, w, h, mm, work, out, dco, map, tma, err, polls);
-  };
-  if (work.list) {
-    // 16-row tiles of 256 threads, three CTAs per SM, in the tensor-core
-    // forms: their cx-major loop needs ~85 registers.
-    small ? launch(fma ? k_epf_box<true, 8, true> : k_epf_box<false, 8, true>)
-    : fma ? launch(k_epf_box<true, 16, true>)
-          : launch(k_epf_box<false, kEpfH, true>);
-  } else {
-    small ? launch(fma ? k_epf_box<true, 8, false> : k_epf_box<false, 8, false>)
-    : fma ? launch(k_epf_box<true, 16, false>)
-          : launch(k_epf_box<false, kEpfH, false>);
-  }
+  });
 }
 
 EpfWork DcEpfWork(const FrameScalars& s) {
@@ -712,7 +731,7 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
         g, f, s, dcpad, dpw, dph, mm_dc); ++ctx->launches;
     const EpfDc dco{f.dc, g.Bx, g.By, ctx->dc_half_step[0],
                     ctx->dc_half_step[1], ctx->dc_half_step[2]};
-    EpfLaunch(sd, ctx->num_sms, ctx->form, dcpad, dcpad, 0, dpw, dph, mm_dc,
+    EpfLaunch(sd, ctx->num_sms, ctx->form, dcpad, 0, dpw, dph, mm_dc,
               DcEpfWork(s), nullptr, nullptr, dco, P<int>(ctx->tc_err), ctx->tc_polls);
     ++ctx->launches;
   }
@@ -859,7 +878,7 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
     work.list = plan.region_list;
     work.count = plan.region_count;
     work.sigma = plan.sigma;
-    EpfLaunch(st, ctx->num_sms, ctx->form, f.idct, f.idct, gab, g.PW, g.PH,
+    EpfLaunch(st, ctx->num_sms, ctx->form, f.idct, gab, g.PW, g.PH,
               mm, work, f.filt,
               ctx->use_guide_ovr ? P<uint8_t>(ctx->guide_ovr) : nullptr,
               EpfDc{}, P<int>(ctx->tc_err), ctx->tc_polls, pdl);

@@ -30,7 +30,8 @@ def patched(w, h, seed, pattern):
 
 @pytest.mark.parametrize("pattern", ["none", "checker", "one cell", "right",
                                      "all"])
-@pytest.mark.parametrize("size", [(64, 32), (72, 40), (203, 101), (600, 264)])
+@pytest.mark.parametrize("size", [(64, 32), (72, 40), (203, 101), (600, 264),
+                                  (1030, 300)])
 def test_partly_filtered_frames_bitexact(size, pattern):
     frame = patched(*size, 7, pattern)
     want = oraclepy.run(frame, precision=32, want=("ar", "linear", "srgb8"),
@@ -59,4 +60,24 @@ def test_region_list_follows_the_frame():
         lin, _ = ctx.reconstruct()
         want = oraclepy.run(frame, precision=32, want=("linear",))
         np.testing.assert_array_equal(lin, want["linear"])
+    ctx.close()
+
+
+@pytest.mark.parametrize("gaborish,sharpened", [(2, 1), (0, 0), (4, 0)])
+@pytest.mark.parametrize("size", [(8, 8), (13, 70), (139, 77), (1030, 300)])
+def test_guide_sources_bitexact(size, gaborish, sharpened):
+    """The guide from the staged tile, smoothed or not, beyond the border of
+    images narrower than a tile's halo too."""
+    frame = dataclasses.replace(patched(*size, 9, "all"), gaborish=gaborish,
+                                epf_use_sharpened=sharpened)
+    want = oraclepy.run(frame, precision=32, want=("linear",),
+                        export_decisions=True)
+    ctx = native.Context(0)
+    ctx.begin(frame)
+    ctx.set_ac()
+    lin, _ = ctx.reconstruct()
+    guide, sigma = ctx.decisions()
+    np.testing.assert_array_equal(guide, want["guide"])
+    np.testing.assert_array_equal(sigma, want["sigma"])
+    np.testing.assert_array_equal(lin, want["linear"])
     ctx.close()
