@@ -916,8 +916,9 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
       // Four blocks per batch; two CTAs per SM (256 tensor-memory columns
       // each); three BF16 terms in both tensor-core forms (see the
       // transforms).
-      const int grid = std::min((n[kC32] + 3) / 4, ctx->num_sms * 2);
-      ch(k_square_ar_tc<32, 3>, grid, tc::kThreads, ArTcSmemBytes<32, 3>(),
+      const int grid = std::min((n[kC32] + 3) / 4,
+                                ctx->num_sms * tc::ArCtasPerSm<32>());
+      ch(k_square_ar_tc<32, 3>, grid, tc::kArThreads, ArTcSmemBytes<32, 3>(),
          g, f, s, P<uint32_t>(ctx->active[kC32]), counters + kC32,
          counters + kWorkAr32, P<int>(ctx->tc_err));
     } else if (n[kC32]) {
@@ -925,14 +926,14 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
          P<uint32_t>(ctx->active[kC32]), counters + kC32);
     }
     if (n[kC16] && ctx->form != PIKGPU_FORM_FP32) {
-      const int grid =
-          std::min((n[kC16] + 7) / 8, ctx->num_sms * ctx->tc_ctas_per_sm);
+      const int per_sm = std::min(ctx->tc_ctas_per_sm, tc::ArCtasPerSm<16>());
+      const int grid = std::min((n[kC16] + 7) / 8, ctx->num_sms * per_sm);
       if (ctx->form == PIKGPU_FORM_SPLIT_BF16) {
-        ch(k_square_ar_tc<16, 2>, grid, tc::kThreads, ArTcSmemBytes<16, 2>(),
+        ch(k_square_ar_tc<16, 2>, grid, tc::kArThreads, ArTcSmemBytes<16, 2>(),
            g, f, s, P<uint32_t>(ctx->active[kC16]), counters + kC16,
            counters + kWorkAr, P<int>(ctx->tc_err));
       } else {
-        ch(k_square_ar_tc<16, 3>, grid, tc::kThreads, ArTcSmemBytes<16, 3>(),
+        ch(k_square_ar_tc<16, 3>, grid, tc::kArThreads, ArTcSmemBytes<16, 3>(),
            g, f, s, P<uint32_t>(ctx->active[kC16]), counters + kC16,
            counters + kWorkAr, P<int>(ctx->tc_err));
       }

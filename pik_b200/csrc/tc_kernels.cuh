@@ -151,6 +151,62 @@ __device__ __forceinline__ void PutRowK(uint8_t* base, int m, const float* v) {
   }
 }
 
+// The 128 rows of a batch in units of four values, N / 4 units per row: unit
+// u of row u / (N / 4). The planes are read and written by units, a thread
+// the units t, t + 128, ..., so that a warp's 16-byte accesses cover whole
+// rows of its blocks; a row per lane touches 32 rows with every access, and
+// that traffic through the L1 bound these kernels (75% of its throughput).
+template <int N>
+__device__ __forceinline__ int UnitRow(int t, int j) {
+  return (t + kThreads * j) / (N / 4);
+}
+template <int N>
+__device__ __forceinline__ int UnitCol(int t) {  // first column
+  return 4 * (t % (N / 4));
+}
+// Values k .. k + 3 of row m of a K-major operand (k a multiple of 4).
+template <int N, int S>
+__device__ __forceinline__ void PutUnitK(uint8_t* base, int m, int k,
+                                         const float4& v) {
+  float rest[4] = {v.x, v.y, v.z, v.w};
+  const uint32_t off = (m >> 3) * (N / 8) * 128 + (k >> 3) * 128 +
+                       (m & 7) * 16 + (k & 4) * 2;
+#pragma unroll
+  for (int t = 0; t < S; ++t) {
+    uint32_t w[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const __nv_bfloat162 h =
+          __floats2bfloat162_rn(rest[2 * i], rest[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&h);
+      if (t + 1 < S) {
+        const float2 b = __bfloat1622float2(h);
+        rest[2 * i] -= b.x;
+        rest[2 * i + 1] -= b.y;
+      }
+    }
+    *reinterpret_cast<uint2*>(base + t * (128 * N * 2) + off) =
+        make_uint2(w[0], w[1]);
+  }
+}
+// The batch's output rows in shared memory (128 x N floats): written a row
+// per thread, read by units. The units of a row are permuted so that neither
+// has bank conflicts.
+template <int N>
+__device__ __forceinline__ float4* OutUnit(uint8_t* base, int m, int q) {
+  const int p = N == 16 ? q ^ ((m >> 1) & 3) : q ^ (m & 7);
+  return reinterpret_cast<float4*>(base) + m * (N / 4) + p;
+}
+template <int N>
+__device__ __forceinline__ void PutOutRow(uint8_t* base, int m,
+                                          const float (&v)[N]) {
+#pragma unroll
+  for (int q = 0; q < N / 4; ++q) {
+    *OutUnit<N>(base, m, q) =
+        make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+  }
+}
+
 // Column k of an M-major operand for rows m0 .. m0 + N - 1: v[i] is element
 // (m0 + i, k); m0 is a multiple of 8.
 template <int N, int S>
@@ -174,9 +230,15 @@ struct Smem {
   alignas(128) uint8_t a[3][S * kOpBytes];
   alignas(128) uint8_t idct[S * kMatBytes];
   alignas(128) uint8_t dct[S * kMatBytes];
-  alignas(8) uint64_t mbar;
+  alignas(8) uint64_t mbar[3];
   uint32_t tmem;
 };
+constexpr int kArThreads = 3 * kThreads;  // a group of four warps per channel
+
+// Barrier of channel c's four warps.
+__device__ __forceinline__ void ChannelSync(int c) {
+  asm volatile("bar.sync %0, %1;" ::"r"(c + 1), "r"(kThreads) : "memory");
+}
 
 // Tensor-memory column of channel c's accumulator j (0 or 1).
 template <int N>
@@ -184,18 +246,18 @@ __device__ __forceinline__ uint32_t AccCol(int c, int j) {
   return uint32_t(c * 2 * N + j * N);
 }
 
-// One split-BF16 GEMM pass for the three channels: D(c, j) = A(c) * B^T over
-// K = N, then waits for it. Called by all threads after writing their rows
-// of the A operands.
+// One split-BF16 GEMM pass of channel c: D(c, j) = A(c) * B^T over K = N,
+// then waits for it. Called by the channel's threads (t = 0 .. 127 of them)
+// after writing their rows of the A operand.
 template <int N, int S>
-__device__ __forceinline__ bool Pass(Smem<N, S>& s, int j, bool a_mn,
-                                     const uint8_t* b, uint32_t& phase,
-                                     uint32_t polls) {
+__device__ __forceinline__ bool Pass(Smem<N, S>& s, int c, int t, int j,
+                                     bool a_mn, const uint8_t* b,
+                                     uint32_t phase, uint32_t polls) {
   using Sm = Smem<N, S>;
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   FenceBefore();
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  ChannelSync(c);
+  if (t == 0) {
     FenceAfter();
     const uint32_t idesc = Idesc(128, N, a_mn ? 1 : 0);
     constexpr uint32_t sbo = (N / 8) * 128;
@@ -204,48 +266,50 @@ __device__ __forceinline__ bool Pass(Smem<N, S>& s, int j, bool a_mn,
     constexpr int kPairs = S == 2 ? 3 : 6;
     constexpr int pi[6] = {0, 0, 1, 0, 2, 1};
     constexpr int pk[6] = {0, 1, 0, 2, 0, 1};
+    const uint32_t d = s.tmem + AccCol<N>(c, j);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const uint32_t d = s.tmem + AccCol<N>(c, j);
+    for (int kk = 0; kk < N / 16; ++kk) {
 #pragma unroll
-      for (int kk = 0; kk < N / 16; ++kk) {
-#pragma unroll
-        for (int p = 0; p < kPairs; ++p) {
-          Mma(d, Desc(s.a[c] + pi[p] * Sm::kOpBytes + kk * 256, 128, sbo),
-              Desc(b + pk[p] * Sm::kMatBytes + kk * 256, 128, sbo), idesc,
-              (kk > 0 || p > 0) ? 1u : 0u);
-        }
+      for (int p = 0; p < kPairs; ++p) {
+        Mma(d, Desc(s.a[c] + pi[p] * Sm::kOpBytes + kk * 256, 128, sbo),
+            Desc(b + pk[p] * Sm::kMatBytes + kk * 256, 128, sbo), idesc,
+            (kk > 0 || p > 0) ? 1u : 0u);
       }
     }
     asm volatile(
         "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster."
-        "b64 [%0];" ::"r"(SmemU32(&s.mbar))
+        "b64 [%0];" ::"r"(SmemU32(&s.mbar[c]))
         : "memory");
   }
-  const bool ok = WaitMma(SmemU32(&s.mbar), phase, polls);
-  phase ^= 1u;
+  const bool ok = WaitMma(SmemU32(&s.mbar[c]), phase, polls);
   FenceAfter();
   return ok;
+}
+
+// CTAs of the clamp that an SM holds, by registers.
+template <int N>
+__host__ __device__ constexpr int ArCtasPerSm() {
+  return N == 16 ? 3 : 2;
 }
 
 // This thread's row of D (N FP32 columns from dcol).
 template <int N, int S>
 __device__ __forceinline__ void LoadRow(const Smem<N, S>& s, uint32_t dcol,
                                         float* v) {
-  const uint32_t lane_base = (threadIdx.x & ~31u) << 16;
+  const uint32_t lane_base = (threadIdx.x & 96u) << 16;
 #pragma unroll
   for (int c = 0; c < N; c += 16) Ld16(s.tmem + lane_base + dcol + c, v + c);
 }
 
-// Transform matrix (row-major n x k in constant memory) as a K-major BF16
-// hi/lo B operand.
+// Transform matrix (row-major n x k, 16-byte aligned in global memory) as a
+// K-major BF16 split B operand.
 template <int N, int S>
 __device__ __forceinline__ void PutMatrix(uint8_t* base, const float* m) {
-  for (int i = threadIdx.x; i < N * N / 8; i += kThreads) {
+  for (int i = threadIdx.x; i < N * N / 8; i += blockDim.x) {
     const int n = i / (N / 8), kc = i % (N / 8);
-    float v[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = m[n * N + kc * 8 + e];
+    const float4 a = *reinterpret_cast<const float4*>(m + 8 * i);
+    const float4 b = *reinterpret_cast<const float4*>(m + 8 * i + 4);
+    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
     PutChunk<S>(base, N * N * 2,
                 (n >> 3) * (N / 8) * 128 + kc * 128 + (n & 7) * 16, v);
   }
@@ -269,6 +333,8 @@ struct Smem1 {
   alignas(128) uint8_t idct[S * kMatBytes];
   // HF prediction: each block's window of cell values.
   float win[128 / N][HfWin<N>() * HfWin<N>()];
+  // ... and the corner of its transform.
+  alignas(16) float corner[128 / N][N / 4 * N / 4];
   alignas(8) uint64_t mbar;
   uint32_t tmem;
 };
@@ -285,7 +351,7 @@ __host__ __device__ constexpr int TmemCols3() {
 // The HF corner table of an N x N block: 2 cov rows of HfWin<N>() taps.
 template <int N>
 __device__ __forceinline__ const float* HfCorner() {
-  return N == 16 ? &c_t.hf_corner16[0][0] : &c_t.hf_corner32[0][0];
+  return N == 16 ? &g_t.hf_corner16[0][0] : &g_t.hf_corner32[0][0];
 }
 
 // This thread's row of D (N FP32 columns from dcol).
@@ -339,10 +405,16 @@ __device__ __forceinline__ bool Pass1(Smem1<N, S>& s, int j, bool a_mn,
 
 // AdaptiveReconstruction clamp for square DCT blocks on the tensor cores
 // (split-BF16 form of k_square_ar_rows, pik/adaptive_reconstruction.cc:
-// 128-244, 334-471): DCT of (filtered - original) for the three channels,
-// the clamp ratio of each coefficient (minimum over X, Y, B) in registers,
-// then the IDCT of the scaled correction added to the original. `count` is
-// read from device memory (the compacted list of k_epf_plan).
+// 128-244, 334-471): DCT of (filtered - original), the clamp ratio of each
+// coefficient (minimum over X, Y, B), then the IDCT of the scaled correction
+// added to the original. Four warps per channel, with an MMA chain and an
+// mbarrier of their own; the channels' ratios meet in shared memory. With
+// four warps for the three channels, and planes read and written a row per
+// lane, the clamp of 32x32 blocks took 42 us on a 256x256 frame and 350 on a
+// 3840x2160 one (of 16x16 blocks 20 and 55); with a group per channel 29 and
+// 257 (13 and 63), and with accesses by units (UnitRow) 25 and 198 (13 and
+// 47). `count` is read from device memory (the compacted list of
+// k_epf_plan).
 // Dynamic shared memory of k_square_ar_tc: its Smem and room to align it
 // to 128 bytes.
 template <int N, int S>
@@ -351,7 +423,7 @@ constexpr size_t ArTcSmemBytes() {
 }
 
 template <int N, int S>
-__global__ void __launch_bounds__(tc::kThreads, N == 16 ? 4 : 2)
+__global__ void __launch_bounds__(tc::kArThreads, tc::ArCtasPerSm<N>())
     k_square_ar_tc(Geo g, DevFrame f, FrameScalars sc, const uint32_t* list,
                    const int* count_ptr, int* work, int* err) {
   PdlLaunchDependents();
@@ -364,7 +436,9 @@ __global__ void __launch_bounds__(tc::kThreads, N == 16 ? 4 : 2)
   Smem<N, S>& s = *reinterpret_cast<Smem<N, S>*>(
       (reinterpret_cast<uintptr_t>(ar_tc_smem) + 127) & ~uintptr_t(127));
   __shared__ int s_next[2];
-  const int t = threadIdx.x, bl = t / N, r = t % N;
+  // Thread t of channel c's group holds row r of block bl.
+  const int c = threadIdx.x / kThreads, t = threadIdx.x % kThreads;
+  const int bl = t / N, r = t % N;
   const int count = *count_ptr;
   const int nbat = (count + BPB - 1) / BPB;
   // Batches are taken from a work counter, one at a time: a CTA that
@@ -372,39 +446,46 @@ __global__ void __launch_bounds__(tc::kThreads, N == 16 ? 4 : 2)
   // first is taken before the set-up, which a CTA without work skips (the
   // grid is sized for all of the class's blocks, the active ones are
   // counted on the device). The next batch is fetched at the start of a
-  // batch and read after the batch's last barrier.
-  if (t == 0) s_next[0] = atomicAdd(work, 1);
+  // batch and read after the ratios' barrier; the channels go on to it on
+  // their own.
+  if (threadIdx.x == 0) s_next[0] = atomicAdd(work, 1);
   __syncthreads();
   int batch = s_next[0];
   if (batch >= nbat) return;
-  if (t < 32) {
+  if (threadIdx.x < 32) {
     asm volatile(
         "tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::
             "r"(SmemU32(&s.tmem)),
         "r"(kCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
-  if (t == 0) {
+  if (threadIdx.x < 3) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(
-        SmemU32(&s.mbar)));
+        SmemU32(&s.mbar[threadIdx.x])));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  PutMatrix<N, S>(s.idct, c_t.idct + MatOffset(N));
-  PutMatrix<N, S>(s.dct, c_t.dct + MatOffset(N));
+  PutMatrix<N, S>(s.idct, g_t.idct + MatOffset(N));
+  PutMatrix<N, S>(s.dct, g_t.dct + MatOffset(N));
   FenceBefore();
   __syncthreads();
   FenceAfter();
-  uint32_t phase = 0;
   const size_t plane = size_t(g.PW) * g.PH;
   const float inv_nn = 1.0f / float(N * N);
+  const float mul_dc = c == 0   ? sc.mul_dc[0]
+                       : c == 1 ? sc.mul_dc[1]
+                                : sc.mul_dc[2];
+  // The channels' clamp ratios, coefficient-major: a channel's A operand is
+  // free between its second and third pass.
+  auto ratio = [&](int ch) { return reinterpret_cast<float*>(s.a[ch]); };
+  static_assert(sizeof(s.a[0]) >= sizeof(float) * N * kThreads,
+                "the ratios fit an operand");
   bool ok = true;
-  for (int k = 1; batch < nbat && ok; ++k) {
-    if (t == 0) s_next[k & 1] = atomicAdd(work, 1);
+  for (int k = 1; batch < nbat; ++k) {
+    if (threadIdx.x == 0) s_next[k & 1] = atomicAdd(work, 1);
     const int idx = batch * BPB + bl;
     const bool active = idx < count;
     const uint32_t pkd = list[active ? idx : 0];
     const int bx = pkd & 0xFFFF, by = pkd >> 16;
-    const size_t row0 = size_t(by * 8 + r) * g.PW + bx * 8;
     // The block's clamp intervals (a chain of dependent table loads) are
     // looked up first, so that the loads resolve during the DCT passes. The
     // class holds only blocks of one type.
@@ -415,120 +496,119 @@ __global__ void __launch_bounds__(tc::kThreads, N == 16 ? 4 : 2)
         ClampInvQuantAc(g, f, sc.inv_global_scale, bx, by, qac);
     const int cf = f.dq_cf[(by >> 3) * g.Tx + (bx >> 3)];
     const int table = f.dq_map[cf * 256 + (qac - 1)];
-    uint32_t dm_off[3];
+    const float* dm =
+        f.table + f.offsets[(table * 7 + QuantKindOf(type)) * 3 + c] + r * N;
+    // The place of unit j in the planes (the first block's for rows past the
+    // last block, which are not written).
+    auto unit = [&](int j, bool* on) {
+      const int m = UnitRow<N>(t, j), i = batch * BPB + m / N;
+      *on = i < count;
+      const uint32_t pk = list[i < count ? i : 0];
+      return c * plane + size_t(int(pk >> 16) * 8 + m % N) * g.PW +
+             (pk & 0xFFFF) * 8 + UnitCol<N>(t);
+    };
+    // The correction, filtered - original.
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      dm_off[c] = f.offsets[(table * 7 + QuantKindOf(type)) * 3 + c] + r * N;
+    for (int j = 0; j < N / 4; ++j) {
+      bool on;
+      const size_t at = unit(j, &on);
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (on) {
+        a = *reinterpret_cast<const float4*>(f.filt + at);
+        const float4 o = *reinterpret_cast<const float4*>(f.idct + at);
+        a = make_float4(a.x - o.x, a.y - o.y, a.z - o.z, a.w - o.w);
+      }
+      PutUnitK<N, S>(s.a[c], UnitRow<N>(t, j), UnitCol<N>(t), a);
     }
     float T[N];
+    ok = Pass<N, S>(s, c, t, 0, false, s.dct, 0, f.tc_polls) && ok;
+    LoadRow<N, S>(s, AccCol<N>(c, 0), T);  // t_y[k]
+    PutColMN<N, S>(s.a[c], N * bl, r, T);
+    ok = Pass<N, S>(s, c, t, 1, true, s.dct, 1, f.tc_polls) && ok;
+    LoadRow<N, S>(s, AccCol<N>(c, 1), T);  // coefficient row k = r
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-#pragma unroll
-      for (int x = 0; x < N; x += 4) {
-        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), o = a;
-        if (active) {
-          a = *reinterpret_cast<const float4*>(f.filt + c * plane + row0 + x);
-          o = *reinterpret_cast<const float4*>(f.idct + c * plane + row0 + x);
-        }
-        T[x] = a.x - o.x, T[x + 1] = a.y - o.y;
-        T[x + 2] = a.z - o.z, T[x + 3] = a.w - o.w;
-      }
-      PutRowK<N, S>(s.a[c], t, T);  // pixel row y = r of the correction
-    }
-    ok = Pass<N, S>(s, 0, false, s.dct, phase, f.tc_polls);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      LoadRow<N, S>(s, AccCol<N>(c, 0), T);  // t_y[k]
-      PutColMN<N, S>(s.a[c], N * bl, r, T);
-    }
-    ok = Pass<N, S>(s, 1, true, s.dct, phase, f.tc_polls) && ok;
-    float Y[3][N];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      LoadRow<N, S>(s, AccCol<N>(c, 1), Y[c]);  // coefficient row k = r
-#pragma unroll
-      for (int l = 0; l < N; ++l) Y[c][l] *= inv_nn;
-    }
-    // Clamp ratios of coefficient row k = r, minimum over the channels.
+    for (int l = 0; l < N; ++l) T[l] *= inv_nn;
+    // This channel's clamp ratios of coefficient row k = r, then the minimum
+    // over the channels.
     {
-      const float* dm[3];
-      bool dm_vec = true;  // rows 16-byte aligned: float4 loads
+      const bool vec = (reinterpret_cast<uintptr_t>(dm) & 15) == 0;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        dm[c] = f.table + dm_off[c];
-        dm_vec = dm_vec && (reinterpret_cast<uintptr_t>(dm[c]) & 15) == 0;
-      }
-      const size_t tape_row = CoefOffset(g, bx, by, cov, r * N);
-      uint8_t* tape =
-          f.clamp_tape && active ? f.clamp_tape + tape_row : nullptr;
-      const uint8_t* tin =
-          f.clamp_tape_in && active ? f.clamp_tape_in + tape_row : nullptr;
-      float dq[3][4];  // dm[c][l0 .. l0 + 3]
+      for (int l0 = 0; l0 < N; l0 += 4) {
+        float iv[4];
+        if (vec) {  // 16-byte aligned rows
+          const float4 q = *reinterpret_cast<const float4*>(dm + l0);
+          iv[0] = q.x, iv[1] = q.y, iv[2] = q.z, iv[3] = q.w;
+        } else {
 #pragma unroll
-      for (int l = 0; l < N; ++l) {
-        if ((l & 3) == 0) {
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            if (dm_vec) {
-              const float4 q = *reinterpret_cast<const float4*>(dm[c] + l);
-              dq[c][0] = q.x, dq[c][1] = q.y, dq[c][2] = q.z, dq[c][3] = q.w;
-            } else {
-#pragma unroll
-              for (int e = 0; e < 4; ++e) dq[c][e] = dm[c][l + e];
-            }
-          }
+          for (int e = 0; e < 4; ++e) iv[e] = dm[l0 + e];
         }
-        const bool llf = r < cov && l < cov;
-        const float ls = llf ? LlfScale(type, l, r) : 0.f;
-        float mr = 1.0f, rt[3];
-        int arg = -1;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          rt[c] = ClampRatio(
-              Y[c][l], llf ? ls * sc.mul_dc[c] : dq[c][l & 3] * inv_quant_ac);
-          if (rt[c] < mr) mr = rt[c], arg = c;
+        for (int e = 0; e < 4; ++e) {
+          const int l = l0 + e;
+          const bool llf = r < cov && l < cov;
+          const float interval =
+              llf ? LlfScale(type, l, r) * mul_dc : iv[e] * inv_quant_ac;
+          ratio(c)[l * kThreads + t] = ClampRatio(T[l], interval);
         }
-        uint8_t code = arg < 0 ? 0 : mr == 0.0f ? 4 : uint8_t(arg + 1);
-        if (tin) {
-          code = tin[l];
-          mr = TapeRatio(code, rt[0], rt[1], rt[2]);
-        }
-        if (tape) tape[l] = code;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) Y[c][l] = Y[c][l] * mr;
       }
     }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) PutRowK<N, S>(s.a[c], t, Y[c]);
-    ok = Pass<N, S>(s, 0, false, s.idct, phase, f.tc_polls) && ok;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      LoadRow<N, S>(s, AccCol<N>(c, 0), T);
-      PutColMN<N, S>(s.a[c], N * bl, r, T);
+    // A wait that ran out in any channel ends the CTA's work.
+    if (__syncthreads_or(!ok)) {
+      ok = false;
+      break;
     }
-    ok = Pass<N, S>(s, 1, true, s.idct, phase, f.tc_polls) && ok;
-    ok = __syncthreads_and(ok);
     const int next = s_next[k & 1];
+    const size_t tape_row = CoefOffset(g, bx, by, cov, r * N);
+    uint8_t* tape =
+        f.clamp_tape && active && c == 0 ? f.clamp_tape + tape_row : nullptr;
+    const uint8_t* tin =
+        f.clamp_tape_in && active ? f.clamp_tape_in + tape_row : nullptr;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      LoadRow<N, S>(s, AccCol<N>(c, 1), T);  // pixel row v = r
-      if (active && ok) {
+    for (int l = 0; l < N; ++l) {
+      const float rt0 = ratio(0)[l * kThreads + t],
+                  rt1 = ratio(1)[l * kThreads + t],
+                  rt2 = ratio(2)[l * kThreads + t];
+      float mr = 1.0f;
+      int arg = -1;
+      if (rt0 < mr) mr = rt0, arg = 0;
+      if (rt1 < mr) mr = rt1, arg = 1;
+      if (rt2 < mr) mr = rt2, arg = 2;
+      uint8_t code = arg < 0 ? 0 : mr == 0.0f ? 4 : uint8_t(arg + 1);
+      if (tin) {
+        code = tin[l];
+        mr = TapeRatio(code, rt0, rt1, rt2);
+      }
+      if (tape) tape[l] = code;
+      T[l] = T[l] * mr;
+    }
+    __syncthreads();  // the ratios are read: their operands may be written
+    PutRowK<N, S>(s.a[c], t, T);
+    ok = Pass<N, S>(s, c, t, 0, false, s.idct, 0, f.tc_polls) && ok;
+    LoadRow<N, S>(s, AccCol<N>(c, 0), T);
+    PutColMN<N, S>(s.a[c], N * bl, r, T);
+    ok = Pass<N, S>(s, c, t, 1, true, s.idct, 1, f.tc_polls) && ok;
+    LoadRow<N, S>(s, AccCol<N>(c, 1), T);  // pixel row v = r
+    PutOutRow<N>(s.a[c], t, T);
+    ChannelSync(c);
 #pragma unroll
-        for (int x = 0; x < N; x += 4) {
-          const float4 o =
-              *reinterpret_cast<const float4*>(f.idct + c * plane + row0 + x);
-          *reinterpret_cast<float4*>(f.filt + c * plane + row0 + x) =
-              make_float4(T[x] + o.x, T[x + 1] + o.y, T[x + 2] + o.z,
-                          T[x + 3] + o.w);
-        }
+    for (int j = 0; j < N / 4; ++j) {
+      bool on;
+      const size_t at = unit(j, &on);
+      if (on && ok) {
+        const float4 v =
+            *OutUnit<N>(s.a[c], UnitRow<N>(t, j), UnitCol<N>(t) / 4);
+        const float4 o = *reinterpret_cast<const float4*>(f.idct + at);
+        *reinterpret_cast<float4*>(f.filt + at) =
+            make_float4(v.x + o.x, v.y + o.y, v.z + o.z, v.w + o.w);
       }
     }
+    ChannelSync(c);  // the operand may be written again
     batch = next;
   }
   if (!ok && t == 0) atomicExch(err, 1);
   FenceBefore();
   __syncthreads();
-  if (t < 32) {
+  if (threadIdx.x < 32) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(
                      s.tmem),
                  "r"(kCols));
@@ -537,12 +617,14 @@ __global__ void __launch_bounds__(tc::kThreads, N == 16 ? 4 : 2)
 
 // HF prediction + AddBlockExceptLFAndLLFTo + IDCT for 16x16 and 32x32 DCT
 // blocks on the tensor cores (split-BF16 form of k_square_idct_rows and
-// k_square_idct). Persistent CTAs of 128 threads; an item is one channel
+// k_square32_idct). Persistent CTAs of 128 threads; an item is one channel
 // of a batch of 128 / N blocks ((batch, channel) pairs, batch-major; the
 // channels of a block are independent here). A thread holds one row of one
 // channel, so several CTAs share an SM (eight for N = 16, four for
-// N = 32), each with its own MMA round trips; the next item's coefficient
-// row is loaded while this item's passes run.
+// N = 32), each with its own MMA round trips; the next item's coefficients
+// are loaded while this item's passes run. Reading and writing the planes by
+// units (UnitRow) instead of a row per lane: 74 -> 62 us on a 3840x2160 frame
+// of 16x16 blocks, 423 -> 367 at 8192x8192.
 template <int N, int S>
 __global__ void __launch_bounds__(tc::kThreads, N == 16 ? 8 : 4)
     k_square_idct_tc1(Geo g, DevFrame f, const uint32_t* list, int count,
@@ -585,7 +667,7 @@ __global__ void __launch_bounds__(tc::kThreads, N == 16 ? 8 : 4)
         SmemU32(&s.mbar)));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  PutMatrix<N, S>(s.idct, c_t.idct + MatOffset(N));
+  PutMatrix<N, S>(s.idct, g_t.idct + MatOffset(N));
   FenceBefore();
   __syncthreads();
   FenceAfter();
@@ -593,35 +675,44 @@ __global__ void __launch_bounds__(tc::kThreads, N == 16 ? 8 : 4)
   const size_t plane_ac = size_t(g.ac_stride) * g.By;
   const size_t plane_px = size_t(g.PW) * g.PH;
   const float inv_nn = 1.0f / float(N * N);
-  // This lane's row of the HF corner table (rows r < 2 cov).
+  // A block's lanes share the (2 cov)^2 values of its HF corner, LV each: row
+  // (r LV) / (2 cov), from column (r LV) % (2 cov) on. Its rows of the corner
+  // table:
+  constexpr int LV = 4 * cov * cov / N;
   const float* ctab = HfCorner<N>();
-  float cr[W];
+  float cr[W], cl[LV][W];
 #pragma unroll
-  for (int m = 0; m < W; ++m) cr[m] = ctab[(r & (2 * cov - 1)) * W + m];
-  bool ok = true;
-  // The next item's coefficient row is loaded while this item's passes
-  // run (the CTAs of an SM otherwise wait for their loads in step).
-  float X[N];
-  auto load_row = [&](int it) {
-    const int bt = it / 3, ch = it - 3 * bt;
-    const int i = bt * BPB + bl;
-    const uint32_t pk = list[i < count ? i : 0];
-    const float* crow = f.ac + ch * plane_ac +
-                        CoefRowOffset(g, pk & 0xFFFF, pk >> 16, N, r);
+  for (int i = 0; i < W; ++i) {
+    cr[i] = ctab[(r * LV / (2 * cov)) * W + i];
 #pragma unroll
-    for (int j = 0; j < N; j += 4) {
-      const float4 v = i < count ? *reinterpret_cast<const float4*>(crow + j)
-                                 : make_float4(0.f, 0.f, 0.f, 0.f);
-      X[j] = v.x, X[j + 1] = v.y, X[j + 2] = v.z, X[j + 3] = v.w;
+    for (int l = 0; l < LV; ++l) {
+      cl[l][i] = ctab[((r * LV) % (2 * cov) + l) * W + i];
     }
-    return pk;
+  }
+  bool ok = true;
+  // The next item's coefficients are loaded while this item's passes run
+  // (the CTAs of an SM otherwise wait for their loads in step).
+  float4 X[N / 4];
+  auto load = [&](int it) {
+    const int bt = it / 3, ch = it - 3 * bt;
+#pragma unroll
+    for (int j = 0; j < N / 4; ++j) {
+      const int m = UnitRow<N>(t, j), i = bt * BPB + m / N;
+      X[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i < count) {
+        const uint32_t pk = list[i];
+        X[j] = *reinterpret_cast<const float4*>(
+            f.ac + ch * plane_ac +
+            CoefRowOffset(g, pk & 0xFFFF, pk >> 16, N, m % N) + UnitCol<N>(t));
+      }
+    }
   };
-  uint32_t pkd_next = item < nitems ? load_row(item) : 0u;
+  load(item);
   for (int k = 0; item < nitems && ok; ++k) {
     const int batch = item / 3, c = item - 3 * batch;
     const int idx = batch * BPB + bl;
     const bool active = idx < count;
-    const uint32_t pkd = pkd_next;
+    const uint32_t pkd = list[active ? idx : 0];
     const int bx = pkd & 0xFFFF, by = pkd >> 16;
     // HF prediction: adding the predicted coefficients outside the
     // 2cov x 2cov corner and transforming back equals transforming the
@@ -629,11 +720,11 @@ __global__ void __launch_bounds__(tc::kThreads, N == 16 ? 8 : 4)
     // = P). The upsampled prediction P of this pixel row is the 3-tap
     // vertical blend of three rows of the 2x2-cell grid (W columns), then
     // the 3-tap horizontal blend; its DCT corner is C Pred C^T over the
-    // block's W x W cell window (C = HfCorner<N>), of which lanes
-    // r < 2 cov subtract row r. The class holds only DCT16X16 (DCT32X32)
-    // blocks, which predict HF. The block's N lanes first stage its cell
-    // window in shared memory (a few loads per lane instead of tens of
-    // scalar loads of cells that the lanes share).
+    // block's W x W cell window (C = HfCorner<N>). The class holds only DCT16X16
+    // (DCT32X32) blocks, which predict HF. The block's N lanes first stage
+    // its cell window in shared memory (a few loads per lane instead of tens
+    // of scalar loads of cells that the lanes share) and share the corner's
+    // values; the threads that hold its units subtract them.
     float P[N];
     const bool hf = active && predict_hf;
     if (predict_hf) {
@@ -663,49 +754,67 @@ __global__ void __launch_bounds__(tc::kThreads, N == 16 ? 8 : 4)
         P[x] = fmaf(col[q + 2], c_t.ub4[2][ix],
                     fmaf(col[q + 1], c_t.ub4[1][ix], col[q] * c_t.ub4[0][ix]));
       }
-      if (r < 2 * cov) {
-        float u[W];
+    }
+    if (predict_hf) {
+      // This thread's values (row, l0 .. l0 + LV - 1) of the corner.
+      const float* w = s.win[bl];
+      float u[W];
 #pragma unroll
-        for (int rho = 0; rho < W; ++rho) {
-          float a = 0.f;
+      for (int rho = 0; rho < W; ++rho) {
+        float a = 0.f;
 #pragma unroll
-          for (int m = 0; m < W; ++m) a = fmaf(w[rho * W + m], cr[m], a);
-          u[rho] = a;
-        }
+        for (int i = 0; i < W; ++i) a = fmaf(w[rho * W + i], cr[i], a);
+        u[rho] = a;
+      }
 #pragma unroll
-        for (int l = 0; l < 2 * cov; ++l) {
-          float v = 0.f;
+      for (int l = 0; l < LV; ++l) {
+        float v = 0.f;
 #pragma unroll
-          for (int rho = 0; rho < W; ++rho) {
-            v = fmaf(ctab[l * W + rho], u[rho], v);
-          }
-          X[l] -= v * inv_nn;
+        for (int rho = 0; rho < W; ++rho) v = fmaf(cl[l][rho], u[rho], v);
+        s.corner[bl][r * LV + l] = hf ? v * inv_nn : 0.f;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < N / 4; ++j) {
+        const int m = UnitRow<N>(t, j), row = m % N, l0 = UnitCol<N>(t);
+        if (row < 2 * cov && l0 < 2 * cov) {
+          const float4 v = *reinterpret_cast<const float4*>(
+              &s.corner[m / N][row * 2 * cov + l0]);
+          X[j].x -= v.x, X[j].y -= v.y, X[j].z -= v.z, X[j].w -= v.w;
         }
       }
     }
     float T[N];
-    PutRowK<N, S>(s.a, t, X);
-    if (item_next < nitems) pkd_next = load_row(item_next);
+#pragma unroll
+    for (int j = 0; j < N / 4; ++j) {
+      PutUnitK<N, S>(s.a, UnitRow<N>(t, j), UnitCol<N>(t), X[j]);
+    }
+    if (item_next < nitems) load(item_next);
     if (t == 0) s_next[k & 1] = atomicAdd(work, 1);
     ok = Pass1<N, S>(s, 0, false, s.idct, phase, f.tc_polls) && ok;
     const int item_after = s_next[k & 1];
     LoadRow1<N, S>(s, 0, T);  // T[k = r][v]
     PutColMN<N, S>(s.a, N * bl, r, T);
     ok = Pass1<N, S>(s, 1, true, s.idct, phase, f.tc_polls) && ok;
-    ok = __syncthreads_and(ok);
     LoadRow1<N, S>(s, N, T);  // pixel row v = r
     if (hf) {
 #pragma unroll
       for (int i = 0; i < N; ++i) T[i] += P[i];
     }
-    if (active && ok) {
-      float* out = f.idct + c * plane_px + size_t(by * 8 + r) * g.PW + bx * 8;
+    PutOutRow<N>(s.a, t, T);
+    __syncthreads();
 #pragma unroll
-      for (int i = 0; i < N; i += 4) {
-        *reinterpret_cast<float4*>(out + i) =
-            make_float4(T[i], T[i + 1], T[i + 2], T[i + 3]);
+    for (int j = 0; j < N / 4; ++j) {
+      const int m = UnitRow<N>(t, j), i = batch * BPB + m / N;
+      if (i < count && ok) {
+        const uint32_t pk = list[i];
+        *reinterpret_cast<float4*>(
+            f.idct + c * plane_px + size_t(int(pk >> 16) * 8 + m % N) * g.PW +
+            (pk & 0xFFFF) * 8 + UnitCol<N>(t)) =
+            *OutUnit<N>(s.a, m, UnitCol<N>(t) / 4);
       }
     }
+    ok = __syncthreads_and(ok);  // the operand may be written again
     item = item_next;
     item_next = item_after;
   }
