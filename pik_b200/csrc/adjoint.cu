@@ -1130,14 +1130,8 @@ int pikgpu_adjoint(pikgpu_ctx* ctx, const float* target, double* loss,
                       sizeof(double), kind, st));
   }
   CUDA_TRY(ctx, cudaStreamSynchronize(st));
-  {
-    int code = 0;
-    CUDA_TRY(ctx, cudaMemcpy(&code, ctx->tc_err.p, sizeof(int),
-                             cudaMemcpyDeviceToHost));
-    if (code) {
-      cudaMemset(ctx->tc_err.p, 0, sizeof(int));
-      return Fail(ctx, PIKGPU_ERR_CUDA, "%s", WaitTimeoutMessage(code));
-    }
+  if (const int code = TakeTimeout(ctx)) {
+    return Fail(ctx, PIKGPU_ERR_CUDA, "%s", WaitTimeoutMessage(code));
   }
   ctx->have_result = true;
   return PIKGPU_OK;

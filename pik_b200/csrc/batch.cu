@@ -28,19 +28,8 @@ struct pikgpu_batch {
   int chains = 0;  // 0: one branch per frame
   int tc_ctas = kTcCtasPerSm;
   bool exec_valid_for_shape = false;  // the graph was captured with these
-  // The frames' wait-timeout flags, gathered (and cleared) by one kernel
-  // after each replay and read back with one copy.
-  int** flag_ptrs = nullptr;  // device: each frame's flag
-  int* flags = nullptr;       // device: the gathered values
-  int* flags_host = nullptr;  // pinned
   std::string err;
 };
-
-// Copies and clears the frames' wait-timeout flags.
-__global__ void k_gather_flags(int* const* src, int n, int* dst) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = atomicExch(src[i], 0);
-}
 
 namespace {
 
@@ -156,17 +145,6 @@ int pikgpu_batch_create(int device, int num_frames, pikgpu_batch** out) {
     ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) ==
                    cudaSuccess;
   }
-  if (ok) {
-    std::vector<int*> ptrs;
-    for (auto* ctx : b->frames) ptrs.push_back(P<int>(ctx->tc_err));
-    ok = cudaMalloc(&b->flag_ptrs, sizeof(int*) * num_frames) ==
-             cudaSuccess &&
-         cudaMalloc(&b->flags, sizeof(int) * num_frames) == cudaSuccess &&
-         cudaMallocHost(&b->flags_host, sizeof(int) * num_frames) ==
-             cudaSuccess &&
-         cudaMemcpy(b->flag_ptrs, ptrs.data(), sizeof(int*) * num_frames,
-                    cudaMemcpyHostToDevice) == cudaSuccess;
-  }
   if (!ok) {
     pikgpu_batch_destroy(b);
     return PIKGPU_ERR_CUDA;
@@ -184,9 +162,6 @@ int pikgpu_batch_destroy(pikgpu_batch* b) {
     if (e) cudaEventDestroy(e);
   }
   if (b->fork) cudaEventDestroy(b->fork);
-  if (b->flag_ptrs) cudaFree(b->flag_ptrs);
-  if (b->flags) cudaFree(b->flags);
-  if (b->flags_host) cudaFreeHost(b->flags_host);
   if (b->stream) cudaStreamDestroy(b->stream);
   for (auto* ctx : b->frames) pikgpu_ctx_destroy(ctx);
   delete b;
@@ -241,24 +216,25 @@ int pikgpu_batch_reconstruct(pikgpu_batch* b, float* const* out_linear,
   }
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : b->stream;
   CUDA_TRY_B(b, cudaGraphLaunch(b->exec, st));
-  k_gather_flags<<<Blocks(n, 256), 256, 0, st>>>(b->flag_ptrs, int(n),
-                                                  b->flags);
-  CUDA_TRY_B(b, cudaMemcpyAsync(b->flags_host, b->flags, sizeof(int) * n,
-                                cudaMemcpyDeviceToHost, st));
   CUDA_TRY_B(b, cudaStreamSynchronize(st));
+  // Every frame's wait-timeout flag is read and cleared.
+  int code = 0;
+  size_t failed = 0;
   for (size_t i = 0; i < n; ++i) {
-    if (const int code = b->flags_host[i]) {
-      return BatchFail(b, PIKGPU_ERR_CUDA, "frame %zu: %s", i,
-                       WaitTimeoutMessage(code));
-    }
-    b->frames[i]->have_result = true;
+    const int c = TakeTimeout(b->frames[i]);
+    if (c && !code) code = c, failed = i;
+    if (!code) b->frames[i]->have_result = true;
+  }
+  if (code) {
+    return BatchFail(b, PIKGPU_ERR_CUDA, "frame %zu: %s", failed,
+                     WaitTimeoutMessage(code));
   }
   return PIKGPU_OK;
 }
 
 int pikgpu_batch_launch_count(const pikgpu_batch* b) {
   if (!b) return PIKGPU_ERR_INVALID_ARG;
-  int n = 1;  // k_gather_flags
+  int n = 0;
   for (const auto* ctx : b->frames) n += ctx->launches;
   return n;
 }

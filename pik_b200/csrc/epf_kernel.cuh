@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(EpfThreads<TH, ROWS>(), TH == 16 ? 3 : 2)
     __syncthreads();  // the mbarrier is initialised before anyone waits
     // (tc::WaitMma is the bounded mbarrier wait of the tensor-core kernels)
     if (!tc::WaitMma(mbar_s, 0, polls) && tid == 0) {
-      atomicExch(err, 2);
+      tc::ReportTimeout(err, 2);
     }
   } else {
     CpAsyncWaitAll();

@@ -114,7 +114,7 @@ struct pikgpu_ctx {
   // none), for pikgpu_encode_pnm.
   const float* last_lin = nullptr;
   size_t last_lin_stride = 0;
-  DevBuf sigma_ovr, counters, active[kNumClasses], tc_err;
+  DevBuf sigma_ovr, counters, active[kNumClasses];
   bool use_guide_ovr = false, use_sigma_ovr = false;
   // Dequantised AC supplied by the caller instead of Dequant::DoAC, and the
   // per-cell clamp scale (pikgpu_frame_set_dequantized_ac / _clamp_scale).
@@ -177,8 +177,9 @@ struct pikgpu_ctx {
   cudaGraphExec_t graph_exec = nullptr;
   int graph_launches = 0, graph_captures = 0;
   bool graph_tape_valid = false, last_replayed = false;
-  // Pinned host word the tensor-core error flag is read back into.
-  int* tc_err_host = nullptr;
+  // Wait-timeout flag of the kernels: a word of pinned host memory that they
+  // write through its device address (the same, under unified addressing).
+  int* tc_err = nullptr;
   // pikgpu_reconstruct_async enqueued work that pikgpu_wait has not yet
   // finished (with the tensor-core flag to check).
   bool pending = false;
@@ -525,6 +526,14 @@ const char* WaitTimeoutMessage(int code) {
                    : "tensor-core transform: MMA completion wait timed out";
 }
 
+// The wait-timeout flag after a synchronisation of the stream; cleared.
+int TakeTimeout(pikgpu_ctx* ctx) {
+  volatile int* flag = ctx->tc_err;
+  const int code = *flag;
+  if (code) *flag = 0;
+  return code;
+}
+
 // cuTensorMapEncodeTiled from the driver, found through the runtime's
 // entry-point query (no link-time dependency on libcuda); NULL if the
 // driver has none.
@@ -732,7 +741,7 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
     const EpfDc dco{f.dc, g.Bx, g.By, ctx->dc_half_step[0],
                     ctx->dc_half_step[1], ctx->dc_half_step[2]};
     EpfLaunch(sd, ctx->num_sms, ctx->form, dcpad, 0, dpw, dph, mm_dc,
-              DcEpfWork(s), nullptr, nullptr, dco, P<int>(ctx->tc_err), ctx->tc_polls);
+              DcEpfWork(s), nullptr, nullptr, dco, ctx->tc_err, ctx->tc_polls);
     ++ctx->launches;
   }
   Mark(ctx, kTDequant);
@@ -802,7 +811,7 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
       const int items = 3 * ((n[kC32] + 3) / 4);
       const int grid = std::min(items, ctx->num_sms * ctx->tc_ctas_per_sm);
       ch(k_square_idct_tc1<32, 3>, grid, tc::kThreads, 0, g, f, L[kC32],
-         n[kC32], s.predict_hf, counters + kWorkIdct32, P<int>(ctx->tc_err));
+         n[kC32], s.predict_hf, counters + kWorkIdct32, ctx->tc_err);
     } else if (n[kC32]) {
       ch(k_square32_idct, 3 * n[kC32], kSquareThreads, 0, g, f, L[kC32],
          s.predict_hf);
@@ -817,10 +826,10 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
       // the tensor cores); frames without it take three terms.
       if (ctx->form == PIKGPU_FORM_SPLIT_BF16 && s.predict_hf) {
         ch(k_square_idct_tc1<16, 2>, grid, tc::kThreads, 0, g, f, L[kC16],
-           n[kC16], s.predict_hf, counters + kWorkIdct, P<int>(ctx->tc_err));
+           n[kC16], s.predict_hf, counters + kWorkIdct, ctx->tc_err);
       } else {
         ch(k_square_idct_tc1<16, 3>, grid, tc::kThreads, 0, g, f, L[kC16],
-           n[kC16], s.predict_hf, counters + kWorkIdct, P<int>(ctx->tc_err));
+           n[kC16], s.predict_hf, counters + kWorkIdct, ctx->tc_err);
       }
     } else if (n[kC16]) {
       ch(k_square_idct_rows<16>, rows_grid(3 * n[kC16], 16), kSquareThreads,
@@ -881,7 +890,7 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
     EpfLaunch(st, ctx->num_sms, ctx->form, f.idct, gab, g.PW, g.PH,
               mm, work, f.filt,
               ctx->use_guide_ovr ? P<uint8_t>(ctx->guide_ovr) : nullptr,
-              EpfDc{}, P<int>(ctx->tc_err), ctx->tc_polls, pdl);
+              EpfDc{}, ctx->tc_err, ctx->tc_polls, pdl);
     ++ctx->launches;
     if (ctx->keep_stages) {
       cudaMemcpyAsync(ctx->dbg_epf.p, f.filt, sizeof(float) * 3 * npx,
@@ -920,7 +929,7 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
                                 ctx->num_sms * tc::ArCtasPerSm<32>());
       ch(k_square_ar_tc<32, 3>, grid, tc::kArThreads, ArTcSmemBytes<32, 3>(),
          g, f, s, P<uint32_t>(ctx->active[kC32]), counters + kC32,
-         counters + kWorkAr32, P<int>(ctx->tc_err));
+         counters + kWorkAr32, ctx->tc_err);
     } else if (n[kC32]) {
       ch(k_square32_ar, n[kC32], square32::kArThreads, 0, g, f, s,
          P<uint32_t>(ctx->active[kC32]), counters + kC32);
@@ -931,11 +940,11 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
       if (ctx->form == PIKGPU_FORM_SPLIT_BF16) {
         ch(k_square_ar_tc<16, 2>, grid, tc::kArThreads, ArTcSmemBytes<16, 2>(),
            g, f, s, P<uint32_t>(ctx->active[kC16]), counters + kC16,
-           counters + kWorkAr, P<int>(ctx->tc_err));
+           counters + kWorkAr, ctx->tc_err);
       } else {
         ch(k_square_ar_tc<16, 3>, grid, tc::kArThreads, ArTcSmemBytes<16, 3>(),
            g, f, s, P<uint32_t>(ctx->active[kC16]), counters + kC16,
-           counters + kWorkAr, P<int>(ctx->tc_err));
+           counters + kWorkAr, ctx->tc_err);
       }
     } else if (n[kC16]) {
       ch(k_square_ar_rows<16>, Blocks(n[kC16], SquareArBlocks<16>()),
@@ -1089,9 +1098,10 @@ int pikgpu_ctx_create(int device, pikgpu_ctx** out) {
   }
   cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount,
                          device);
-  if (Ensure(ctx, &ctx->tc_err, sizeof(int)) != PIKGPU_OK ||
-      cudaMemset(ctx->tc_err.p, 0, sizeof(int)) != cudaSuccess ||
-      cudaMallocHost(&ctx->tc_err_host, sizeof(int)) != cudaSuccess) {
+  if (cudaHostAlloc(&ctx->tc_err, sizeof(int), cudaHostAllocMapped) ==
+      cudaSuccess) {
+    *ctx->tc_err = 0;
+  } else {
     pikgpu_ctx_destroy(ctx);
     return PIKGPU_ERR_NO_MEMORY;
   }
@@ -1127,9 +1137,8 @@ int pikgpu_ctx_destroy(pikgpu_ctx* ctx) {
   for (auto& b : ctx->list) FreeBuf(&b);
   for (auto& b : ctx->active) FreeBuf(&b);
   FreeBuf(&ctx->counters);
-  FreeBuf(&ctx->tc_err);
   DropFrameGraph(ctx);
-  if (ctx->tc_err_host) cudaFreeHost(ctx->tc_err_host);
+  if (ctx->tc_err) cudaFreeHost(ctx->tc_err);
   for (auto& e : ctx->ev) {
     if (e) cudaEventDestroy(e);
   }
@@ -1535,9 +1544,6 @@ int EnqueueReconstruct(pikgpu_ctx* ctx, float* const out_linear[3],
                                       cudaMemcpyDeviceToHost, ctx->stream));
     }
   }
-  // The wait-timeout flag comes back with the same synchronisation.
-  CUDA_TRY(ctx, cudaMemcpyAsync(ctx->tc_err_host, ctx->tc_err.p, sizeof(int),
-                                cudaMemcpyDeviceToHost, ctx->stream));
   ctx->pending = true;
   return PIKGPU_OK;
 }
@@ -1546,9 +1552,7 @@ int EnqueueReconstruct(pikgpu_ctx* ctx, float* const out_linear[3],
 int FinishReconstruct(pikgpu_ctx* ctx) {
   ctx->pending = false;
   CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-  if (const int code = *ctx->tc_err_host) {
-    *ctx->tc_err_host = 0;
-    cudaMemset(ctx->tc_err.p, 0, sizeof(int));
+  if (const int code = TakeTimeout(ctx)) {
     return Fail(ctx, PIKGPU_ERR_CUDA, "%s", WaitTimeoutMessage(code));
   }
   if (ctx->profile) {

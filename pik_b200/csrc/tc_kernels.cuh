@@ -96,6 +96,13 @@ __device__ __forceinline__ bool WaitMma(uint32_t mbar, uint32_t phase,
   return false;
 }
 
+// Sets the context's wait-timeout flag, a word of pinned host memory: the host
+// reads it after the stream's synchronisation, without a copy.
+__device__ __forceinline__ void ReportTimeout(int* err, int code) {
+  *reinterpret_cast<volatile int*>(err) = code;
+  __threadfence_system();
+}
+
 // 16 consecutive FP32 columns of this thread's tensor-memory lane.
 __device__ __forceinline__ void Ld16(uint32_t taddr, float* v) {
   uint32_t r[16];
@@ -605,7 +612,7 @@ __global__ void __launch_bounds__(tc::kArThreads, tc::ArCtasPerSm<N>())
     ChannelSync(c);  // the operand may be written again
     batch = next;
   }
-  if (!ok && t == 0) atomicExch(err, 1);
+  if (!ok && t == 0) tc::ReportTimeout(err, 1);
   FenceBefore();
   __syncthreads();
   if (threadIdx.x < 32) {
@@ -818,7 +825,7 @@ __global__ void __launch_bounds__(tc::kThreads, N == 16 ? 8 : 4)
     item = item_next;
     item_next = item_after;
   }
-  if (!ok && t == 0) atomicExch(err, 1);
+  if (!ok && t == 0) tc::ReportTimeout(err, 1);
   FenceBefore();
   __syncthreads();
   if (t < 32) {
