@@ -854,7 +854,7 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
     // stream (no per-group events).
     const bool pdl = !ctx->profile && !ctx->keep_stages;
     if (gab) {
-      const int warps = Blocks(g.PW, 128) * Blocks(g.PH, kGmmRows);
+      const int warps = Blocks(g.PW, kStripW) * Blocks(g.PH, kGmmRows);
       k_gaborish_minmax<<<dim3(Blocks(warps, 8), 3), 256, 0, st>>>(
           f.idct, g.PW, g.PH, gab, mm); ++ctx->launches;
     } else {
@@ -963,16 +963,19 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
   {
     const int vec_lin = lin && lin_stride % 4 == 0 && g.W % 4 == 0 &&
                         reinterpret_cast<uintptr_t>(lin) % 16 == 0;
-    const int warps = Blocks(g.W, 128) * Blocks(g.H, kFinRows);
+    const int vec_rgb = rgb8_stride % 4 == 0 &&
+                        reinterpret_cast<uintptr_t>(rgb8) % 4 == 0;
     float* pre = ctx->keep_stages ? P<float>(ctx->dbg_pre) : nullptr;
-    if (s.gaborish) {
-      k_final_direct<true><<<Blocks(warps, 8), 256, 0, st>>>(
+    auto launch = [&](auto kernel, int strip_w) {
+      const int warps = Blocks(g.W, strip_w) * Blocks(g.H, kFinRows);
+      kernel<<<Blocks(warps, 8), 256, 0, st>>>(
           final_in, f.idct, final_region, g.PW, g.PH, g.W, g.H, s.gaborish,
-          pre, lin, lin_stride, vec_lin, rgb8, rgb8_stride);
+          pre, lin, lin_stride, vec_lin, rgb8, rgb8_stride, vec_rgb);
+    };
+    if (s.gaborish) {
+      launch(k_final_direct<true>, FinalStripW<true>());
     } else {
-      k_final_direct<false><<<Blocks(warps, 8), 256, 0, st>>>(
-          final_in, f.idct, final_region, g.PW, g.PH, g.W, g.H, 0, pre, lin,
-          lin_stride, vec_lin, rgb8, rgb8_stride);
+      launch(k_final_direct<false>, FinalStripW<false>());
     }
     ++ctx->launches;
   }

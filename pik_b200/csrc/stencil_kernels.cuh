@@ -168,70 +168,134 @@ __global__ void __launch_bounds__(kTileThreads)
   }
 }
 
-// Min/max of gaborish #1 without staging or barriers: each warp owns 128
-// columns (4 per lane) of kGmmRows rows and loads its kGmmRows + 2 input
-// rows as independent 16-byte loads (all in flight at once); lanes take
-// their left/right neighbours from the adjacent lanes, lane 0 and the
-// warp's last lane by scalar loads. Coordinates mirror at the image border
-// and each output follows Sym3's operation order, so the min/max equal
-// those of k_gaborish_tile. Grid: (warps of a plane / 8, 3).
+// A warp's strip of a plane row for the 3x3 stencils: 30 lanes own 4 columns
+// each, and lanes 0 and 31 hold the columns beside the strip, so that every
+// lane's left and right neighbours come from the adjacent lanes (with 32
+// owning lanes the outer neighbours were loads of single lanes and a select
+// per value). Beyond the plane's border the neighbour mirrors to the border
+// column itself.
+constexpr int kStripW = 120;
+struct StripLane {
+  int x;     // first column; a halo lane's may lie outside
+  int load;  // where its four values are read
+  bool edge;  // warp-uniform: some lane lies outside
+  __device__ StripLane(int x0, int w) {
+    const int lane = threadIdx.x & 31;
+    x = x0 - 4 + 4 * lane;
+    load = min(max(x, 0), w - 4);
+    edge = x0 == 0 || x0 + kStripW >= w;
+  }
+  // The lane's values of a row, mirrored at the border.
+  __device__ float4 Load(const float* row, int w) const {
+    float4 q = *reinterpret_cast<const float4*>(row + load);
+    if (edge) {
+      if (x < 0) q.w = q.x;
+      if (x >= w) q.x = q.w;
+    }
+    return q;
+  }
+};
+// Columns x - 1 .. x + 4 of an owning lane.
+__device__ __forceinline__ void StripRow6(const float4& q, float (&v)[6]) {
+  v[0] = __shfl_up_sync(0xFFFFFFFFu, q.w, 1);
+  v[1] = q.x, v[2] = q.y, v[3] = q.z, v[4] = q.w;
+  v[5] = __shfl_down_sync(0xFFFFFFFFu, q.x, 1);
+}
+
+// Minimum and maximum of three values, NaN if any is.
+__device__ __forceinline__ float Min3NaN(float a, float b, float c) {
+  float d;
+  asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+__device__ __forceinline__ float Max3NaN(float a, float b, float c) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
+// Ordered min/max of gaborish #1 over n columns from x and rows y0 .. y1 - 1
+// of a plane, value by value (the order of NaNs, which min.NaN and max.NaN
+// do not keep, is that of their bits).
+__device__ __noinline__ void GaborishMinMaxScalar(const float* p, int w, int h,
+                                                  int strength, int x, int n,
+                                                  int y0, int y1, uint32_t* lo,
+                                                  uint32_t* hi) {
+  const float* wt = c_t.gaborish[strength];
+  for (int y = y0; y < y1; ++y) {
+    for (int i = x; i < x + n; ++i) {
+      float v[3][6];  // columns i - 1 .. i + 1 of the three rows
+      for (int r = 0; r < 3; ++r)
+        for (int k = 0; k < 3; ++k)
+          v[r][k] = p[size_t(MirrorIdx(y - 1 + r, h)) * w +
+                      MirrorIdx(i - 1 + k, w)];
+      const uint32_t ob =
+          OrderedBits(Sym3Rows(v[0], v[1], v[2], 0, wt[0], wt[1], wt[2]));
+      *lo = min(*lo, ob);
+      *hi = max(*hi, ob);
+    }
+  }
+}
+
+// Min/max of gaborish #1 without staging or barriers: each warp owns a strip
+// of kGmmRows rows and loads its kGmmRows + 2 input rows as independent
+// 16-byte loads (all in flight at once). Coordinates mirror at the image
+// border and each output follows Sym3's operation order, so the min/max equal
+// those of k_gaborish_tile. Grid: (warps of a plane / 8, 3). Issue bound it:
+// with an integer min and max of every value's ordered bits, and edge loads
+// by single lanes, it took 36 us at 4K and 260 at 8192x8192; now 28 and 191
+// (4.2 TB/s).
 constexpr int kGmmRows = 8;
 __global__ void __launch_bounds__(256, 3)
     k_gaborish_minmax(const float* in, int w, int h, int strength,
                       uint32_t* mm) {
-  PdlLaunchDependents();  // the EPF may start on free SMs
+  PdlLaunchDependents();  // the plan may start on free SMs
   constexpr int R = kGmmRows;
   __shared__ uint32_t s_lo[8], s_hi[8];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int c = blockIdx.y;
-  const int tiles_x = (w + 127) / 128;
+  const int tiles_x = (w + kStripW - 1) / kStripW;
   const int wg = blockIdx.x * 8 + wib;
-  const int x0 = (wg % tiles_x) * 128, y0 = (wg / tiles_x) * R;
-  const int x = x0 + 4 * lane;
+  const int x0 = (wg % tiles_x) * kStripW, y0 = (wg / tiles_x) * R;
   uint32_t lo = 0xFFFFFFFFu, hi = 0u;
   if (y0 < h) {  // warp-uniform
     const float* p = in + c * size_t(w) * h;
-    const bool xv = x < w;
-    // Lanes whose right neighbour is not in the next lane's registers.
-    const bool own_right = lane == 31 || x + 4 >= w;
-    const int xl = MirrorIdx(x0 - 1, w), xr = MirrorIdx(x + 4, w);
+    const StripLane sl(x0, w);
     float4 q[R + 2];
-    float el[R + 2], er[R + 2];
 #pragma unroll
     for (int r = 0; r < R + 2; ++r) {
-      const float* row = p + size_t(MirrorIdx(y0 - 1 + r, h)) * w;
-      q[r] = xv ? *reinterpret_cast<const float4*>(row + x)
-                : make_float4(0.f, 0.f, 0.f, 0.f);
-      el[r] = lane == 0 ? row[xl] : 0.f;
-      er[r] = own_right && xv ? row[xr] : 0.f;
+      q[r] = sl.Load(p + size_t(MirrorIdx(y0 - 1 + r, h)) * w, w);
     }
     const float* wt = c_t.gaborish[strength];
     const float w0 = wt[0], w1 = wt[1], w2 = wt[2];
-    auto row6 = [&](int r, float v[6]) {
-      const float left = __shfl_up_sync(0xFFFFFFFFu, q[r].w, 1);
-      const float right = __shfl_down_sync(0xFFFFFFFFu, q[r].x, 1);
-      v[0] = lane == 0 ? el[r] : left;
-      v[1] = q[r].x, v[2] = q[r].y, v[3] = q[r].z, v[4] = q[r].w;
-      v[5] = own_right ? er[r] : right;
-    };
+    const float inf = __int_as_float(0x7F800000);
+    float mn = inf, mx = -inf;
     float a[6], m[6], b[6];
-    row6(0, a);
-    row6(1, m);
+    StripRow6(q[0], a);
+    StripRow6(q[1], m);
 #pragma unroll
     for (int j = 0; j < R; ++j) {
-      row6(j + 2, b);
-      if (xv) {
+      StripRow6(q[j + 2], b);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint32_t ob = OrderedBits(Sym3Rows(a, m, b, i, w0, w1, w2));
-          lo = min(lo, ob);
-          hi = max(hi, ob);
-        }
+      for (int i = 0; i < 4; i += 2) {
+        const float v0 = Sym3Rows(a, m, b, i, w0, w1, w2);
+        const float v1 = Sym3Rows(a, m, b, i + 1, w0, w1, w2);
+        mn = Min3NaN(mn, v0, v1);
+        mx = Max3NaN(mx, v0, v1);
       }
 #pragma unroll
       for (int i = 0; i < 6; ++i) {
         a[i] = m[i];
         m[i] = b[i];
+      }
+    }
+    // Planes are a multiple of 8 rows: all of the strip's exist.
+    if (lane >= 1 && lane <= 30 && sl.x < w) {
+      lo = OrderedBits(mn);
+      hi = OrderedBits(mx);
+      if (mn != mn || mx != mx) {
+        lo = 0xFFFFFFFFu, hi = 0u;
+        GaborishMinMaxScalar(p, w, h, strength, sl.x, 4, y0, y0 + R, &lo, &hi);
       }
     }
   }
@@ -276,18 +340,6 @@ __device__ __forceinline__ void XybToRgb(float x, float y, float b, float* r,
   *bl = lb + tb;
 }
 
-// The final pass without staging or barriers: each warp owns 128 columns x
-// kFinRows output rows of the three planes and loads its input rows
-// (kFinRows + 2 per plane with gaborish, kFinRows without) as independent
-// 16-byte loads up front;
-// horizontal neighbours come from the adjacent lanes, lane 0's and the
-// row's last lane's by scalar loads. Coordinates mirror at the padded
-// plane's border (pw x ph). `region` (NULL: always `in`): the EPF's region
-// flags; where a region's flag is 0 its pixels are read from `alt` (the
-// EPF's input). `vec_lin`: the linear outputs may be written as
-// float4 (width, stride and base all multiples of 4 floats / 16 bytes).
-// Grid: warps / 8.
-constexpr int kFinRows = 2;
 // Completes the EPF's output planes for the stage export: regions that it
 // left out get its input. One thread per 4 pixels of a plane.
 __global__ void k_fill_regions(const float* in, const uint32_t* region, int w,
@@ -300,88 +352,104 @@ __global__ void k_fill_regions(const float* in, const uint32_t* region, int w,
   *reinterpret_cast<float4*>(out + o) =
       *reinterpret_cast<const float4*>(in + o);
 }
+
+// The final pass without staging or barriers: each warp owns a strip of
+// kFinRows output rows of the three planes and loads its input rows
+// (kFinRows + 2 per plane with gaborish, kFinRows without) as independent
+// 16-byte loads; the horizontal neighbours come from the adjacent lanes
+// (StripLane). Coordinates mirror at the padded plane's border (pw x ph).
+// `region` (NULL: always `in`): the EPF's region flags; where a region's flag
+// is 0 its pixels are read from `alt` (the EPF's input). `vec_lin`: the
+// linear outputs may be written as float4 (width, stride and base all
+// multiples of 4 floats / 16 bytes); `vec_rgb`: the 8-bit rows of 4 pixels as
+// three words (stride and base multiples of 4 bytes). Grid: warps / 8.
+//
+// Issue bound it too: with 128 owned columns per warp, the rows of all planes
+// held at once (122 registers) and byte stores it took 55 us at 4K, 416 at
+// 8192x8192 and 30 at 1920x1080 with the 8-bit output; now 43, 307 (5.2 TB/s)
+// and 24. One row per warp: 48, 354 and 24; four: 44, 310 and 29.
+constexpr int kFinRows = 2;
 template <bool kGab>
-__global__ void __launch_bounds__(256)
+__host__ __device__ constexpr int FinalStripW() {
+  return kGab ? kStripW : 128;
+}
+template <bool kGab>
+__global__ void __launch_bounds__(256, 2)
     k_final_direct(const float* in, const float* alt, const uint32_t* region,
-                   int pw, int ph, int w, int h, int strength, float* pre, float* lin, size_t lin_stride,
-                   int vec_lin, uint8_t* rgb8, size_t rgb8_stride) {
+                   int pw, int ph, int w, int h, int strength, float* pre,
+                   float* lin, size_t lin_stride, int vec_lin, uint8_t* rgb8,
+                   size_t rgb8_stride, int vec_rgb) {
   constexpr int R = kFinRows, NR = kGab ? R + 2 : R;
   const int lane = threadIdx.x & 31;
   const int wg = blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int tiles_x = (w + 127) / 128;
-  const int x0 = (wg % tiles_x) * 128, y0 = (wg / tiles_x) * R;
+  constexpr int kW = FinalStripW<kGab>();
+  const int tiles_x = (w + kW - 1) / kW;
+  const int x0 = (wg % tiles_x) * kW, y0 = (wg / tiles_x) * R;
   if (y0 >= h) return;  // warp-uniform; no barriers below
   const size_t plane = size_t(pw) * ph;
-  const int x = x0 + 4 * lane;
-  const bool xv = x < pw;
-  const bool own_right = lane == 31 || x + 4 >= pw;
-  const int xl = MirrorIdx(x0 - 1, pw), xr = MirrorIdx(x + 4, pw);
+  StripLane sl(x0, pw);
+  if (!kGab) {
+    sl.x = x0 + 4 * lane;
+    sl.load = min(sl.x, pw - 4);
+    sl.edge = false;
+  }
+  const int x = sl.x;
   const int rw = (pw + kRegionW - 1) / kRegionW;
-  float4 q[3][NR];
-  float el[3][NR], er[3][NR];
+  const float* row[NR];
 #pragma unroll
   for (int r = 0; r < NR; ++r) {
     const int y = MirrorIdx(kGab ? y0 - 1 + r : y0 + r, ph);
-    // The source planes of column xx.
-    auto src = [&](int xx) {
-      return !region || region[(y / kRegionH) * rw + xx / kRegionW] ? in : alt;
-    };
-    const float* own = (xv ? src(x) : in) + size_t(y) * pw;
-    const float* left = (kGab && lane == 0 ? src(xl) : in) + size_t(y) * pw;
-    const float* right =
-        (kGab && own_right && xv ? src(xr) : in) + size_t(y) * pw;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      q[c][r] = xv ? *reinterpret_cast<const float4*>(own + c * plane + x)
-                   : make_float4(0.f, 0.f, 0.f, 0.f);
-      if (kGab) {
-        el[c][r] = lane == 0 ? left[c * plane + xl] : 0.f;
-        er[c][r] = own_right && xv ? right[c * plane + xr] : 0.f;
-      }
-    }
+    const float* src =
+        !region || region[(y / kRegionH) * rw + sl.load / kRegionW] ? in : alt;
+    row[r] = src + size_t(y) * pw;
   }
   const float* wt = c_t.gaborish[strength];
   const float w0 = wt[0], w1 = wt[1], w2 = wt[2];
-  auto row6 = [&](int c, int r, float v[6]) {
-    const float left = __shfl_up_sync(0xFFFFFFFFu, q[c][r].w, 1);
-    const float right = __shfl_down_sync(0xFFFFFFFFu, q[c][r].x, 1);
-    v[0] = lane == 0 ? el[c][r] : left;
-    v[1] = q[c][r].x, v[2] = q[c][r].y, v[3] = q[c][r].z, v[4] = q[c][r].w;
-    v[5] = own_right ? er[c][r] : right;
-  };
+  float v[R][3][4];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    float4 q[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) q[r] = sl.Load(row[r] + c * plane, pw);
+    if (kGab) {
+      float a[6], m[6], b[6];
+      StripRow6(q[0], a);
+      StripRow6(q[1], m);
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        StripRow6(q[j + 2], b);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          v[j][c][i] = Sym3Rows(a, m, b, i, w0, w1, w2);
+        }
+#pragma unroll
+        for (int i = 0; i < 6; ++i) a[i] = m[i], m[i] = b[i];
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        v[j][c][0] = q[j].x, v[j][c][1] = q[j].y;
+        v[j][c][2] = q[j].z, v[j][c][3] = q[j].w;
+      }
+    }
+  }
+  if (x >= w || (kGab && (lane == 0 || lane == 31))) return;
+  const int n = min(4, w - x);
 #pragma unroll
   for (int j = 0; j < R; ++j) {
     const int y = y0 + j;
-    float v[3][4];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      if (kGab) {
-        float a[6], m[6], b[6];
-        row6(c, j, a);
-        row6(c, j + 1, m);
-        row6(c, j + 2, b);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          v[c][i] = Sym3Rows(a, m, b, i, w0, w1, w2);
-        }
-      } else {
-        v[c][0] = q[c][j].x, v[c][1] = q[c][j].y;
-        v[c][2] = q[c][j].z, v[c][3] = q[c][j].w;
-      }
-    }
-    if (x >= w || y >= h) continue;
-    const int n = min(4, w - x);
+    if (y >= h) break;
     if (pre) {
 #pragma unroll
       for (int c = 0; c < 3; ++c)
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-          if (i < n) pre[(size_t(c) * h + y) * w + x + i] = v[c][i];
+          if (i < n) pre[(size_t(c) * h + y) * w + x + i] = v[j][c][i];
     }
     float r[4], g[4], bl[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      XybToRgb(v[0][i], v[1][i], v[2][i], &r[i], &g[i], &bl[i]);
+      XybToRgb(v[j][0][i], v[j][1][i], v[j][2][i], &r[i], &g[i], &bl[i]);
     }
     if (lin) {
       float* o0 = lin + size_t(y) * lin_stride + x;
@@ -405,12 +473,24 @@ __global__ void __launch_bounds__(256)
     }
     if (rgb8) {
       uint8_t* o = rgb8 + size_t(y) * rgb8_stride + 3 * size_t(x);
+      uint32_t px[12];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        if (i < n) {
-          o[3 * i + 0] = Srgb8(r[i]);
-          o[3 * i + 1] = Srgb8(g[i]);
-          o[3 * i + 2] = Srgb8(bl[i]);
+        px[3 * i] = Srgb8(r[i]);
+        px[3 * i + 1] = Srgb8(g[i]);
+        px[3 * i + 2] = Srgb8(bl[i]);
+      }
+      if (vec_rgb && n == 4) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          reinterpret_cast<uint32_t*>(o)[k] = px[4 * k] | px[4 * k + 1] << 8 |
+                                              px[4 * k + 2] << 16 |
+                                              px[4 * k + 3] << 24;
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < 12; ++k) {
+          if (k < 3 * n) o[k] = uint8_t(px[k]);
         }
       }
     }
