@@ -166,29 +166,41 @@ __global__ void k_adj_build_jac(AdjJac* J) {
 constexpr int kAdjLossBlocks = 592, kAdjThreads = 256;
 
 // g_pre = 2 (pre - target) inside xsize x ysize, 0 in the padding; the loss
-// partial sums of each CTA in FP64.
+// partial sums of each CTA in FP64. A warp per 256 columns of a row and turn,
+// eight loads of each plane in flight per lane (a flat index divided into
+// plane, row and column, with one, took 22 us at 1024x1024, this 8).
+constexpr int kAdjLossCols = 256;
 __global__ void __launch_bounds__(kAdjThreads)
     k_adj_loss(const float* pre, const float* target, int w, int h, int pw,
                int ph, float* g_pre, double* partial) {
   __shared__ double s_sum[kAdjThreads / 32];
-  const size_t plane = size_t(pw) * ph, n = 3 * plane;
+  const int lane = threadIdx.x & 31;
+  const int warps = gridDim.x * (kAdjThreads / 32);
   double acc = 0.0;
-  for (size_t i = blockIdx.x * size_t(kAdjThreads) + threadIdx.x; i < n;
-       i += size_t(gridDim.x) * kAdjThreads) {
-    const int c = int(i / plane);
-    const size_t rem = i % plane;
-    const int y = int(rem / pw), x = int(rem % pw);
-    float gv = 0.0f;
-    if (x < w && y < h) {
-      const size_t o = (size_t(c) * h + y) * w + x;
-      const double d = double(pre[o]) - double(target[o]);
-      acc += d * d;
-      gv = 2.0f * (pre[o] - target[o]);
+  const int segs = (pw + kAdjLossCols - 1) / kAdjLossCols;
+  for (int i = blockIdx.x * (kAdjThreads / 32) + (threadIdx.x >> 5);
+       i < 3 * ph * segs; i += warps) {
+    const int cy = i / segs, x0 = (i - cy * segs) * kAdjLossCols + lane;
+    const int c = cy / ph, y = cy - c * ph;
+    const size_t in = (size_t(c) * h + y) * w;
+    const int n = y < h ? w : 0;
+    float a[kAdjLossCols / 32], b[kAdjLossCols / 32];
+#pragma unroll
+    for (int k = 0; k < kAdjLossCols / 32; ++k) {
+      const int x = x0 + 32 * k;
+      a[k] = x < n ? pre[in + x] : 0.0f;
+      b[k] = x < n ? target[in + x] : 0.0f;
     }
-    g_pre[i] = gv;
+#pragma unroll
+    for (int k = 0; k < kAdjLossCols / 32; ++k) {
+      const int x = x0 + 32 * k;
+      const double d = double(a[k]) - double(b[k]);
+      acc += d * d;
+      if (x < pw) g_pre[size_t(cy) * pw + x] = 2.0f * (a[k] - b[k]);
+    }
   }
   for (int off = 16; off; off >>= 1) acc += __shfl_xor_sync(~0u, acc, off);
-  if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = acc;
+  if (lane == 0) s_sum[threadIdx.x >> 5] = acc;
   __syncthreads();
   if (threadIdx.x == 0) {
     double t = 0.0;
@@ -197,46 +209,44 @@ __global__ void __launch_bounds__(kAdjThreads)
   }
 }
 
+// One warp (a single thread's chain of dependent adds took 17 us).
 __global__ void k_adj_sum(const double* partial, int n, double* out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
   double t = 0.0;
-  for (int i = 0; i < n; ++i) t += partial[i];
-  *out = t;
+  for (int i = threadIdx.x; i < n; i += 32) t += partial[i];
+  for (int off = 16; off; off >>= 1) t += __shfl_xor_sync(~0u, t, off);
+  if (threadIdx.x == 0) *out = t;
 }
 
-// Transpose of Symmetric3 with mirrored borders (the forward stencil is
-// symmetric, so interior pixels gather with the same weights; border pixels
-// collect every tap whose mirrored source is them).
-__global__ void k_adj_gab(const float* gin, int pw, int ph, int strength,
-                          float* gout) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+// Transpose of Symmetric3 with mirrored borders: the stencil again, since
+// it is symmetric with its mirrored taps too (a border pixel's tap beyond the
+// frame reads that pixel's own row or column, -1 -> 0, at the same distance
+// as the tap that reads it). Four columns of a row per thread (pw is a
+// multiple of 8): 18 us at 1024x1024 with a pixel per thread, now 6.5.
+__global__ void __launch_bounds__(kAdjThreads)
+    k_adj_gab(const float* gin, int pw, int ph, int strength, float* gout) {
+  const int x0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   const int c = blockIdx.z;
-  if (x >= pw || y >= ph) return;
+  if (x0 >= pw || y >= ph) return;
   const float* wt = c_t.gaborish[strength];
   const float* p = gin + size_t(c) * pw * ph;
-  float s = 0.0f;
-  if (x >= 1 && x + 1 < pw && y >= 1 && y + 1 < ph) {
-    const float* t = p + size_t(y - 1) * pw + x;
-    const float* m = p + size_t(y) * pw + x;
-    const float* b = p + size_t(y + 1) * pw + x;
-    s = m[0] * wt[0] + (t[0] + b[0] + m[-1] + m[1]) * wt[1] +
-        (t[-1] + t[1] + b[-1] + b[1]) * wt[2];
-  } else {
-    for (int yy = max(y - 1, 0); yy <= min(y + 1, ph - 1); ++yy) {
-      for (int dy = -1; dy <= 1; ++dy) {
-        if (MirrorIdx(yy + dy, ph) != y) continue;
-        for (int xx = max(x - 1, 0); xx <= min(x + 1, pw - 1); ++xx) {
-          for (int dx = -1; dx <= 1; ++dx) {
-            if (MirrorIdx(xx + dx, pw) != x) continue;
-            const int k = abs(dx) + abs(dy);
-            s += wt[k == 0 ? 0 : k == 1 ? 1 : 2] * p[size_t(yy) * pw + xx];
-          }
-        }
-      }
-    }
+  float v[3][6], s[4];
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    const float* row = p + size_t(MirrorIdx(y - 1 + r, ph)) * pw;
+    const float4 q = *reinterpret_cast<const float4*>(row + x0);
+    v[r][0] = row[max(x0 - 1, 0)];
+    v[r][1] = q.x, v[r][2] = q.y, v[r][3] = q.z, v[r][4] = q.w;
+    v[r][5] = row[min(x0 + 4, pw - 1)];
   }
-  gout[size_t(c) * pw * ph + size_t(y) * pw + x] = s;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    s[i] = v[1][i + 1] * wt[0] +
+           (v[0][i + 1] + v[2][i + 1] + v[1][i] + v[1][i + 2]) * wt[1] +
+           (v[0][i] + v[0][i + 2] + v[2][i] + v[2][i + 2]) * wt[2];
+  }
+  *reinterpret_cast<float4*>(gout + size_t(c) * pw * ph + size_t(y) * pw +
+                             x0) = make_float4(s[0], s[1], s[2], s[3]);
 }
 
 // Clamp backward of one coefficient, on the branch the forward took (its
@@ -616,41 +626,65 @@ __global__ void __launch_bounds__(kEpfThreads, 2)
 }
 
 // Pass 3: the EPF terms that the forward mirrored back into the frame
-// (p + d outside it), scattered from the 4-pixel border band.
-__global__ void k_adj_epf_border(int w, int h, const uint8_t* guide,
-                                 const int32_t* sigma, const float* gv,
-                                 float* g_idct) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= w || y >= h) return;
-  if (x >= 3 && x < w - 4 && y >= 3 && y < h - 3) return;  // interior
+// (p + d outside it), scattered from the border band: the rows y < 3 and
+// y >= h - 3, and the columns x < 3 and x >= w - 4 of the others. One thread
+// per pixel of the band and offset d (a pixel per thread, its 56 offsets in
+// turn: 79 us at 1024x1024, now 9).
+constexpr int kAdjBand = 4;  // pixels per CTA
+__host__ __device__ inline size_t AdjBandPixels(int w, int h) {
+  // (an 8-row frame has its two bands of rows, an 8-column one all columns)
+  return size_t(6) * w + size_t(7) * (h - 6);
+}
+__global__ void __launch_bounds__(64 * kAdjBand, 4)
+    k_adj_epf_border(int w, int h, const uint8_t* guide, const int32_t* sigma,
+                     const float* gv, float* g_idct) {
+  const size_t i =
+      blockIdx.x * size_t(kAdjBand) + (threadIdx.x >> 6);
+  const int d = threadIdx.x & 63;
+  if (i >= AdjBandPixels(w, h) || d >= 56) return;
+  int x, y;
+  if (i < size_t(6) * w) {
+    x = int(i % w);
+    y = int(i / w);
+    if (y >= 3) y = h - 6 + y;
+  } else {
+    const size_t j = i - size_t(6) * w;
+    x = int(j % 7);
+    y = 3 + int(j / 7);
+    if (x >= 3) x = w - 7 + x;
+  }
   const int sg = sigma[(y >> 3) * (w / 8) + (x >> 3)];
   if (sg < kMinSigma) return;
+  const int cy = d / 8 - 3, cx = d % 8 - 3;
+  const int tx = x + cx, ty = y + cy;
+  if (tx >= 0 && tx < w && ty >= 0 && ty < h) return;  // gathered
   const size_t plane = size_t(w) * h;
   const int gwid = w + 12, ght = h + 12;
-  const int m64 = c_t.mul_table[sg] * 64;
-  auto gb = [&](int c, int yy, int xx) {
-    return int(guide[(size_t(c) * ght + yy + 6) * gwid + xx + 6]);
+  // The guide's four bytes x .. x + 3 of a row from the two aligned words
+  // around them (gwid is a multiple of 4; the rows read lie at least two
+  // above the buffer's end, so the second word is always inside it).
+  auto gw = [&](int c, int yy, int xx) {
+    const size_t o = (size_t(c) * ght + yy + 6) * gwid + xx + 6;
+    const uint32_t* p =
+        reinterpret_cast<const uint32_t*>(guide + (o & ~size_t(3)));
+    return __funnelshift_r(p[0], p[1], 8 * uint32_t(o & 3));
   };
-  float gvp[3];
-  for (int c = 0; c < 3; ++c) gvp[c] = gv[c * plane + size_t(y) * w + x];
-  for (int cy = -3; cy <= 3; ++cy) {
-    for (int cx = -3; cx <= 4; ++cx) {
-      const int tx = x + cx, ty = y + cy;
-      if (tx >= 0 && tx < w && ty >= 0 && ty < h) continue;  // gathered
-      int sad_max = 0;
-      for (int c = 0; c < 3; ++c) {
-        int sad = 0;
-        for (int py = -1; py <= 1; ++py)
-          for (int q = -1; q <= 2; ++q)
-            sad += abs(gb(c, y + py, x + q) - gb(c, ty + py, tx + q));
-        sad_max = max(sad_max, sad);
-      }
-      float wgt = EpfWeight(m64, sad_max);
-      if (!(wgt >= 0.05f)) continue;
-      const size_t o = size_t(MirrorIdx(ty, h)) * w + MirrorIdx(tx, w);
-      for (int c = 0; c < 3; ++c) atomicAdd(&g_idct[c * plane + o], gvp[c] * wgt);
+  uint32_t sad_max = 0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    uint32_t sad = 0;
+#pragma unroll
+    for (int py = -1; py <= 1; ++py) {
+      sad = Sad4(gw(c, y + py, x - 1), gw(c, ty + py, tx - 1), sad);
     }
+    sad_max = max(sad_max, sad);
+  }
+  const float wgt = EpfWeight(c_t.mul_table[sg] * 64, int(sad_max));
+  if (!(wgt >= 0.05f)) return;
+  const size_t o = size_t(MirrorIdx(ty, h)) * w + MirrorIdx(tx, w);
+  for (int c = 0; c < 3; ++c) {
+    atomicAdd(&g_idct[c * plane + o],
+              gv[c * plane + size_t(y) * w + x] * wgt);
   }
 }
 
@@ -804,19 +838,29 @@ __global__ void k_adj_lf(Geo g, DevFrame f, const AdjJac* J, int predict_hf,
 }
 
 // Quant field: every coefficient of a cell scales with 1 / qf, so
-// d L / d qf += -sum(g * ac) / qf (FP64 sum).
-__global__ void k_adj_qf(Geo g, DevFrame f, const float* ac0,
-                         const float* g_coef, float* g_qf) {
-  const int cell = blockIdx.x * blockDim.x + threadIdx.x;
+// d L / d qf += -sum(g * ac) / qf (FP64 sum). One warp per cell, two
+// coefficients per lane and channel (a cell per thread read 192 strided
+// values in turn: 54 us at 1024x1024, now 6.5).
+constexpr int kAdjQfCells = 8;  // warps per CTA
+__global__ void __launch_bounds__(32 * kAdjQfCells)
+    k_adj_qf(Geo g, DevFrame f, const float* ac0, const float* g_coef,
+             float* g_qf) {
+  const int cell = blockIdx.x * kAdjQfCells + (threadIdx.x >> 5);
   if (cell >= g.Bx * g.By) return;
+  const int lane = threadIdx.x & 31;
   const int bx = cell % g.Bx, by = cell / g.Bx;
   const size_t plane_ac = size_t(g.ac_stride) * g.By;
-  const size_t o = size_t(by) * g.ac_stride + size_t(bx) * 64;
+  const size_t o = size_t(by) * g.ac_stride + size_t(bx) * 64 + 2 * lane;
   double s = 0.0;
-  for (int c = 0; c < 3; ++c)
-    for (int k = 0; k < 64; ++k)
-      s += double(g_coef[c * plane_ac + o + k]) *
-           double(ac0[c * plane_ac + o + k]);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const float2 u = *reinterpret_cast<const float2*>(g_coef + c * plane_ac + o);
+    const float2 v = *reinterpret_cast<const float2*>(ac0 + c * plane_ac + o);
+    s += double(u.x) * double(v.x);
+    s += double(u.y) * double(v.y);
+  }
+  for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(~0u, s, off);
+  if (lane) return;
   double q = double(f.qf[cell]);
   if (f.clamp_scale) q /= double(f.clamp_scale[cell]);
   g_qf[cell] += float(-s / q);
@@ -866,7 +910,7 @@ int LaunchAdjoint(pikgpu_ctx* ctx, const float* target) {
   ctx->launches += 2;
   const float* g_cur = ga;
   if (s.gaborish) {
-    dim3 b(32, 8), gr(Blocks(g.PW, 32), Blocks(g.PH, 8), 3);
+    dim3 b(32, 8), gr(Blocks(g.PW / 4, 32), Blocks(g.PH, 8), 3);
     k_adj_gab<<<gr, b, 0, st>>>(ga, g.PW, g.PH, s.gaborish, gb);
     ++ctx->launches;
     g_cur = gb;
@@ -877,14 +921,10 @@ int LaunchAdjoint(pikgpu_ctx* ctx, const float* target) {
     // Guide bytes of the forward pass (the override, or MakeGuide again).
     const uint8_t* guide = P<uint8_t>(ctx->guide_ovr);
     if (!ctx->use_guide_ovr) {
-      const bool smoothed = s.gaborish && !s.use_sharpened;
-      int rc;
-      if (smoothed && (rc = EnsureSmoothed(ctx)) != PIKGPU_OK) return rc;
-      const float* src =
-          smoothed ? P<float>(ctx->smoothed) : P<float>(ctx->idct);
-      dim3 b(32, 8), gr(Blocks(g.PW + 12, 32), Blocks(g.PH + 12, 8), 3);
-      k_export_guide<<<gr, b, 0, st>>>(src, g.PW, g.PH, P<uint32_t>(ctx->mm),
-                                       P<uint8_t>(ctx->adj_guide));
+      dim3 b(32, 8), gr(Blocks(g.PW / 4 + 3, 32), Blocks(g.PH + 12, 8), 3);
+      k_export_guide<<<gr, b, 0, st>>>(
+          f.idct, s.use_sharpened ? 0 : s.gaborish, g.PW, g.PH,
+          P<uint32_t>(ctx->mm), P<uint8_t>(ctx->adj_guide));
       ++ctx->launches;
       guide = P<uint8_t>(ctx->adj_guide);
     }
@@ -920,8 +960,8 @@ int LaunchAdjoint(pikgpu_ctx* ctx, const float* target) {
         g.PW, g.PH, guide, sig, g_filt, nullptr, gv);
     k_adj_epf_pass<true><<<gr, kEpfThreads, kAdjEpfSmemBytes, st>>>(
         g.PW, g.PH, guide, sig, g_filt, gv, gc);
-    dim3 b3(32, 8), g3(Blocks(g.PW, 32), Blocks(g.PH, 8));
-    k_adj_epf_border<<<g3, b3, 0, st>>>(g.PW, g.PH, guide, sig, gv, gc);
+    k_adj_epf_border<<<Blocks(AdjBandPixels(g.PW, g.PH), kAdjBand),
+                       64 * kAdjBand, 0, st>>>(g.PW, g.PH, guide, sig, gv, gc);
     ctx->launches += 3;
     g_idct = gc;
   }
@@ -962,7 +1002,8 @@ int LaunchAdjoint(pikgpu_ctx* ctx, const float* target) {
   }
   const float* ac0 =
       ctx->use_dq_ovr ? P<float>(ctx->dq_ovr) : P<float>(ctx->dbg_dequant);
-  k_adj_qf<<<Blocks(nb, 256), 256, 0, st>>>(g, f, ac0, g_coef, g_qf);
+  k_adj_qf<<<Blocks(nb, kAdjQfCells), 32 * kAdjQfCells, 0, st>>>(
+      g, f, ac0, g_coef, g_qf);
   ++ctx->launches;
   (void)nac;
   CUDA_TRY(ctx, cudaGetLastError());

@@ -1712,17 +1712,13 @@ int pikgpu_get_epf_decisions(pikgpu_ctx* ctx, uint8_t* guide,
   }
   if (guide) {
     const size_t n = 3 * size_t(g.PW + 12) * (g.PH + 12);
-    const bool smoothed = ctx->s.gaborish && !ctx->s.use_sharpened;
     int rc;
-    if (smoothed && (rc = EnsureSmoothed(ctx)) != PIKGPU_OK) return rc;
     DevBuf tmp;
     if ((rc = Ensure(ctx, &tmp, n))) return rc;
-    const float* src =
-        smoothed ? P<float>(ctx->smoothed) : P<float>(ctx->idct);
-    dim3 b(32, 8), gr(Blocks(g.PW + 12, 32), Blocks(g.PH + 12, 8), 3);
-    k_export_guide<<<gr, b, 0, ctx->stream>>>(src, g.PW, g.PH,
-                                              P<uint32_t>(ctx->mm),
-                                              P<uint8_t>(tmp));
+    dim3 b(32, 8), gr(Blocks(g.PW / 4 + 3, 32), Blocks(g.PH + 12, 8), 3);
+    k_export_guide<<<gr, b, 0, ctx->stream>>>(
+        P<float>(ctx->idct), ctx->s.use_sharpened ? 0 : ctx->s.gaborish, g.PW,
+        g.PH, P<uint32_t>(ctx->mm), P<uint8_t>(tmp));
     cudaStreamSynchronize(ctx->stream);
     const cudaError_t e =
         cudaMemcpy(guide, tmp.p, n, cudaMemcpyDeviceToHost);

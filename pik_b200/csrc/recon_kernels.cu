@@ -359,21 +359,6 @@ __device__ __forceinline__ int ScaledSigma(float unscaled, float stretch) {
   return min(sg, kMaxSigma);
 }
 
-// Guide decision export (verification hook): u8 guide with the 6-pixel
-// mirrored border, 3 x (h + 12) x (w + 12).
-__global__ void k_export_guide(const float* src, int w, int h,
-                               const uint32_t* mm, uint8_t* guide) {
-  const int gx = blockIdx.x * blockDim.x + threadIdx.x - 6;
-  const int gy = blockIdx.y * blockDim.y + threadIdx.y - 6;
-  const int c = blockIdx.z;
-  if (gx >= w + 6 || gy >= h + 6) return;
-  float amin, mul, stretch;
-  GuideParams(mm, &amin, &mul, &stretch);
-  const float s = src[(size_t(c) * h + MirrorIdx(gy, h)) * w + MirrorIdx(gx, w)];
-  guide[(size_t(c) * (h + 12) + gy + 6) * (w + 12) + gx + 6] =
-      uint8_t(uint32_t(__float2int_rz((s - amin) * mul)));
-}
-
 // ---------------------------------------------------------------------------
 // sRGB-8 of one linear value on the 0..255 scale: TF_SRGB's rational
 // polynomial (pik/color_management.cc:323-345) and the rounding of

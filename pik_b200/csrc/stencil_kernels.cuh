@@ -202,6 +202,48 @@ __device__ __forceinline__ void StripRow6(const float4& q, float (&v)[6]) {
   v[5] = __shfl_down_sync(0xFFFFFFFFu, q.x, 1);
 }
 
+// The frame's u8 guide with the 6-pixel mirrored border, 3 x (h + 12) x
+// (w + 12), as the EPF takes it from `src` (gab > 0: smoothed by gaborish of
+// that strength): the verification export and the adjoint's guide. A word of
+// four pixels per thread (w + 12 is a multiple of 4), from the values at the
+// mirrored coordinates around it, which is the smoothed value at the mirrored
+// position: Sym3Rows adds each pair of neighbours first. At 1024x1024 a pixel per
+// thread took 26 us, and with the smoothed plane written and read again 37
+// and a host synchronisation; this takes 14.
+__global__ void __launch_bounds__(256)
+    k_export_guide(const float* src, int gab, int w, int h, const uint32_t* mm,
+                   uint8_t* guide) {
+  const int wd = blockIdx.x * blockDim.x + threadIdx.x;
+  const int gy = blockIdx.y * blockDim.y + threadIdx.y;
+  const int c = blockIdx.z;
+  if (4 * wd >= w + 12 || gy >= h + 12) return;
+  float amin, mul, stretch;
+  GuideParams(mm, &amin, &mul, &stretch);
+  const float* p = src + size_t(c) * w * h;
+  int x[6];
+#pragma unroll
+  for (int i = 0; i < 6; ++i) x[i] = MirrorIdx(4 * wd - 7 + i, w);
+  float v[3][6];
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    if (!gab && r != 1) continue;
+    const float* row = p + size_t(MirrorIdx(gy - 7 + r, h)) * w;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) v[r][i] = row[x[i]];
+  }
+  const float* wt = c_t.gaborish[gab];
+  uint32_t word = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float s = gab ? Sym3Rows(v[0], v[1], v[2], i, wt[0], wt[1], wt[2])
+                        : v[1][i + 1];
+    word |= uint32_t(uint8_t(uint32_t(__float2int_rz((s - amin) * mul))))
+            << (8 * i);
+  }
+  *reinterpret_cast<uint32_t*>(
+      guide + (size_t(c) * (h + 12) + gy) * (w + 12) + 4 * wd) = word;
+}
+
 // Minimum and maximum of three values, NaN if any is.
 __device__ __forceinline__ float Min3NaN(float a, float b, float c) {
   float d;
