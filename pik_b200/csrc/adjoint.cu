@@ -282,26 +282,58 @@ __device__ __forceinline__ float QfEff(const Geo& g, const DevFrame& f,
   return f.clamp_scale ? q / f.clamp_scale[cell] : q;
 }
 
+// Column e of a 64 x 64 matrix times the three channels' vectors in shared
+// memory: one matrix value serves the channels, 16-byte reads four of them.
+// 32 matrix values are in flight at a time (few frames have enough of these
+// blocks to fill the chip: what they cost is the loads' latency).
+__device__ __forceinline__ void DenseCols(const float (*m)[64], int e,
+                                          const float (*v)[64], float o[3]) {
+  o[0] = o[1] = o[2] = 0.0f;
+#pragma unroll 8
+  for (int p = 0; p < 64; p += 4) {
+    const float m0 = m[p][e], m1 = m[p + 1][e], m2 = m[p + 2][e],
+                m3 = m[p + 3][e];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const float4 q = *reinterpret_cast<const float4*>(&v[c][p]);
+      o[c] = fmaf(m0, q.x, o[c]);
+      o[c] = fmaf(m1, q.y, o[c]);
+      o[c] = fmaf(m2, q.z, o[c]);
+      o[c] = fmaf(m3, q.w, o[c]);
+    }
+  }
+}
+
+// The 8x8 types without a separable transform (DCT4X4 and the small ones):
+// two launches of 23 and 23 us at 1024x1024, one per class and with a channel
+// after the other, now 19.
 constexpr int kAdj8Blocks = 4;  // 8x8 blocks per CTA, 64 threads each
+struct Adj8Lists {
+  const uint32_t* list[2];
+  int count[2];
+  __device__ uint32_t At(int i) const {
+    return i < count[0] ? list[0][i] : list[1][i - count[0]];
+  }
+};
 
 // Clamp backward of 8x8 blocks (all cov = 1 types) from the dense
 // Jacobians. Blocks the EPF left unfiltered have EPF output == IDCT output,
 // a zero correction and ratio 0: the gradient passes to the IDCT output.
 __global__ void __launch_bounds__(kAdjThreads)
     k_adj_ar8(Geo g, DevFrame f, FrameScalars s, const AdjJac* J,
-              const uint32_t* list, int count, const int32_t* sigma,
-              const uint8_t* tape, const float* epf, const float* g_cur,
-              float* g_filt, float* g_idct, float* g_qf) {
-  __shared__ float s_a[kAdj8Blocks][3][64];  // diff, then g_corr
-  __shared__ float s_o[kAdj8Blocks][3][64];  // gradient of the output
+              Adj8Lists lists, const int32_t* sigma, const uint8_t* tape,
+              const float* epf, const float* g_cur, float* g_filt,
+              float* g_idct, float* g_qf) {
+  __shared__ __align__(16) float s_a[kAdj8Blocks][3][64];  // diff, then g_corr
+  __shared__ __align__(16) float s_o[kAdj8Blocks][3][64];  // gradient of the output
   __shared__ float s_q[kAdj8Blocks][2];
   const int lb = threadIdx.x >> 6, e = threadIdx.x & 63;
   const int item = blockIdx.x * kAdj8Blocks + lb;
-  const bool valid = item < count;
+  const bool valid = item < lists.count[0] + lists.count[1];
   int bx = 0, by = 0, type = 0;
   bool active = false;
   if (valid) {
-    const uint32_t pk = list[item];
+    const uint32_t pk = lists.At(item);
     bx = pk & 0xFFFF;
     by = pk >> 16;
     type = f.acs[by * g.Bx + bx] >> 4;
@@ -321,15 +353,8 @@ __global__ void __launch_bounds__(kAdjThreads)
   float gq = 0.0f, gc[3] = {0.0f, 0.0f, 0.0f};
   if (valid && active) {
     float co[3], gs[3], iv[3];
-    for (int c = 0; c < 3; ++c) {
-      float a = 0.0f, b = 0.0f;
-      for (int p = 0; p < 64; ++p) {
-        a += J->j1t[t][p][e] * s_a[lb][c][p];
-        b += J->j0[t][p][e] * s_o[lb][c][p];
-      }
-      co[c] = a;
-      gs[c] = b;
-    }
+    DenseCols(J->j1t[t], e, s_a[lb], co);
+    DenseCols(J->j0[t], e, s_o[lb], gs);
     const ArBlockInfo info = ArInfo(g, f, s, bx, by, type);
     for (int c = 0; c < 3; ++c) {
       iv[c] = e == 0 ? 1.0f * s.mul_dc[c] : info.dm[c][e] * info.inv_quant_ac;
@@ -346,13 +371,11 @@ __global__ void __launch_bounds__(kAdjThreads)
   __syncthreads();
   if (!valid) return;
   if (e == 0 && active) g_qf[by * g.Bx + bx] = s_q[lb][0] + s_q[lb][1];
+  float gd[3] = {0.0f, 0.0f, 0.0f};
+  if (active) DenseCols(J->j1[t], e, s_a[lb], gd);
   for (int c = 0; c < 3; ++c) {
-    float gd = 0.0f;
-    if (active) {
-      for (int k = 0; k < 64; ++k) gd += J->j1[t][k][e] * s_a[lb][c][k];
-    }
-    g_filt[c * plane + o] = gd;
-    g_idct[c * plane + o] = s_o[lb][c][e] - gd;
+    g_filt[c * plane + o] = gd[c];
+    g_idct[c * plane + o] = s_o[lb][c][e] - gd[c];
   }
 }
 
@@ -451,6 +474,127 @@ __global__ void __launch_bounds__(kAdjThreads)
     float t = 0.0f;
     for (int i = 0; i < kAdjThreads / 32; ++i) t += s_q[i];
     g_qf[by * g.Bx + bx] = t;
+  }
+}
+
+// A row times one of the transform matrices M (the inverse's A, or the
+// forward's B): o[k] = sum_i M[k][i] v[i], or with kT sum_i M[i][k] v[i].
+template <int N, bool kInverse, bool kT>
+__device__ __forceinline__ void MatRow(const float (&v)[N], float (&o)[N]) {
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    float a = 0.0f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int at = MatOffset(N) + (kT ? i * N + k : k * N + i);
+      a = fmaf(v[i], kInverse ? c_t.idct[at] : c_t.dct[at], a);
+    }
+    o[k] = a;
+  }
+}
+
+// The same for 8x8 DCT blocks, by rows in registers: a warp per channel of
+// four blocks, the element-wise step on the three channels' coefficients in
+// shared memory. With the dense Jacobians of k_adj_ar8 the 8x8 DCT blocks of
+// a 1024x1024 frame took 17 us, now 9. (16x16 blocks by the same split: 44 us
+// against 41 for k_adj_ar_sq, which has more warps per block.)
+__global__ void __launch_bounds__(kSquareArThreads)
+    k_adj_ar_dct8(Geo g, DevFrame f, FrameScalars s, const uint32_t* list,
+               int count, const int32_t* sigma, const uint8_t* tape,
+               const float* epf, const float* g_cur, float* g_filt,
+               float* g_idct, float* g_qf) {
+  using namespace square;
+  constexpr int N = 8, cov = 1, UPW = 32 / N, tile_size = N * (N + 1);
+  __shared__ float s_co[kSquareArGroups][UPW][3][tile_size];
+  __shared__ float s_g[kSquareArGroups][UPW][3][tile_size];
+  __shared__ float s_q[kSquareArGroups][UPW][3];
+  constexpr float scale = 1.0f / float(N * N);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = warp % 3, grp = warp / 3;
+  const int unit = lane / N, r = lane % N;
+  const int item = (blockIdx.x * kSquareArGroups + grp) * UPW + unit;
+  const bool valid = item < count;
+  const uint32_t pk = list[valid ? item : 0];
+  const int bx = pk & 0xFFFF, by = pk >> 16;
+  const int type = f.acs[by * g.Bx + bx] >> 4;
+  const bool active = sigma[by * g.Bx + bx] >= kMinSigma;
+  const size_t row = c * size_t(g.PW) * g.PH + size_t(by * 8 + r) * g.PW +
+                     bx * 8;
+  float G[N], D[N], T[N];
+#pragma unroll
+  for (int x = 0; x < N; x += 4) {
+    const float4 a = *reinterpret_cast<const float4*>(epf + row + x);
+    const float4 o = *reinterpret_cast<const float4*>(f.idct + row + x);
+    const float4 q = *reinterpret_cast<const float4*>(g_cur + row + x);
+    D[x] = a.x - o.x, D[x + 1] = a.y - o.y;
+    D[x + 2] = a.z - o.z, D[x + 3] = a.w - o.w;
+    G[x] = q.x, G[x + 1] = q.y, G[x + 2] = q.z, G[x + 3] = q.w;
+  }
+  float* tco = s_co[grp][unit][c];
+  float* tg = s_g[grp][unit][c];
+  MatRow<N, false, false>(D, T);  // the correction's coefficients
+  PutCol<N>(tco, r, T);
+  MatRow<N, true, true>(G, T);  // the gradient of the scaled correction
+  PutRow<N>(tg, r, T);
+  __syncwarp();
+  GetRow<N>(tco, r, D);
+  MatRow<N, false, false>(D, T);
+#pragma unroll
+  for (int x = 0; x < N; ++x) T[x] *= scale;
+  __syncwarp();
+  PutRow<N>(tco, r, T);
+  GetCol<N>(tg, r, D);
+  MatRow<N, true, true>(D, T);
+  __syncwarp();
+  PutRow<N>(tg, r, T);
+  __syncthreads();
+  // A block's 24 lanes share its 64 coefficients.
+  const ArBlockInfo info = ArInfo(g, f, s, bx, by, type);
+  const float qf_eff = QfEff(g, f, bx, by);
+  float gq = 0.0f;
+  for (int e = c * N + r; e < N * N && valid && active; e += 3 * N) {
+    const int y = e / N, x = e % N, at = y * (N + 1) + x;
+    const bool llf = e == 0;
+    float co[3], gs[3], iv[3], gc[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      co[k] = s_co[grp][unit][k][at];
+      gs[k] = s_g[grp][unit][k][at];
+      iv[k] = llf ? s.mul_dc[k]
+                  : info.dm[k][e] * info.inv_quant_ac;
+    }
+    ClampBackward(tape[CoefOffset(g, bx, by, cov, e)], co, iv, gs, llf,
+                  qf_eff, gc, &gq);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) s_g[grp][unit][k][at] = gc[k];
+  }
+  for (int off = N / 2; off; off >>= 1) {
+    gq += __shfl_xor_sync(~0u, gq, off);
+  }
+  if (r == 0) s_q[grp][unit][c] = gq;
+  __syncthreads();
+  GetRow<N>(tg, r, D);
+  MatRow<N, false, true>(D, T);
+  __syncwarp();
+  PutCol<N>(tg, r, T);
+  __syncwarp();
+  GetRow<N>(tg, r, D);
+  MatRow<N, false, true>(D, T);
+  if (!valid) return;
+#pragma unroll
+  for (int x = 0; x < N; ++x) T[x] = active ? T[x] * scale : 0.0f;
+#pragma unroll
+  for (int x = 0; x < N; x += 4) {
+    const float4 q = *reinterpret_cast<const float4*>(g_cur + row + x);
+    *reinterpret_cast<float4*>(g_filt + row + x) =
+        make_float4(T[x], T[x + 1], T[x + 2], T[x + 3]);
+    *reinterpret_cast<float4*>(g_idct + row + x) =
+        make_float4(q.x - T[x], q.y - T[x + 1], q.z - T[x + 2],
+                    q.w - T[x + 3]);
+  }
+  if (active && c == 0 && r == 0) {
+    const float* q = s_q[grp][unit];
+    g_qf[by * g.Bx + bx] = q[0] + q[1] + q[2];
   }
 }
 
@@ -692,16 +836,17 @@ __global__ void __launch_bounds__(64 * kAdjBand, 4)
 // masked coefficient gradient (all but 0, 1, 8, 9) through
 // TransformFromPixels transposed into the upsampled-prediction gradient.
 __global__ void __launch_bounds__(kAdjThreads)
-    k_adj_topix8(Geo g, DevFrame f, const AdjJac* J, const uint32_t* list,
-                 int count, int predict_hf, const float* g_idct,
+    k_adj_topix8(Geo g, DevFrame f, const AdjJac* J, Adj8Lists lists,
+                 int predict_hf, const float* g_idct,
                  float* g_coef, float* g_up) {
-  __shared__ float s_p[kAdj8Blocks][3][64], s_m[kAdj8Blocks][3][64];
+  __shared__ __align__(16) float s_p[kAdj8Blocks][3][64];
+  __shared__ __align__(16) float s_m[kAdj8Blocks][3][64];
   const int lb = threadIdx.x >> 6, e = threadIdx.x & 63;
   const int item = blockIdx.x * kAdj8Blocks + lb;
-  const bool valid = item < count;
+  const bool valid = item < lists.count[0] + lists.count[1];
   int bx = 0, by = 0, type = 0;
   if (valid) {
-    const uint32_t pk = list[item];
+    const uint32_t pk = lists.At(item);
     bx = pk & 0xFFFF;
     by = pk >> 16;
     type = f.acs[by * g.Bx + bx] >> 4;
@@ -716,19 +861,82 @@ __global__ void __launch_bounds__(kAdjThreads)
   const int t = JIndex(type);
   const bool masked = e == 0 || e == 1 || e == 8 || e == 9;
   if (valid) {
+    float gc[3];
+    DenseCols(J->j0[t], e, s_p[lb], gc);
     for (int c = 0; c < 3; ++c) {
-      float gc = 0.0f;
-      for (int p = 0; p < 64; ++p) gc += J->j0[t][p][e] * s_p[lb][c][p];
-      g_coef[c * plane_ac + size_t(by) * g.ac_stride + bx * 64 + e] = gc;
-      s_m[lb][c][e] = masked ? 0.0f : gc;
+      g_coef[c * plane_ac + size_t(by) * g.ac_stride + bx * 64 + e] = gc[c];
+      s_m[lb][c][e] = masked ? 0.0f : gc[c];
     }
   }
   __syncthreads();
   if (!valid || !predict_hf || !PredictHFOf(type)) return;
-  for (int c = 0; c < 3; ++c) {
-    float gp = 0.0f;
-    for (int k = 0; k < 64; ++k) gp += J->j1[t][k][e] * s_m[lb][c][k];
-    g_up[c * plane + o] = gp;
+  float gp[3];
+  DenseCols(J->j1[t], e, s_m[lb], gp);
+  for (int c = 0; c < 3; ++c) g_up[c * plane + o] = gp[c];
+}
+
+// The same for 8x8 and 16x16 DCT blocks, by rows in registers (a unit of N
+// lanes per block and channel, as k_square_idct_rows). At 1024x1024 the 16x16
+// blocks took 55 us with a CTA per block and the cooperative transforms, now
+// 25; the 8x8 ones 9 us with the dense Jacobians, now 3.5.
+template <int N>
+__global__ void __launch_bounds__(kSquareThreads)
+    k_adj_topix_rows(Geo g, DevFrame f, const uint32_t* list, int count,
+                  int predict_hf, const float* g_idct, float* g_coef,
+                  float* g_up) {
+  using namespace square;
+  constexpr int cov = N / 8;
+  __shared__ float s_tile[kSquareThreads / N][N * (N + 1)];
+  const int unit = threadIdx.x / N, r = threadIdx.x % N;
+  const int item = blockIdx.x * (kSquareThreads / N) + unit;
+  const bool active = item < 3 * count;
+  float* tile = s_tile[unit];
+  const int c = active ? item % 3 : 0;
+  const uint32_t pk = list[active ? item / 3 : 0];
+  const int bx = pk & 0xFFFF, by = pk >> 16;
+  const size_t px =
+      c * size_t(g.PW) * g.PH + size_t(by * 8 + r) * g.PW + bx * 8;
+  float X[N], T[N];
+#pragma unroll
+  for (int i = 0; i < N; i += 4) {
+    const float4 v = *reinterpret_cast<const float4*>(g_idct + px + i);
+    X[i] = v.x, X[i + 1] = v.y, X[i + 2] = v.z, X[i + 3] = v.w;
+  }
+  MatRow<N, true, true>(X, T);
+  PutRow<N>(tile, r, T);
+  __syncwarp();
+  GetCol<N>(tile, r, X);
+  MatRow<N, true, true>(X, T);  // row r of the coefficient gradient
+  __syncwarp();
+  if (active) {
+    float* out = g_coef + c * size_t(g.ac_stride) * g.By +
+                 CoefRowOffset(g, bx, by, N, r);
+#pragma unroll
+    for (int i = 0; i < N; i += 4) {
+      *reinterpret_cast<float4*>(out + i) =
+          make_float4(T[i], T[i + 1], T[i + 2], T[i + 3]);
+    }
+  }
+  if (!predict_hf) return;
+  // DCT_NOHF shares the 8x8 class; its gradient is formed but not stored.
+  const bool hf = active && PredictHFOf(f.acs[by * g.Bx + bx] >> 4);
+  if (r < 2 * cov) {
+#pragma unroll
+    for (int i = 0; i < 2 * cov; ++i) T[i] = 0.0f;
+  }
+  MatRow<N, false, true>(T, X);
+  PutCol<N>(tile, r, X);
+  __syncwarp();
+  GetRow<N>(tile, r, X);
+  MatRow<N, false, true>(X, T);
+  if (hf) {
+    constexpr float scale = 1.0f / float(N * N);
+#pragma unroll
+    for (int i = 0; i < N; i += 4) {
+      *reinterpret_cast<float4*>(g_up + px + i) =
+          make_float4(T[i] * scale, T[i + 1] * scale, T[i + 2] * scale,
+                      T[i + 3] * scale);
+    }
   }
 }
 
@@ -901,6 +1109,7 @@ int LaunchAdjoint(pikgpu_ctx* ctx, const float* target) {
     L[k] = P<uint32_t>(ctx->list[k]);
     n[k] = int(ctx->lists[k].size());
   }
+  const Adj8Lists lists8 = {{L[kC4], L[kCSmall]}, {n[kC4], n[kCSmall]}};
 
   k_adj_loss<<<kAdjLossBlocks, kAdjThreads, 0, st>>>(
       P<float>(ctx->dbg_pre), target, g.W, g.H, g.PW, g.PH, ga,
@@ -934,11 +1143,15 @@ int LaunchAdjoint(pikgpu_ctx* ctx, const float* target) {
     // g_filt goes to ga (g_pre is dead once g_cur exists; without
     // gaborish g_cur is ga itself, so g_filt then takes gb).
     float* g_filt = s.gaborish ? ga : gb;
-    const int k8[3] = {kC8, kC4, kCSmall};
-    for (int k : k8) {
-      if (!n[k]) continue;
-      k_adj_ar8<<<Blocks(n[k], kAdj8Blocks), kAdjThreads, 0, st>>>(
-          g, f, s, J, L[k], n[k], sig, tape, epf, g_cur, g_filt, gc, g_qf);
+    if (n[kC8]) {
+      k_adj_ar_dct8<<<Blocks(n[kC8], SquareArBlocks<8>()), kSquareArThreads, 0,
+                      st>>>(
+          g, f, s, L[kC8], n[kC8], sig, tape, epf, g_cur, g_filt, gc, g_qf);
+      ++ctx->launches;
+    }
+    if (n[kC4] + n[kCSmall]) {
+      k_adj_ar8<<<Blocks(n[kC4] + n[kCSmall], kAdj8Blocks), kAdjThreads, 0,
+                  st>>>(g, f, s, J, lists8, sig, tape, epf, g_cur, g_filt, gc, g_qf);
       ++ctx->launches;
     }
     if (n[kC16]) {
@@ -971,15 +1184,20 @@ int LaunchAdjoint(pikgpu_ctx* ctx, const float* target) {
   if (s.predict_hf) {
     CUDA_TRY(ctx, cudaMemsetAsync(g_up, 0, sizeof(float) * 3 * npx, st));
   }
-  const int k8[3] = {kC8, kC4, kCSmall};
-  for (int k : k8) {
-    if (!n[k]) continue;
-    k_adj_topix8<<<Blocks(n[k], kAdj8Blocks), kAdjThreads, 0, st>>>(
-        g, f, J, L[k], n[k], s.predict_hf, g_idct, g_coef, g_up);
+  if (n[kC8]) {
+    k_adj_topix_rows<8><<<Blocks(3 * n[kC8], kSquareThreads / 8),
+                          kSquareThreads, 0, st>>>(
+        g, f, L[kC8], n[kC8], s.predict_hf, g_idct, g_coef, g_up);
+    ++ctx->launches;
+  }
+  if (n[kC4] + n[kCSmall]) {
+    k_adj_topix8<<<Blocks(n[kC4] + n[kCSmall], kAdj8Blocks), kAdjThreads, 0,
+                   st>>>(g, f, J, lists8, s.predict_hf, g_idct, g_coef, g_up);
     ++ctx->launches;
   }
   if (n[kC16]) {
-    k_adj_topix_sq<16><<<n[kC16], kAdjThreads, 0, st>>>(
+    k_adj_topix_rows<16><<<Blocks(3 * n[kC16], kSquareThreads / 16),
+                           kSquareThreads, 0, st>>>(
         g, f, L[kC16], n[kC16], s.predict_hf, g_idct, g_coef, g_up);
     ++ctx->launches;
   }
