@@ -25,9 +25,9 @@
 //                   forward's clamp kernels wrote (which channel set the
 //                   minimum ratio, or none, or a +0.0 correction), the
 //                   gradients of the correction and of the quant field
-//   k_adj_epf       the EPF with frozen weights: each filtered pixel's
-//                   normalised weights scattered back to its (mirrored)
-//                   neighbours through a shared-memory tile
+//   k_adj_epf*      the EPF with frozen weights: every pixel gathers the
+//                   normalised weights of its filtered neighbours, and the
+//                   border pixels' mirrored terms are scattered
 //   k_adj_topix*    TransformToPixels transposed per first block, and for HF
 //                   prediction TransformFromPixels transposed of the masked
 //                   coefficient gradient (the upsampled prediction's
@@ -37,10 +37,10 @@
 //                   corner (pik/ac_predictions.cc:560-635); LLF gets zero
 //                   (it is overwritten from DC)
 //   k_adj_qf        the quant field: -sum(g * ac) / qf per cell
-// Square DCT blocks of 16 and 32 use the separable transforms with
-// transposed matrices; the 8x8 types use dense 64 x 64 Jacobians built on
-// the device from the forward transforms applied to unit vectors
-// (k_adj_build_jac). The backward arithmetic is FP32 (sums of the quant
+// Square DCT blocks use the separable transforms with transposed matrices;
+// the other 8x8 types use dense 64 x 64 Jacobians built on the device from
+// the forward transforms applied to unit vectors (k_adj_build_jac). The
+// backward arithmetic is FP32 (sums of the quant
 // field gradient and the loss in FP64).
 //
 // Included by pikgpu.cu (single translation unit).
@@ -322,10 +322,11 @@ struct Adj8Lists {
 __global__ void __launch_bounds__(kAdjThreads)
     k_adj_ar8(Geo g, DevFrame f, FrameScalars s, const AdjJac* J,
               Adj8Lists lists, const int32_t* sigma, const uint8_t* tape,
-              const float* epf, const float* g_cur, float* g_filt,
-              float* g_idct, float* g_qf) {
-  __shared__ __align__(16) float s_a[kAdj8Blocks][3][64];  // diff, then g_corr
-  __shared__ __align__(16) float s_o[kAdj8Blocks][3][64];  // gradient of the output
+              const float* epf, const float* sum_w, const float* g_cur,
+              float* g_filt, float* g_idct, float* g_qf) {
+  // The difference, then g_corr; the gradient of the output.
+  __shared__ __align__(16) float s_a[kAdj8Blocks][3][64];
+  __shared__ __align__(16) float s_o[kAdj8Blocks][3][64];
   __shared__ float s_q[kAdj8Blocks][2];
   const int lb = threadIdx.x >> 6, e = threadIdx.x & 63;
   const int item = blockIdx.x * kAdj8Blocks + lb;
@@ -373,8 +374,9 @@ __global__ void __launch_bounds__(kAdjThreads)
   if (e == 0 && active) g_qf[by * g.Bx + bx] = s_q[lb][0] + s_q[lb][1];
   float gd[3] = {0.0f, 0.0f, 0.0f};
   if (active) DenseCols(J->j1[t], e, s_a[lb], gd);
+  const float sw = active ? sum_w[o] : 1.0f;
   for (int c = 0; c < 3; ++c) {
-    g_filt[c * plane + o] = gd[c];
+    g_filt[c * plane + o] = gd[c] / sw;
     g_idct[c * plane + o] = s_o[lb][c][e] - gd[c];
   }
 }
@@ -400,8 +402,8 @@ template <int N>
 __global__ void __launch_bounds__(kAdjThreads)
     k_adj_ar_sq(Geo g, DevFrame f, FrameScalars s, const uint32_t* list,
                 int count, const int32_t* sigma, const uint8_t* tape,
-                const float* epf, const float* g_cur, float* g_filt,
-                float* g_idct, float* g_qf) {
+                const float* epf, const float* sum_w, const float* g_cur,
+                float* g_filt, float* g_idct, float* g_qf) {
   constexpr int NN = N * N, cov = N / 8;
   __shared__ float s_b[NN], s_a[NN], s_bt[NN];
   __shared__ float s_co[3][NN], s_g[3][NN], s_t[NN];
@@ -464,7 +466,9 @@ __global__ void __launch_bounds__(kAdjThreads)
     const int c = i / NN, e = i % NN;
     const size_t o = pix(c, e);
     const float gd = s_g[c][e];
-    g_filt[o] = gd;
+    const int x = bx * 8 + e % N, y = by * 8 + e / N;
+    const bool filtered = sigma[(y >> 3) * g.Bx + (x >> 3)] >= kMinSigma;
+    g_filt[o] = filtered ? gd / sum_w[size_t(y) * g.PW + x] : gd;
     g_idct[o] = g_cur[o] - gd;
   }
   for (int off = 16; off; off >>= 1) gq += __shfl_xor_sync(~0u, gq, off);
@@ -501,8 +505,8 @@ __device__ __forceinline__ void MatRow(const float (&v)[N], float (&o)[N]) {
 __global__ void __launch_bounds__(kSquareArThreads)
     k_adj_ar_dct8(Geo g, DevFrame f, FrameScalars s, const uint32_t* list,
                int count, const int32_t* sigma, const uint8_t* tape,
-               const float* epf, const float* g_cur, float* g_filt,
-               float* g_idct, float* g_qf) {
+               const float* epf, const float* sum_w, const float* g_cur,
+               float* g_filt, float* g_idct, float* g_qf) {
   using namespace square;
   constexpr int N = 8, cov = 1, UPW = 32 / N, tile_size = N * (N + 1);
   __shared__ float s_co[kSquareArGroups][UPW][3][tile_size];
@@ -586,8 +590,13 @@ __global__ void __launch_bounds__(kSquareArThreads)
 #pragma unroll
   for (int x = 0; x < N; x += 4) {
     const float4 q = *reinterpret_cast<const float4*>(g_cur + row + x);
-    *reinterpret_cast<float4*>(g_filt + row + x) =
-        make_float4(T[x], T[x + 1], T[x + 2], T[x + 3]);
+    float4 sw = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+    if (active) {
+      sw = *reinterpret_cast<const float4*>(
+          sum_w + size_t(by * 8 + r) * g.PW + bx * 8 + x);
+    }
+    *reinterpret_cast<float4*>(g_filt + row + x) = make_float4(
+        T[x] / sw.x, T[x + 1] / sw.y, T[x + 2] / sw.z, T[x + 3] / sw.w);
     *reinterpret_cast<float4*>(g_idct + row + x) =
         make_float4(q.x - T[x], q.y - T[x + 1], q.z - T[x + 2],
                     q.w - T[x + 3]);
@@ -602,170 +611,201 @@ __global__ void __launch_bounds__(kSquareArThreads)
 // filtered pixel p, out(p) = sum_d w(p, d) in(p + d) / sum_d w(p, d) over
 // the 7 x 8 window d = (cx, cy), cx in [-3, 4], cy in [-3, 3], where
 // w(p, d) = W(mul(p), SAD(p, p + d)) and in() is mirrored at the frame
-// border. Its transpose sends g(p) w(p, d) / sum_w(p) to p + d. The patch
-// SAD is symmetric, SAD(p, p + d) = SAD(q, q - d) for q = p + d, so the
-// transpose is a gather at q over the mirrored window e = -d
-// (cx in [-4, 3]) with the weight of the sending pixel p = q + e:
-//   pass 1 (k_adj_epf_pass<false>): gv(p) = g(p) / sum_w(p) for filtered
-//          pixels, 0 for copied ones;
-//   pass 2 (k_adj_epf_pass<true>):  g_idct(q) += sum_e gv(q + e)
-//          W(mul(q + e), SAD(q, q + e)) (+ g(q) itself where q was copied),
-//          for q + e inside the frame;
-//   pass 3 (k_adj_epf_border): the terms whose target p + d lies outside
-//          the frame (p within 4 pixels of the border), scattered to the
-//          mirrored position.
-// Passes 1 and 2 follow the forward kernel's design (k_epf_box): 64 x 32
-// tiles, one column of four rows per lane, the u8 guide staged as one
-// 32-bit word per byte offset and patch SADs by __vsadu4, summed vertically
-// across the lane's rows.
-constexpr int kAdjEpfTH = kEpfH + 6;   // gather tile rows y0 - 3 .. y0 + 34
-constexpr int kAdjEpfTW = kEpfW + 8;   // gather tile cols x0 - 4 .. x0 + 67
-constexpr size_t kAdjEpfSmemBytes =
-    kEpfGuideWords * 4 + size_t(3) * kAdjEpfTH * kAdjEpfTW * 4;
+// border. Its transpose sends gv(p) w(p, d), gv(p) = g(p) / sum_w(p), to
+// p + d; the sums are the forward pass's. g_filt holds gv for filtered pixels
+// (the clamp's backward kernels divide) and g(p) itself for copied ones. The
+// patch SAD is symmetric, SAD(p, p + d) = SAD(q, q - d) for q = p + d, so the
+// transpose is a gather at q over the mirrored window e = -d (cx in [-4, 3])
+// with the weight of the sending pixel p = q + e:
+//   k_adj_epf         g_idct(q) += sum_e gv(q + e) W(mul(q + e),
+//                     SAD(q, q + e)) (+ g(q) itself where q was copied), for
+//                     q + e inside the frame;
+//   k_adj_epf_border  the terms whose target p + d lies outside the frame (p
+//                     within 4 pixels of the border), scattered to the
+//                     mirrored position.
+// k_adj_epf follows the forward kernel's tensor-core form (k_epf_box): 64 x
+// 16 tiles, one column of four rows per lane, the u8 guide staged as one
+// 32-bit word per byte offset, cx outermost so that the seven vertical
+// offsets share their guide rows and staged values, and the weight's cut-off
+// as a SAD threshold, here of the sender's block: a lane's senders at one cx
+// lie in two block rows. The sums and their normaliser recomputed from the
+// guide in a pass of their own, and the offsets one by one, took 53 + 101 us
+// at 1024x1024; this takes 53.
+constexpr int kAdjEpfH = 16, kAdjEpfThreads = 16 * kAdjEpfH;
+constexpr int kAdjEpfGH = kAdjEpfH + 8;   // guide rows y0 - 4 .. y0 + 19
+constexpr int kAdjEpfGPlane = kAdjEpfGH * kEpfGRow;
+constexpr int kAdjEpfTH = kAdjEpfH + 6;   // gather tile rows y0 - 3 .. y0 + 18
+constexpr int kAdjEpfTW = kEpfW + 8;      // gather tile cols x0 - 4 .. x0 + 67
+constexpr size_t kAdjEpfSmemBytes = size_t(3) * kAdjEpfGPlane * 4 +
+                                    size_t(3) * kAdjEpfTH * kAdjEpfTW * 4;
 
-template <bool kGather>
-__global__ void __launch_bounds__(kEpfThreads, 2)
-    k_adj_epf_pass(int w, int h, const uint8_t* guide, const int32_t* sigma,
-                   const float* g_filt, const float* gv_in, float* out) {
+// CpAsync16, or 16 zero bytes.
+__device__ __forceinline__ void CpAsync16OrZero(void* smem, const void* gmem,
+                                                bool copy) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                   uint32_t(__cvta_generic_to_shared(smem))),
+               "l"(gmem), "r"(copy ? 16 : 0)
+               : "memory");
+}
+
+__global__ void __launch_bounds__(kAdjEpfThreads, 3)
+    k_adj_epf(int w, int h, const uint8_t* guide, const int32_t* sigma,
+              const float* g_filt, float* out) {
   extern __shared__ __align__(16) uint32_t adj_epf_smem[];
-  uint32_t* sg = adj_epf_smem;  // [3][kEpfGH][kEpfGRow]
+  uint32_t* sg = adj_epf_smem;  // [3][kAdjEpfGH][kEpfGRow]
   float(*tile)[kAdjEpfTH][kAdjEpfTW] =
       reinterpret_cast<float(*)[kAdjEpfTH][kAdjEpfTW]>(adj_epf_smem +
-                                                       kEpfGuideWords);
-  __shared__ int s_m64[6][10];  // mul * 64 of blocks y0/8-1.., x0/8-1..
-  const int x0 = blockIdx.x * kEpfW, y0 = blockIdx.y * kEpfH;
+                                                       3 * kAdjEpfGPlane);
+  // Blocks y0 / 8 - 1 .., x0 / 8 - 1 ..: mul * 64, the SAD threshold (-1:
+  // no weight) and the weight's bits beyond it.
+  __shared__ int4 s_cut[4][10];
+  const int x0 = blockIdx.x * kEpfW, y0 = blockIdx.y * kAdjEpfH;
   const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
   const int band = wp >> 1, col0 = 32 * (wp & 1);
   const size_t plane = size_t(w) * h;
   const int bw = w / 8, bh = h / 8;
   const int px = x0 + lane + col0, py0 = y0 + 4 * band;
   const bool inside = px < w && py0 < h;
-  const int sig = inside ? sigma[(py0 >> 3) * bw + (px >> 3)] : 0;
-  const bool filtered = sig >= kMinSigma;
-  // The u8 guide (6-pixel mirrored border) as words: bytes x0 - 8 ..
-  // x0 + 71 of rows y0 - 4 .. y0 + 35; bytes outside the buffer read 0.
-  const int gwid = w + 12, ght = h + 12;
-  constexpr int kAligned = kEpfGBytes / 4;
-  for (int i = tid; i < 3 * kEpfGH * kAligned; i += kEpfThreads) {
-    const int c = i / (kEpfGH * kAligned);
-    const int r = (i / kAligned) % kEpfGH, wd = i % kAligned;
-    const int gy = y0 - 4 + r;
-    uint32_t word = 0;
-    for (int b = 0; b < 4; ++b) {
-      const int gx = x0 - 8 + 4 * wd + b;
-      const bool ok = gx >= -6 && gx < w + 6 && gy >= -6 && gy < h + 6;
-      const uint32_t v =
-          ok ? guide[(size_t(c) * ght + gy + 6) * gwid + gx + 6] : 0u;
-      word |= v << (8 * b);
-    }
-    sg[c * kEpfGPlane + r * kEpfGRow + 4 * wd] = word;
-  }
-  if (kGather) {
-    // gv around the tile, 0 outside the frame (those terms are pass 3's).
-    for (int i = tid; i < 3 * kAdjEpfTH * kAdjEpfTW; i += kEpfThreads) {
-      const int c = i / (kAdjEpfTH * kAdjEpfTW);
-      const int r = (i / kAdjEpfTW) % kAdjEpfTH, col = i % kAdjEpfTW;
-      const int gx = x0 - 4 + col, gy = y0 - 3 + r;
-      tile[c][r][col] = (gx >= 0 && gx < w && gy >= 0 && gy < h)
-                            ? gv_in[c * plane + size_t(gy) * w + gx]
-                            : 0.0f;
-    }
-    for (int i = tid; i < 60; i += kEpfThreads) {
-      const int by = y0 / 8 - 1 + i / 10, bx = x0 / 8 - 1 + i % 10;
-      int m = 0;
-      if (by >= 0 && by < bh && bx >= 0 && bx < bw) {
-        const int sg_ = sigma[by * bw + bx];
-        m = sg_ >= kMinSigma ? c_t.mul_table[sg_] * 64 : 0;
+  bool sends = false;
+  if (tid < 40) {
+    const int by = y0 / 8 - 1 + tid / 10, bx = x0 / 8 - 1 + tid % 10;
+    int4 cut = make_int4(0, -1, 0, 0);
+    if (by >= 0 && by < bh && bx >= 0 && bx < bw) {
+      const int sg_ = sigma[by * bw + bx];
+      if (sg_ >= kMinSigma) {
+        const int m64 = c_t.mul_table[sg_] * 64;
+        const EpfCut k = EpfCutOf(sg_, m64);
+        cut = make_int4(m64, int(k.thr), __float_as_int(k.cap), 0);
+        sends = true;
       }
-      s_m64[i / 10][i % 10] = m;
     }
+    s_cut[tid / 10][tid % 10] = cut;
   }
+  if (!__syncthreads_or(sends)) {  // nothing around the tile was filtered
+    if (!inside) return;
+    for (int c = 0; c < 3; ++c)
+      for (int j = 0; j < 4; ++j) {
+        const size_t o = c * plane + size_t(py0 + j) * w + px;
+        out[o] += g_filt[o];
+      }
+    return;
+  }
+  // gv of the filtered pixels around the tile, 0 for the others and outside
+  // the frame (those terms are the border kernel's); four pixels of one block
+  // per copy.
+  constexpr int kQ = kAdjEpfTW / 4;
+  for (int i = tid; i < 3 * kAdjEpfTH * kQ; i += kAdjEpfThreads) {
+    const int c = i / (kAdjEpfTH * kQ);
+    const int r = (i / kQ) % kAdjEpfTH, q = i % kQ;
+    const int gx = x0 - 4 + 4 * q, gy = y0 - 3 + r;
+    const bool ok = gx >= 0 && gx < w && gy >= 0 && gy < h &&
+                    s_cut[(gy >> 3) - y0 / 8 + 1][(gx >> 3) - x0 / 8 + 1].x;
+    CpAsync16OrZero(&tile[c][r][4 * q],
+                    g_filt + (ok ? c * plane + size_t(gy) * w + gx : 0), ok);
+  }
+  // The u8 guide (6-pixel mirrored border) as words: bytes x0 - 8 ..
+  // x0 + 71 of rows y0 - 4 .. y0 + 19 from the aligned words of its rows
+  // (w + 12 is a multiple of 4); what lies outside the buffer reads 0.
+  const int gwid = w + 12, ght = h + 12;
+  constexpr int kAligned = kEpfGBytes / 4, kWords = 3 * kAdjEpfGH * kAligned;
+  constexpr int kTurns = (kWords + kAdjEpfThreads - 1) / kAdjEpfThreads;
+  uint32_t lo[kTurns], hi[kTurns];  // all of a thread's loads in flight
+#pragma unroll
+  for (int t = 0; t < kTurns; ++t) {
+    const int i = tid + t * kAdjEpfThreads;
+    const int c = i / (kAdjEpfGH * kAligned);
+    const int r = (i / kAligned) % kAdjEpfGH, wd = i % kAligned;
+    const int gy = y0 - 4 + r + 6, gx = x0 - 8 + 4 * wd + 6 - 2;
+    const uint8_t* row = guide + (size_t(c) * ght + gy) * gwid;
+    const bool in_row = i < kWords && gy >= 0 && gy < ght;
+    lo[t] = in_row && gx >= 0 && gx < gwid
+                ? *reinterpret_cast<const uint32_t*>(row + gx)
+                : 0u;
+    hi[t] = in_row && gx + 4 >= 0 && gx + 4 < gwid
+                ? *reinterpret_cast<const uint32_t*>(row + gx + 4)
+                : 0u;
+  }
+#pragma unroll
+  for (int t = 0; t < kTurns; ++t) {
+    const int i = tid + t * kAdjEpfThreads;
+    if (i < kWords) sg[4 * i] = __funnelshift_r(lo[t], hi[t], 16);
+  }
+  CpAsyncWaitAll();
   __syncthreads();
-  for (int i = tid; i < 3 * kEpfGH * kAligned * 3; i += kEpfThreads) {
-    const int sft = 1 + i % 3;
-    const int j = i / 3;
-    const int c = j / (kEpfGH * kAligned);
-    const int r = (j / kAligned) % kEpfGH, wd = j % kAligned;
-    const uint32_t* row = sg + c * kEpfGPlane + r * kEpfGRow;
-    const uint32_t lo = row[4 * wd];
-    const uint32_t hi = wd + 1 < kAligned ? row[4 * wd + 4] : 0u;
-    sg[c * kEpfGPlane + r * kEpfGRow + 4 * wd + sft] =
-        __funnelshift_r(lo, hi, 8 * sft);
+  // The words of the offsets between (bytes past the row end read as 0).
+  for (int i = tid; i < kWords; i += kAdjEpfThreads) {
+    const int wd = i % kAligned;
+    const uint32_t a = sg[4 * i];
+    const uint32_t b = wd + 1 < kAligned ? sg[4 * i + 4] : 0u;
+    sg[4 * i + 1] = __funnelshift_r(a, b, 8);
+    sg[4 * i + 2] = __funnelshift_r(a, b, 16);
+    sg[4 * i + 3] = __funnelshift_r(a, b, 24);
   }
   __syncthreads();
   if (!inside) return;  // no barrier follows
-  if (!kGather && !filtered) {
-    for (int c = 0; c < 3; ++c)
-      for (int j = 0; j < 4; ++j)
-        out[c * plane + size_t(py0 + j) * w + px] = 0.0f;
-    return;
-  }
   const int gr0 = 4 * band + 3;  // guide smem row of py0 - 1
-  uint32_t ref[3][6];
-  {
-    const uint32_t* g = sg + gr0 * kEpfGRow + lane + col0 + 7;
+  const int gc0 = lane + col0 + 7;
+  float acc[3][4];
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-      for (int r = 0; r < 6; ++r) ref[c][r] = g[c * kEpfGPlane + r * kEpfGRow];
-  }
-  const int m64c = filtered ? c_t.mul_table[sig] * 64 : 0;
-  float acc[3][4], sw[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    acc[0][j] = acc[1][j] = acc[2][j] = 0.f;
-    sw[j] = 0.f;
-  }
-  constexpr int kCx0 = kGather ? -4 : -3;
+  for (int j = 0; j < 4; ++j) acc[0][j] = acc[1][j] = acc[2][j] = 0.f;
+  // Sender rows py0 - 3 + R, R = 0..9, lie in block rows first (R < 3, or
+  // R < 7 if py0 is in a block's lower half) and first + 1.
+  const bool low = (py0 & 4) != 0;
+  const int first = (py0 >> 3) - y0 / 8 + (low ? 1 : 0);
 #pragma unroll 1
-  for (int cy = -3; cy <= 3; ++cy) {
-#pragma unroll 1
-    for (int cx = kCx0; cx <= kCx0 + 7; ++cx) {
-      const uint32_t* g = sg + (gr0 + cy) * kEpfGRow + lane + col0 + 7 + cx;
-      int sad[4] = {0, 0, 0, 0};
+  for (int cx = -4; cx <= 3; ++cx) {
+    const uint32_t* g = sg + (gr0 - 3) * kEpfGRow + gc0 + cx;
+    uint32_t sad[7][4];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        int hs[6];
+    for (int c = 0; c < 3; ++c) {
+      uint32_t wd[12];
 #pragma unroll
-        for (int r = 0; r < 6; ++r) {
-          hs[r] = int(__vsadu4(ref[c][r], g[c * kEpfGPlane + r * kEpfGRow]));
-        }
-        const int p12 = hs[1] + hs[2], p34 = hs[3] + hs[4];
-        sad[0] = max(sad[0], hs[0] + p12);
-        sad[1] = max(sad[1], p12 + hs[3]);
-        sad[2] = max(sad[2], hs[2] + p34);
-        sad[3] = max(sad[3], p34 + hs[5]);
+      for (int t = 0; t < 12; ++t) wd[t] = g[c * kAdjEpfGPlane + t * kEpfGRow];
+      uint32_t rf[6];
+#pragma unroll
+      for (int r = 0; r < 6; ++r) {
+        rf[r] = sg[c * kAdjEpfGPlane + (gr0 + r) * kEpfGRow + gc0];
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (kGather) {
-          // The sending pixel q + e and its block's weight multiplier.
-          const int sy = py0 + j + cy, sx = px + cx;
-          const int m = s_m64[(sy >> 3) - y0 / 8 + 1][(sx >> 3) - x0 / 8 + 1];
-          float wgt = EpfWeight(m, sad[j]);
-          if (!(wgt >= 0.05f) || m == 0) wgt = 0.0f;
-          const int tr = 4 * band + j + 3 + cy, tc = lane + col0 + 4 + cx;
-          acc[0][j] = fmaf(tile[0][tr][tc], wgt, acc[0][j]);
-          acc[1][j] = fmaf(tile[1][tr][tc], wgt, acc[1][j]);
-          acc[2][j] = fmaf(tile[2][tr][tc], wgt, acc[2][j]);
+      for (int k = 0; k < 7; ++k) {
+        if (c == 0) {
+          PatchSads<true, 4>(rf, wd + k, sad[k]);
         } else {
-          float wgt = EpfWeight(m64c, sad[j]);
-          if (!(wgt >= 0.05f)) wgt = 0.0f;
-          sw[j] += wgt;
+          PatchSads<false, 4>(rf, wd + k, sad[k]);
         }
       }
     }
+    const int bxi = ((px + cx) >> 3) - x0 / 8 + 1;
+    const int4 up = s_cut[first][bxi], dn = s_cut[first + 1][bxi];
+    const int4 mid = low ? up : dn;
+    const int col = lane + col0 + 4 + cx;
+#pragma unroll
+    for (int R = 0; R < 10; ++R) {
+      const int4 cut = R < 3 ? up : R >= 7 ? dn : mid;
+      const int tr = 4 * band + R;
+      const float v0 = tile[0][tr][col], v1 = tile[1][tr][col],
+                  v2 = tile[2][tr][col];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int k = R - j;  // cy + 3
+        if (k < 0 || k > 6) continue;
+        const uint32_t u = sad[k][j] * uint32_t(cut.x) + 0x3F800000u;
+        const float wgt = int(sad[k][j]) <= cut.y
+                              ? __uint_as_float(u & 0xFFFF0000u)
+                              : __int_as_float(cut.z);
+        acc[0][j] = fmaf(v0, wgt, acc[0][j]);
+        acc[1][j] = fmaf(v1, wgt, acc[1][j]);
+        acc[2][j] = fmaf(v2, wgt, acc[2][j]);
+      }
+    }
   }
+  const bool filtered = sigma[(py0 >> 3) * bw + (px >> 3)] >= kMinSigma;
 #pragma unroll
   for (int c = 0; c < 3; ++c)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const size_t o = c * plane + size_t(py0 + j) * w + px;
-      if (kGather) {
-        out[o] += acc[c][j] + (filtered ? 0.0f : g_filt[o]);
-      } else {
-        out[o] = g_filt[o] / sw[j];
-      }
+      out[o] += acc[c][j] + (filtered ? 0.0f : g_filt[o]);
     }
 }
 
@@ -1062,7 +1102,8 @@ __global__ void __launch_bounds__(32 * kAdjQfCells)
   double s = 0.0;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const float2 u = *reinterpret_cast<const float2*>(g_coef + c * plane_ac + o);
+    const float2 u =
+        *reinterpret_cast<const float2*>(g_coef + c * plane_ac + o);
     const float2 v = *reinterpret_cast<const float2*>(ac0 + c * plane_ac + o);
     s += double(u.x) * double(v.x);
     s += double(u.y) * double(v.y);
@@ -1140,42 +1181,42 @@ int LaunchAdjoint(pikgpu_ctx* ctx, const float* target) {
     const int32_t* sig = P<int32_t>(ctx->sigma);
     const uint8_t* tape = P<uint8_t>(ctx->adj_tape);
     const float* epf = P<float>(ctx->dbg_epf);
+    const float* sum_w = P<float>(ctx->adj_sw);
     // g_filt goes to ga (g_pre is dead once g_cur exists; without
     // gaborish g_cur is ga itself, so g_filt then takes gb).
     float* g_filt = s.gaborish ? ga : gb;
     if (n[kC8]) {
       k_adj_ar_dct8<<<Blocks(n[kC8], SquareArBlocks<8>()), kSquareArThreads, 0,
                       st>>>(
-          g, f, s, L[kC8], n[kC8], sig, tape, epf, g_cur, g_filt, gc, g_qf);
+          g, f, s, L[kC8], n[kC8], sig, tape, epf, sum_w, g_cur, g_filt, gc,
+          g_qf);
       ++ctx->launches;
     }
     if (n[kC4] + n[kCSmall]) {
       k_adj_ar8<<<Blocks(n[kC4] + n[kCSmall], kAdj8Blocks), kAdjThreads, 0,
-                  st>>>(g, f, s, J, lists8, sig, tape, epf, g_cur, g_filt, gc, g_qf);
+                  st>>>(g, f, s, J, lists8, sig, tape, epf, sum_w, g_cur,
+                        g_filt, gc, g_qf);
       ++ctx->launches;
     }
     if (n[kC16]) {
       k_adj_ar_sq<16><<<n[kC16], kAdjThreads, 0, st>>>(
-          g, f, s, L[kC16], n[kC16], sig, tape, epf, g_cur, g_filt, gc,
+          g, f, s, L[kC16], n[kC16], sig, tape, epf, sum_w, g_cur, g_filt, gc,
           g_qf);
       ++ctx->launches;
     }
     if (n[kC32]) {
       k_adj_ar_sq<32><<<n[kC32], kAdjThreads, 0, st>>>(
-          g, f, s, L[kC32], n[kC32], sig, tape, epf, g_cur, g_filt, gc,
+          g, f, s, L[kC32], n[kC32], sig, tape, epf, sum_w, g_cur, g_filt, gc,
           g_qf);
       ++ctx->launches;
     }
-    // gv = g_filt / sum_w in the plane g_cur no longer needs.
-    float* gv = g_filt == ga ? gb : ga;
-    dim3 gr(Blocks(g.PW, kEpfW), Blocks(g.PH, kEpfH));
-    k_adj_epf_pass<false><<<gr, kEpfThreads, kAdjEpfSmemBytes, st>>>(
-        g.PW, g.PH, guide, sig, g_filt, nullptr, gv);
-    k_adj_epf_pass<true><<<gr, kEpfThreads, kAdjEpfSmemBytes, st>>>(
-        g.PW, g.PH, guide, sig, g_filt, gv, gc);
+    dim3 gr(Blocks(g.PW, kEpfW), Blocks(g.PH, kAdjEpfH));
+    k_adj_epf<<<gr, kAdjEpfThreads, kAdjEpfSmemBytes, st>>>(
+        g.PW, g.PH, guide, sig, g_filt, gc);
     k_adj_epf_border<<<Blocks(AdjBandPixels(g.PW, g.PH), kAdjBand),
-                       64 * kAdjBand, 0, st>>>(g.PW, g.PH, guide, sig, gv, gc);
-    ctx->launches += 3;
+                       64 * kAdjBand, 0, st>>>(g.PW, g.PH, guide, sig, g_filt,
+                                              gc);
+    ctx->launches += 2;
     g_idct = gc;
   }
   // g_up: the upsampled-prediction gradient (zero outside HF blocks), in
@@ -1339,6 +1380,7 @@ int pikgpu_adjoint(pikgpu_ctx* ctx, const float* target, double* loss,
                    sizeof(double) * (kAdjLossBlocks + 1))) ||
       (rc = Ensure(ctx, &ctx->adj_jac, sizeof(AdjJac))) ||
       (rc = Ensure(ctx, &ctx->adj_tape, nac)) ||
+      (rc = Ensure(ctx, &ctx->adj_sw, 4 * npx)) ||
       (rc = Ensure(ctx, &ctx->dbg_dequant, 4 * 3 * nac)) ||
       (rc = Ensure(ctx, &ctx->dbg_epf, 4 * 3 * npx)) ||
       (rc = Ensure(ctx, &ctx->dbg_pre, 4 * ntg))) {
@@ -1347,12 +1389,7 @@ int pikgpu_adjoint(pikgpu_ctx* ctx, const float* target, double* loss,
   cudaStream_t st = ctx->stream;
   if (!ctx->adj_jac_built) {
     CUDA_TRY(ctx, cudaFuncSetAttribute(
-                      k_adj_epf_pass<false>,
-                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                      int(kAdjEpfSmemBytes)));
-    CUDA_TRY(ctx, cudaFuncSetAttribute(
-                      k_adj_epf_pass<true>,
-                      cudaFuncAttributeMaxDynamicSharedMemorySize,
+                      k_adj_epf, cudaFuncAttributeMaxDynamicSharedMemorySize,
                       int(kAdjEpfSmemBytes)));
     k_adj_build_jac<<<2 * kJTypes + 9, 64, 0, st>>>(P<AdjJac>(ctx->adj_jac));
     CUDA_TRY(ctx, cudaGetLastError());

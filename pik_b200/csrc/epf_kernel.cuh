@@ -140,11 +140,14 @@ __device__ __forceinline__ void PatchSads(const uint32_t* rf,
 // all taken; its blocks share one sigma (SigmaFromQuant of the constant
 // `dc_qf` with a DCT strategy and LUT 0, AdaptiveDCReconstruction,
 // pik/adaptive_reconstruction.cc:300-318).
+// `sum_w` (NULL: not written): the plane of the filtered pixels' weight sums,
+// for the adjoint.
 struct EpfWork {
   const uint32_t* list;
   const int* count;
   const int32_t* sigma;
   int dc_qf;
+  float* sum_w;
 };
 constexpr int kEpfRegionH = kRegionH;  // every tile height divides it
 static_assert(kEpfW == kRegionW, "a region is as wide as a tile");
@@ -334,7 +337,7 @@ __host__ __device__ constexpr int EpfThreads() {
 // this thread's block, and stores the result. No CTA barrier.
 template <bool kFma, int TH, int ROWS>
 __device__ __forceinline__ void EpfFilterCore(
-    int tid, int sig, float* out, const EpfDc& dco, int w, int h,
+    int tid, int sig, float* out, float* sum_w, const EpfDc& dco, int w, int h,
     const uint32_t* sg, float (*tile)[TH + 10][kEpfTS], int x0, int y0) {
   constexpr int kGH = TH + 8;
   constexpr int kGPlane = kGH * kEpfGRow;
@@ -470,6 +473,10 @@ __device__ __forceinline__ void EpfFilterCore(
     }
   }
   if (!inside) return;
+  if (sum_w) {
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) sum_w[size_t(py0 + j) * w + px] = sw[j];
+  }
   // The normalisation: an IEEE division in the FP32 form (the reference's
   // rounding); in the tensor-core forms one reciprocal per row (the weight
   // sum is in [1, 56]) and a multiply per channel, within 2 ulp.
@@ -499,8 +506,8 @@ __device__ __forceinline__ void EpfFilterCore(
 template <bool kFma, int TH, int ROWS>
 __device__ __forceinline__ void EpfFilterTile(
     const uint8_t* guide_ovr, int gab, int w, int h, float amin, float mul,
-    int sig, float* out, const EpfDc& dco, uint32_t* sg, uint32_t* sa,
-    float (*tile)[TH + 10][kEpfTS], int x0, int y0) {
+    int sig, float* out, float* sum_w, const EpfDc& dco, uint32_t* sg,
+    uint32_t* sa, float (*tile)[TH + 10][kEpfTS], int x0, int y0) {
   const int tid = threadIdx.x;
   // Tiles without filtered blocks are copies (CopyOriginalBlock): every warp
   // copies, and no guide is needed.
@@ -509,7 +516,8 @@ __device__ __forceinline__ void EpfFilterTile(
                                               guide_ovr, gab, w, h, amin, mul,
                                               sg, sa, tile, x0, y0);
   }
-  EpfFilterCore<kFma, TH, ROWS>(tid, sig, out, dco, w, h, sg, tile, x0, y0);
+  EpfFilterCore<kFma, TH, ROWS>(tid, sig, out, sum_w, dco, w, h, sg, tile, x0,
+                                y0);
 }
 
 // One CTA per 64 x TH tile (1-D grid). More CTAs than resident slots balance
@@ -604,8 +612,9 @@ __global__ void __launch_bounds__(EpfThreads<TH, ROWS>(), TH == 16 ? 3 : 2)
   } else {
     CpAsyncWaitAll();
   }
-  EpfFilterTile<kFma, TH, ROWS>(guide_ovr, gab, w, h, amin, mul, sig, out, dco,
-                                sg, sa, tile, x0, y0);
+  EpfFilterTile<kFma, TH, ROWS>(guide_ovr, gab, w, h, amin, mul, sig, out,
+                                kList ? work.sum_w : nullptr, dco, sg, sa,
+                                tile, x0, y0);
 }
 
 }  // namespace pikgpu

@@ -124,7 +124,7 @@ struct pikgpu_ctx {
   // pred2x2 gradient, quant-field gradient, guide bytes, loss partials,
   // per-type Jacobians, host target staging.
   DevBuf adj_a, adj_b, adj_c, adj_coef, adj_pred, adj_qf, adj_guide;
-  DevBuf adj_partial, adj_jac, adj_target, adj_tape;
+  DevBuf adj_partial, adj_jac, adj_target, adj_tape, adj_sw;
   bool adj_jac_built = false;
   // The clamp kernels record their branches (the clamp tape) in the
   // adjoint's forward pass and with PIKGPU_OPT_KEEP_STAGES; tape_valid: the
@@ -887,6 +887,7 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
     work.list = plan.region_list;
     work.count = plan.region_count;
     work.sigma = plan.sigma;
+    work.sum_w = ctx->record_tape ? P<float>(ctx->adj_sw) : nullptr;
     EpfLaunch(st, ctx->num_sms, ctx->form, f.idct, gab, g.PW, g.PH,
               mm, work, f.filt,
               ctx->use_guide_ovr ? P<uint8_t>(ctx->guide_ovr) : nullptr,
@@ -1135,6 +1136,7 @@ int pikgpu_ctx_destroy(pikgpu_ctx* ctx) {
                     &ctx->adj_c,   &ctx->adj_coef,  &ctx->adj_pred,
                     &ctx->adj_qf,  &ctx->adj_guide, &ctx->adj_partial,
                     &ctx->adj_jac, &ctx->adj_target, &ctx->adj_tape,
+                    &ctx->adj_sw,
                     &ctx->tape_in, &ctx->pnm};
   for (DevBuf* b : bufs) FreeBuf(b);
   for (auto& b : ctx->list) FreeBuf(&b);

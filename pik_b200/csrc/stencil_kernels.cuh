@@ -207,9 +207,9 @@ __device__ __forceinline__ void StripRow6(const float4& q, float (&v)[6]) {
 // that strength): the verification export and the adjoint's guide. A word of
 // four pixels per thread (w + 12 is a multiple of 4), from the values at the
 // mirrored coordinates around it, which is the smoothed value at the mirrored
-// position: Sym3Rows adds each pair of neighbours first. At 1024x1024 a pixel per
-// thread took 26 us, and with the smoothed plane written and read again 37
-// and a host synchronisation; this takes 14.
+// position: Sym3Rows adds each pair of neighbours first. At 1024x1024 a pixel
+// per thread took 26 us, and with the smoothed plane written and read again
+// 37 and a host synchronisation; this takes 14.
 __global__ void __launch_bounds__(256)
     k_export_guide(const float* src, int gab, int w, int h, const uint32_t* mm,
                    uint8_t* guide) {
