@@ -630,7 +630,8 @@ __global__ void __launch_bounds__(kSquareArThreads)
 // as a SAD threshold, here of the sender's block: a lane's senders at one cx
 // lie in two block rows. The sums and their normaliser recomputed from the
 // guide in a pass of their own, and the offsets one by one, took 53 + 101 us
-// at 1024x1024; this takes 53.
+// at 1024x1024; this takes 52, and
+// 59 with eight rows per lane, which leaves the last wave of CTAs empty.
 constexpr int kAdjEpfH = 16, kAdjEpfThreads = 16 * kAdjEpfH;
 constexpr int kAdjEpfGH = kAdjEpfH + 8;   // guide rows y0 - 4 .. y0 + 19
 constexpr int kAdjEpfGPlane = kAdjEpfGH * kEpfGRow;
@@ -785,17 +786,26 @@ __global__ void __launch_bounds__(kAdjEpfThreads, 3)
       const int tr = 4 * band + R;
       const float v0 = tile[0][tr][col], v1 = tile[1][tr][col],
                   v2 = tile[2][tr][col];
+      auto weight = [&](int k, int j) {
+        const uint32_t u = sad[k][j] * uint32_t(cut.x) + 0x3F800000u;
+        return int(sad[k][j]) <= cut.y ? __uint_as_float(u & 0xFFFF0000u)
+                                       : __int_as_float(cut.z);
+      };
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int k = R - j;  // cy + 3
         if (k < 0 || k > 6) continue;
-        const uint32_t u = sad[k][j] * uint32_t(cut.x) + 0x3F800000u;
-        const float wgt = int(sad[k][j]) <= cut.y
-                              ? __uint_as_float(u & 0xFFFF0000u)
-                              : __int_as_float(cut.z);
-        acc[0][j] = fmaf(v0, wgt, acc[0][j]);
-        acc[1][j] = fmaf(v1, wgt, acc[1][j]);
-        acc[2][j] = fmaf(v2, wgt, acc[2][j]);
+        if (j % 2 == 0 && k > 0) {  // with row j + 1, whose offset is k - 1
+          const float w0 = weight(k, j), w1 = weight(k - 1, j + 1);
+          Fma2(acc[0][j], acc[0][j + 1], v0, w0, w1);
+          Fma2(acc[1][j], acc[1][j + 1], v1, w0, w1);
+          Fma2(acc[2][j], acc[2][j + 1], v2, w0, w1);
+        } else if (j % 2 == 0 || k == 6) {
+          const float w0 = weight(k, j);
+          acc[0][j] = fmaf(v0, w0, acc[0][j]);
+          acc[1][j] = fmaf(v1, w0, acc[1][j]);
+          acc[2][j] = fmaf(v2, w0, acc[2][j]);
+        }
       }
     }
   }

@@ -11,8 +11,8 @@
 // of a patch row at any offset are then one 32-bit load (and the 32 lanes'
 // loads of 32 consecutive offsets hit 32 consecutive words, free of bank
 // conflicts), and the sum of absolute differences against the centre
-// pixel's patch row is one __vsadu4. For every displacement (cy, cx) of the 7 x 8 neighbourhood and
-// every channel, a lane forms ROWS + 2 patch-row SADs of its column and
+// pixel's patch row is one __vsadu4. For every displacement (cy, cx) of the
+// 7 x 8 neighbourhood and every channel, a lane forms ROWS + 2 patch-row SADs of its column and
 // sums them vertically into the 3 x 4 patch SADs of its rows; the SAD is
 // the maximum over the channels. The SADs are exact integers; the weights
 // (WeightFast's bit construction) and the weighted sums follow the
@@ -27,25 +27,28 @@
 // its strength). Border tiles hold mirrored values and take the same steps:
 // 402 -> 380 us at 3001x2003, 22 -> 14 on the DC image of a 256x256 frame,
 // against mirroring every guide byte's coordinates.
+// Bound by the issue slots and the shared-memory reads. A thread takes eight
+// rows, a whole block row: against four, ten row SADs serve eight patches
+// instead of six serving four, and fewer guide rows are read per pixel; the
+// packed products and sums (packed_fp32.cuh) take another 4% (FP32) and 5%.
+// Together 220 -> 198 us on a 4K frame with a third of the blocks filtered
+// (FP32; split-BF16 176 -> 164) and 375 -> 342 at 3001x2003 with all of them.
+// Tiles of 32 rows: 8% slower (two CTAs fewer per SM).
 // Included by recon_kernels.cu.
 #pragma once
 
 namespace pikgpu {
 
-constexpr int kEpfW = 64, kEpfH = 32;   // output tile (TH = kEpfH)
-constexpr int kEpfThreads = 16 * kEpfH;  // four rows per thread
-constexpr int kEpfGH = kEpfH + 8;       // guide rows: y0 - 4 .. y0 + 35
+constexpr int kEpfW = 64;               // tile width
+constexpr int kEpfH = 16, kEpfRows = 8;  // its rows, and those of a thread
 constexpr int kEpfGBytes = 80;          // guide bytes x0 - 8 .. x0 + 71
 constexpr int kEpfGRow = kEpfGBytes;    // words per guide row (one per byte)
-constexpr int kEpfGPlane = kEpfGH * kEpfGRow;
 // Input tile with a 5-pixel halo (enough for gaborish at the guide's
-// 4-pixel halo): rows y0 - 5 .. y0 + 36, cols x0 - 12 .. x0 + 75 (the
+// 4-pixel halo): rows y0 - 5 .. y0 + TH + 4, cols x0 - 12 .. x0 + 75 (the
 // column range is widened to 16-byte boundaries for vector loads).
-constexpr int kEpfTH = kEpfH + 10;
 constexpr int kEpfTW = kEpfW + 24;
 constexpr int kEpfTS = kEpfTW;               // row stride in floats
 constexpr int kEpfTRow0 = 2, kEpfTCol0 = 9;  // tile index of (y0-3, x0-3)
-constexpr size_t kEpfGuideWords = size_t(3) * kEpfGPlane;
 constexpr int kEpfAligned = kEpfGBytes / 4;  // aligned guide words per row
 // Shared memory of k_epf_box with a tile of `th` rows: the guide words (one
 // per byte offset), the input tile and the aligned guide words.
@@ -100,16 +103,35 @@ __device__ __forceinline__ uint32_t Sad4(uint32_t a, uint32_t b, uint32_t c) {
   return d;
 }
 
-// The 3-row patch SADs of R = 4, 2 or 1 pixel rows from R + 2 patch-row
-// pairs (centre row r against window row r): for four rows six byte-SADs
-// (rows 1 + 2 and 3 + 4 accumulated onto rows 2 and 3, rows 0 and 5 onto
-// those pairs) and two adds, which need not run on the integer ALU. c0: the
-// first channel (no maximum).
+// The 3-row patch SADs of R = 8, 4, 2 or 1 pixel rows from R + 2 patch-row
+// pairs (centre row r against window row r): for eight rows ten byte-SADs,
+// where the sums of two neighbouring rows accumulate one onto the other, and
+// eight adds, which need not run on the integer ALU. c0: the first channel
+// (no maximum).
 template <bool c0, int R>
 __device__ __forceinline__ void PatchSads(const uint32_t* rf,
                                           const uint32_t* wd, uint32_t* sad) {
+  static_assert(R == 8 || R == 4 || R == 2 || R == 1, "rows per thread");
   uint32_t s[R];
-  if constexpr (R == 4) {
+  if constexpr (R == 8) {
+    const uint32_t h2 = Sad4(rf[2], wd[2], 0u);
+    const uint32_t h3 = Sad4(rf[3], wd[3], 0u);
+    const uint32_t h4 = Sad4(rf[4], wd[4], 0u);
+    const uint32_t h5 = Sad4(rf[5], wd[5], 0u);
+    const uint32_t h7 = Sad4(rf[7], wd[7], 0u);
+    const uint32_t p12 = Sad4(rf[1], wd[1], h2);
+    const uint32_t p34 = h3 + h4;
+    const uint32_t p56 = Sad4(rf[6], wd[6], h5);
+    const uint32_t p78 = Sad4(rf[8], wd[8], h7);
+    s[0] = Sad4(rf[0], wd[0], p12);
+    s[1] = p12 + h3;
+    s[2] = p34 + h2;
+    s[3] = p34 + h5;
+    s[4] = p56 + h4;
+    s[5] = p56 + h7;
+    s[6] = p78 + (p56 - h5);
+    s[7] = Sad4(rf[9], wd[9], p78);
+  } else if constexpr (R == 4) {
     const uint32_t h2 = Sad4(rf[2], wd[2], 0u);
     const uint32_t h3 = Sad4(rf[3], wd[3], 0u);
     const uint32_t p12 = Sad4(rf[1], wd[1], h2);
@@ -379,9 +401,10 @@ __device__ __forceinline__ void EpfFilterCore(
     // Tensor-core forms: cx outermost. For one cx the 7 vertical offsets
     // read ROWS + 8 distinct guide rows per channel (one load each), and
     // each staged input row serves every pixel of the lane it reaches: for
-    // four rows about 84 shared-memory loads per cx and lane instead of 210. Each pixel's
-    // sums run cx-major, not in the reference's cy-major order (these
-    // forms are not bound to its rounding).
+    // eight rows about 120 shared-memory loads per cx and lane instead of
+    // 378. Each pixel's sums run cx-major, not in the reference's cy-major
+    // order (these forms are not bound to its rounding), two neighbouring
+    // rows' at a time.
 #pragma unroll 1
     for (int cx = -3; cx <= 4; ++cx) {
       const uint32_t* g = sg + (gr0 - 3) * kEpfGRow + gc0 + cx;
@@ -427,14 +450,21 @@ __device__ __forceinline__ void EpfFilterCore(
         for (int j = 0; j < ROWS; ++j) {
           const int k = R - j;  // cy + 3
           if (k < 0 || k > 6) continue;
-          ws[0][j] = fmaf(v0, wt[j][k], ws[0][j]);
-          ws[1][j] = fmaf(v1, wt[j][k], ws[1][j]);
-          ws[2][j] = fmaf(v2, wt[j][k], ws[2][j]);
+          if (j % 2 == 0 && j + 1 < ROWS && k > 0) {
+            Fma2(ws[0][j], ws[0][j + 1], v0, wt[j][k], wt[j + 1][k - 1]);
+            Fma2(ws[1][j], ws[1][j + 1], v1, wt[j][k], wt[j + 1][k - 1]);
+            Fma2(ws[2][j], ws[2][j + 1], v2, wt[j][k], wt[j + 1][k - 1]);
+          } else if (j % 2 == 0 || k == 6) {  // no such pair
+            ws[0][j] = fmaf(v0, wt[j][k], ws[0][j]);
+            ws[1][j] = fmaf(v1, wt[j][k], ws[1][j]);
+            ws[2][j] = fmaf(v2, wt[j][k], ws[2][j]);
+          }
         }
       }
     }
   } else {
-    // The reference's order: cy-major, products and sums rounded separately.
+    // The reference's order: cy-major, products and sums rounded separately
+    // (two rows' products in one instruction).
     uint32_t ref[3][ROWS + 2];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
@@ -443,7 +473,7 @@ __device__ __forceinline__ void EpfFilterCore(
         ref[c][r] = sg[c * kGPlane + (gr0 + r) * kEpfGRow + gc0];
 #pragma unroll 1
     for (int cy = -3; cy <= 3; ++cy) {
-#pragma unroll(ROWS == 4 ? 1 : 4)
+#pragma unroll(ROWS > 2 ? 1 : 4)
       for (int cx = -3; cx <= 4; ++cx) {
         // Window byte offset: the patch start moved by cx.
         const uint32_t* g = sg + (gr0 + cy) * kEpfGRow + gc0 + cx;
@@ -460,14 +490,27 @@ __device__ __forceinline__ void EpfFilterCore(
           }
         }
         const int col = tc0 + cx;
+        float wt[ROWS];
 #pragma unroll
-        for (int j = 0; j < ROWS; ++j) {
+        for (int j = 0; j < ROWS; ++j) wt[j] = EpfCutWeight(m64, cut, sad[j]);
+#pragma unroll
+        for (int j = 0; j < ROWS; j += 2) {
           const int ir = tr0 + j + cy;
-          const float wgt = EpfCutWeight(m64, cut, sad[j]);
-          ws[0][j] += tile[0][ir][col] * wgt;
-          ws[1][j] += tile[1][ir][col] * wgt;
-          ws[2][j] += tile[2][ir][col] * wgt;
-          sw[j] += wgt;
+          if constexpr (ROWS == 1) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) ws[c][j] += tile[c][ir][col] * wt[j];
+            sw[j] += wt[j];
+          } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              float p0, p1;
+              Mul2(p0, p1, tile[c][ir][col], tile[c][ir + 1][col], wt[j],
+                   wt[j + 1]);
+              ws[c][j] += p0;
+              ws[c][j + 1] += p1;
+            }
+            Add2(sw[j], sw[j + 1], wt[j], wt[j + 1]);
+          }
         }
       }
     }
@@ -543,7 +586,7 @@ __device__ __forceinline__ void EpfFilterTile(
 // bounded, so that no copy is in flight when the CTA exits. Border tiles,
 // and all tiles without a tensor map, are staged with cp.async (EpfStage).
 template <bool kFma, int TH, int ROWS, bool kList>
-__global__ void __launch_bounds__(EpfThreads<TH, ROWS>(), TH == 16 ? 3 : 2)
+__global__ void __launch_bounds__(EpfThreads<TH, ROWS>(), ROWS < 8 ? 2 : kFma ? 3 : 4)
     k_epf_box(const float* in, const uint8_t* guide_ovr, int gab, int w, int h,
               const uint32_t* mm, EpfWork work, float* out, EpfDc dco,
               const __grid_constant__ CUtensorMap tmap, int use_tma,

@@ -401,30 +401,24 @@ void ComputeScalars(const pikgpu_frame_params* p, FrameScalars* s) {
   s->epf_fixed_sigma = p->epf_enable_adaptive ? -1 : int(p->epf_sigma);
 }
 
-// Calls fn with the EPF kernel of a form, tile height, rows per thread and
-// kind of work. The tensor-core forms' 16-row tiles have 256 threads, three
-// CTAs per SM: their cx-major loop needs ~85 registers.
+// Calls fn with the EPF kernel of a form, rows per thread and kind of work.
 template <typename Fn>
-void ForEpfKernel(bool fma, int th, int rows, bool list, Fn&& fn) {
-  auto pick = [&](auto r) {
-    constexpr int R = decltype(r)::value;
+void ForEpfKernel(bool fma, int rows, bool list, Fn&& fn) {
+  auto pick = [&](auto t, auto r) {
+    constexpr int TH = decltype(t)::value, R = decltype(r)::value;
     if (list) {
-      fma ? fn(k_epf_box<true, 8, R, true>) : fn(k_epf_box<false, 8, R, true>);
+      fma ? fn(k_epf_box<true, TH, R, true>)
+          : fn(k_epf_box<false, TH, R, true>);
     } else {
-      fma ? fn(k_epf_box<true, 8, R, false>)
-          : fn(k_epf_box<false, 8, R, false>);
+      fma ? fn(k_epf_box<true, TH, R, false>)
+          : fn(k_epf_box<false, TH, R, false>);
     }
   };
-  if (th == 8) {
-    rows == 1 ? pick(std::integral_constant<int, 1>())
-              : pick(std::integral_constant<int, 2>());
-  } else if (list) {
-    fma ? fn(k_epf_box<true, 16, 4, true>)
-        : fn(k_epf_box<false, kEpfH, 4, true>);
-  } else {
-    fma ? fn(k_epf_box<true, 16, 4, false>)
-        : fn(k_epf_box<false, kEpfH, 4, false>);
-  }
+  using std::integral_constant;
+  rows == 1   ? pick(integral_constant<int, 8>(), integral_constant<int, 1>())
+  : rows == 2 ? pick(integral_constant<int, 8>(), integral_constant<int, 2>())
+              : pick(integral_constant<int, kEpfH>(),
+                     integral_constant<int, kEpfRows>());
 }
 
 int UploadTables(pikgpu_ctx* ctx) {
@@ -436,10 +430,10 @@ int UploadTables(pikgpu_ctx* ctx) {
   CUDA_TRY(ctx, cudaMemcpyToSymbol(g_t, &t, sizeof(t)));
   for (int i = 0; i < 12; ++i) {  // every EPF kernel
     const bool fma = i & 1, list = i & 2;
-    const int rows = i < 4 ? 1 : i < 8 ? 2 : 4;
-    const int th = rows < 4 ? 8 : fma ? 16 : kEpfH;
+    const int rows = i < 4 ? 1 : i < 8 ? 2 : kEpfRows;
+    const int th = rows < kEpfRows ? 8 : kEpfH;
     cudaError_t e = cudaSuccess;
-    ForEpfKernel(fma, th, rows, list, [&](auto kernel) {
+    ForEpfKernel(fma, rows, list, [&](auto kernel) {
       e = cudaFuncSetAttribute(kernel,
                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                int(EpfSmemBytes(th)));
@@ -578,17 +572,17 @@ void EpfLaunch(cudaStream_t st, int num_sms, int form, const float* in,
                int gab, int w, int h, const uint32_t* mm, const EpfWork& work, float* out,
                const uint8_t* guide_ovr, const EpfDc& dco, int* err,
                uint32_t polls = tc::kMaxPolls, bool pdl = false) {
-  // Images that fill fewer than two CTAs per SM with 32-row tiles (the DC
-  // image, small frames) take 8-row tiles with fewer rows per thread: more
-  // CTAs and threads, a shorter chain in each. With 8-row tiles of four rows
-  // per thread the DC EPF of a 4K frame took 33 us (FP32; 29 split-BF16),
-  // with one row 19 (16); on a 1030x530 frame two rows took 25 us, four 31,
-  // one 29; up to 5 CTAs per SM instead of 2 made 1600x900 5% slower.
+  // Images of fewer than two 64 x 32 regions per SM (the DC image, small
+  // frames) take 8-row tiles with fewer rows per thread: more CTAs and
+  // threads, a shorter chain in each. With 8-row tiles of four rows per thread
+  // the DC EPF of a 4K frame took 33 us (FP32; 29 split-BF16), with one row
+  // 19 (16); on a 1030x530 frame two rows took 25 us, four 31, one 29; at
+  // 1600x900 the small tiles made the frame 5% slower.
   const bool fma = form != PIKGPU_FORM_FP32;
-  const bool small = Blocks(w, kEpfW) * Blocks(h, kEpfH) < 2 * num_sms;
+  const bool small = Blocks(w, kEpfW) * Blocks(h, kEpfRegionH) < 2 * num_sms;
   const int tiles8 = Blocks(w, kEpfW) * Blocks(h, 8);
-  const int rows = !small ? 4 : tiles8 <= 2 * num_sms ? 1 : 2;
-  const int th = small ? 8 : fma ? 16 : kEpfH;
+  const int rows = !small ? kEpfRows : tiles8 <= 2 * num_sms ? 1 : 2;
+  const int th = small ? 8 : kEpfH;
   CUtensorMap map;
   memset(&map, 0, sizeof(map));
   const int tma = err && EpfTileMap(&map, in, w, h, th) ? 1 : 0;
@@ -597,7 +591,7 @@ void EpfLaunch(cudaStream_t st, int num_sms, int form, const float* in,
                    (work.list ? Blocks(h, kEpfRegionH) * (kEpfRegionH / th)
                               : Blocks(h, th));
   // Errors of the launch surface through cudaGetLastError.
-  ForEpfKernel(fma, th, rows, work.list != nullptr, [&](auto kernel) {
+  ForEpfKernel(fma, rows, work.list != nullptr, [&](auto kernel) {
     LaunchPdl(pdl, kernel, grid, kEpfW * th / rows, EpfSmemBytes(th), st, in,
               guide_ovr, gab, w, h, mm, work, out, dco, map, tma, err, polls);
   });

@@ -2237,6 +2237,7 @@ __global__ void __launch_bounds__(3 * kSmallArBlocks)
 
 }  // namespace pikgpu
 
+#include "packed_fp32.cuh"
 #include "square_kernels.cuh"
 #include "tc_kernels.cuh"
 #include "stencil_kernels.cuh"
