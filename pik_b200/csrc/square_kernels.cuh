@@ -11,51 +11,41 @@
 namespace pikgpu {
 namespace square {
 
-// tsIDCT pass 1 on coefficient row c (row = horizontal frequency k):
-// t[v] = sum_l c[l] A[v][l].
+// A row times the transform matrix `m` (in constant memory): o[k] =
+// sum_i M[k][i] v[i], two outputs' sums in one instruction: three issue slots
+// for two rounded products and sums instead of four, and the FP32 pipe is the
+// bound. 16x16 blocks of a 4K frame: inverse 141 -> 128 us, clamp 66 -> 57.
 template <int N>
-__device__ __forceinline__ void IdctRow(const float (&c)[N], float (&t)[N]) {
+__device__ __forceinline__ void MatRow(const float* m, const float (&v)[N],
+                                       float (&o)[N]) {
 #pragma unroll
-  for (int v = 0; v < N; ++v) {
-    float s = 0.f;
+  for (int k = 0; k < N; k += 2) {
+    float s0 = 0.f, s1 = 0.f;
 #pragma unroll
-    for (int l = 0; l < N; ++l) s += c[l] * c_t.idct[MatOffset(N) + v * N + l];
-    t[v] = s;
+    for (int i = 0; i < N; ++i) {
+      Add2(s0, s1, v[i] * m[k * N + i], v[i] * m[(k + 1) * N + i]);
+    }
+    o[k] = s0;
+    o[k + 1] = s1;
   }
 }
-// tsIDCT pass 2 on column u[k] = tmp[k][v]: out[x] = sum_k A[x][k] u[k].
+// tsIDCT pass: t[v] = sum_l c[l] A[v][l], on coefficient row c (row =
+// horizontal frequency k), then on the columns of its output.
 template <int N>
-__device__ __forceinline__ void IdctCol(const float (&u)[N], float (&o)[N]) {
-#pragma unroll
-  for (int x = 0; x < N; ++x) {
-    float s = 0.f;
-#pragma unroll
-    for (int k = 0; k < N; ++k) s += c_t.idct[MatOffset(N) + x * N + k] * u[k];
-    o[x] = s;
-  }
+__device__ __forceinline__ void IdctRow(const float (&c)[N], float (&t)[N]) {
+  MatRow<N>(c_t.idct + MatOffset(N), c, t);
 }
 // tsDCT pass 1 on pixel row p (row y): t[k] = sum_x B[k][x] p[x].
 template <int N>
 __device__ __forceinline__ void DctRow(const float (&p)[N], float (&t)[N]) {
-#pragma unroll
-  for (int k = 0; k < N; ++k) {
-    float s = 0.f;
-#pragma unroll
-    for (int x = 0; x < N; ++x) s += c_t.dct[MatOffset(N) + k * N + x] * p[x];
-    t[k] = s;
-  }
+  MatRow<N>(c_t.dct + MatOffset(N), p, t);
 }
 // tsDCT pass 2 on q[y] = tmp[k][y]: o[l] = (sum_y q[y] B[l][y]) / N^2.
 template <int N>
 __device__ __forceinline__ void DctCol(const float (&q)[N], float (&o)[N]) {
-  const float scale = 1.0f / float(N * N);
+  DctRow<N>(q, o);
 #pragma unroll
-  for (int l = 0; l < N; ++l) {
-    float s = 0.f;
-#pragma unroll
-    for (int y = 0; y < N; ++y) s += q[y] * c_t.dct[MatOffset(N) + l * N + y];
-    o[l] = s * scale;
-  }
+  for (int l = 0; l < N; ++l) o[l] *= 1.0f / float(N * N);
 }
 
 // Writes `v` as row r of the unit's tile (stride N + 1) ...
@@ -148,7 +138,7 @@ __global__ void __launch_bounds__(kSquareThreads)
   PutRow<N>(tile, r, T);  // tmp[k = r][v]
   __syncwarp();
   GetCol<N>(tile, r, X);  // column v = r
-  IdctCol<N>(X, T);       // pixel row v = r
+  IdctRow<N>(X, T);       // pixel row v = r
   if (active) {
     float* out = f.idct + c * size_t(g.PW) * g.PH +
                  size_t(by * 8 + r) * g.PW + bx * 8;
@@ -363,7 +353,7 @@ __global__ void __launch_bounds__(kSquareArThreads)
   PutRow<N>(tile, r, D);
   __syncwarp();
   GetCol<N>(tile, r, Y);
-  IdctCol<N>(Y, D);
+  IdctRow<N>(Y, D);
   if (active) {
 #pragma unroll
     for (int x = 0; x < N; x += 4) {
@@ -389,9 +379,10 @@ __global__ void __launch_bounds__(kSquareArThreads)
 // 3001x2003 with 89% of the area in such blocks the inverse's 8192 rounded
 // operations per lane, block and channel take 0.11 ms at one per clock. A CTA
 // per block with both operands of every product in shared memory took 0.565
-// ms there (clamp 0.544); this split takes 0.241 (0.290), and 9 us instead of
-// 49 on a 256x256 frame of mixed blocks. One warp per item, or per two items,
-// without barriers: 0.248 and 0.223 ms there, but 18 and 31 us on small
+// ms there (clamp 0.544); this split takes 0.221 (0.265), with scalar instead
+// of packed products 0.244 (0.291), and 9 us instead of 49 on a 256x256 frame
+// of mixed blocks. One warp per item, or per two items, without barriers:
+// 0.248 and 0.223 ms there (scalar products), but 18 and 31 us on small
 // frames, and 72 instead of 46 us at 1000x1000, where its longer turns leave
 // the last wave empty.
 namespace square32 {
@@ -423,10 +414,11 @@ __device__ __forceinline__ void Pass(const float* m, int w,
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const float4 c = *reinterpret_cast<const float4*>(row + u * kN + i);
-        o[h + u] += v[i] * c.x;
-        o[h + u] += v[i + 1] * c.y;
-        o[h + u] += v[i + 2] * c.z;
-        o[h + u] += v[i + 3] * c.w;
+        float p[4];
+        Mul2(p[0], p[1], v[i], v[i + 1], c.x, c.y);
+        Mul2(p[2], p[3], v[i + 2], v[i + 3], c.z, c.w);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) o[h + u] += p[q];
       }
     }
   }
