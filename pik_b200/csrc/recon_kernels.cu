@@ -454,10 +454,18 @@ __global__ void k_encode_pnm(const float* lin, size_t stride, int w, int h,
 // of the int16 input and the matrix row, 128-bit stores); a CTA covers
 // 256 / (64 / kDequantCoefs) cells of one block row. The loads come first,
 // the int16 coefficients, then the chain quant field -> table -> matrix
-// row. Four coefficients per thread: 0.040 ms at 4K against 0.048 with
-// eight (twice the threads; the kernel is bound by latency, not traffic).
+// row, each link of it for all channels at once. Four coefficients per
+// thread: 0.040 ms at 4K against 0.048 with eight and 0.043 with two; a second
+// block row per thread: 0.039 against 0.035.
+//
+// Bound by issue slots next to the traffic (10 bytes per coefficient, 0.19 ms
+// at 8192x8192), most of them the biased value's division and branches: the
+// CTA tabulates it for magnitudes below kDequantTable (it is odd in q, and
+// nearly all coefficients are small), and a thread with a larger one takes its
+// coefficients again in full. 36 -> 31 us at 4K, 260 -> 221 at 8192x8192.
 constexpr int kDequantCoefs = 4;
 constexpr int kDequantCells = 256 / (64 / kDequantCoefs);
+constexpr int kDequantTable = 64;  // a power of two
 
 __device__ __forceinline__ float AdjustQuantBias(float q, float one_bias) {
   const float qa = fabsf(q);
@@ -466,62 +474,78 @@ __device__ __forceinline__ float AdjustQuantBias(float q, float one_bias) {
   return q;
 }
 
-__global__ void __launch_bounds__(256) k_dequant_ac(Geo g, DevFrame f,
-                                                    FrameScalars s) {
+__global__ void __launch_bounds__(256)
+    k_dequant_ac(Geo g, DevFrame f, FrameScalars s) {
   constexpr int K = kDequantCoefs, TPC = 64 / K;
-  static_assert(K == 4 || K == 8, "uint2 or uint4 loads of the int16 input");
+  static_assert(K == 4, "uint2 loads of the int16 input");
+  __shared__ float s_adj[3][kDequantTable];
   const int part = threadIdx.x % TPC;  // coefficients K part .. K part + K-1
-  const int bx = blockIdx.x * kDequantCells + threadIdx.x / TPC;
+  const int cell_x = blockIdx.x * kDequantCells + threadIdx.x / TPC;
+  const int bx = min(cell_x, g.Bx - 1);
   const int by = blockIdx.y;
-  if (bx >= g.Bx) return;
   const size_t plane = size_t(g.ac_stride) * g.By;
   const size_t pos = size_t(by) * g.ac_stride + size_t(bx) * 64 + K * part;
-  uint32_t raw[3][K / 2];
+  uint2 raw[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const int16_t* src = f.qac + c * plane + pos;
-    if constexpr (K == 8) {
-      const uint4 v = *reinterpret_cast<const uint4*>(src);
-      raw[c][0] = v.x, raw[c][1] = v.y, raw[c][2] = v.z, raw[c][3] = v.w;
-    } else {
-      const uint2 v = *reinterpret_cast<const uint2*>(src);
-      raw[c][0] = v.x, raw[c][1] = v.y;
-    }
+    raw[c] = *reinterpret_cast<const uint2*>(f.qac + c * plane + pos);
   }
   const int cell = by * g.Bx + bx;
+  const int color = (by >> 3) * g.Tx + (bx >> 3);
   const int qf = f.qf[cell];
-  const float scaled = qf == 0 ? 1E10f : s.inv_global_scale / float(qf);
-  const int tx = bx >> 3, ty = by >> 3;
-  const int cf = f.dq_cf[ty * g.Tx + tx];
-  const int table = f.dq_map[cf * 256 + (qf - 1)];
   const int a = f.acs[cell];
+  const int cf = f.dq_cf[color];
+  const int ytox = f.ytox[color], ytob = f.ytob[color];
+  if (threadIdx.x < 3 * kDequantTable) {
+    const int c = threadIdx.x / kDequantTable, q = threadIdx.x % kDequantTable;
+    s_adj[c][q] = AdjustQuantBias(float(q), c_t.one_bias[c]);
+  }
+  const int table = f.dq_map[cf * 256 + (qf - 1)];
   const int kind = QuantKindOf(a >> 4);
   const int blk = a & 0xF;
-  const float x_cc = 1.0f * float(f.ytox[ty * g.Tx + tx] - 128) * (1.0f / 256);
-  const float b_cc = 1.0f * float(f.ytob[ty * g.Tx + tx]) * (1.0f / 128);
-  float dq[3][K];
+  uint32_t mat[3];  // the matrix rows in the table
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const float* m = f.table + f.offsets[(table * 7 + kind) * 3 + c] +
-                     blk * 64 + K * part;
+    mat[c] = f.offsets[(table * 7 + kind) * 3 + c] + blk * 64 + K * part;
+  }
+  __syncthreads();
+  if (cell_x >= g.Bx) return;
+  const float scaled = qf == 0 ? 1E10f : s.inv_global_scale / float(qf);
+  const float x_cc = 1.0f * float(ytox - 128) * (1.0f / 256);
+  const float b_cc = 1.0f * float(ytob) * (1.0f / 128);
+  float dq[3][K];
+  int large = 0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const float* m = f.table + mat[c];
     float mv[K];
     if ((reinterpret_cast<uintptr_t>(m) & 15) == 0) {
-#pragma unroll
-      for (int i = 0; i < K / 4; ++i) {
-        const float4 v = reinterpret_cast<const float4*>(m)[i];
-        mv[4 * i] = v.x, mv[4 * i + 1] = v.y, mv[4 * i + 2] = v.z,
-               mv[4 * i + 3] = v.w;
-      }
+      const float4 v = *reinterpret_cast<const float4*>(m);
+      mv[0] = v.x, mv[1] = v.y, mv[2] = v.z, mv[3] = v.w;
     } else {
 #pragma unroll
       for (int k = 0; k < K; ++k) mv[k] = m[k];
     }
-    const float ob = c_t.one_bias[c];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-      const int16_t qi = int16_t(raw[c][k >> 1] >> (16 * (k & 1)));
+      const uint32_t w = k < 2 ? raw[c].x : raw[c].y;
+      const int q = int16_t(w >> (16 * (k & 1))), qa = abs(q);
+      large |= qa;
+      const float adj = s_adj[c][min(qa, kDequantTable - 1)];
       const float mulc = mv[k] * scaled;
-      dq[c][k] = AdjustQuantBias(float(qi), ob) * mulc;
+      dq[c][k] = __int_as_float(__float_as_int(adj) | (q & int(1u << 31))) *
+                 mulc;
+    }
+  }
+  if (large >= kDequantTable) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const float mulc = f.table[mat[c] + k] * scaled;
+        const float q = float(f.qac[c * plane + pos + k]);
+        dq[c][k] = AdjustQuantBias(q, c_t.one_bias[c]) * mulc;
+      }
     }
   }
   float o0[K], o2[K];
@@ -530,18 +554,12 @@ __global__ void __launch_bounds__(256) k_dequant_ac(Geo g, DevFrame f,
     o0[k] = x_cc * dq[1][k] + dq[0][k];
     o2[k] = b_cc * dq[1][k] + dq[2][k];
   }
-  float4* d0 = reinterpret_cast<float4*>(f.ac + pos);
-  float4* d1 = reinterpret_cast<float4*>(f.ac + plane + pos);
-  float4* d2 = reinterpret_cast<float4*>(f.ac + 2 * plane + pos);
-#pragma unroll
-  for (int i = 0; i < K / 4; ++i) {
-    d1[i] = make_float4(dq[1][4 * i], dq[1][4 * i + 1], dq[1][4 * i + 2],
-                        dq[1][4 * i + 3]);
-    d0[i] = make_float4(o0[4 * i], o0[4 * i + 1], o0[4 * i + 2],
-                        o0[4 * i + 3]);
-    d2[i] = make_float4(o2[4 * i], o2[4 * i + 1], o2[4 * i + 2],
-                        o2[4 * i + 3]);
-  }
+  float* out = f.ac + pos;
+  *reinterpret_cast<float4*>(out) = make_float4(o0[0], o0[1], o0[2], o0[3]);
+  *reinterpret_cast<float4*>(out + plane) =
+      make_float4(dq[1][0], dq[1][1], dq[1][2], dq[1][3]);
+  *reinterpret_cast<float4*>(out + 2 * plane) =
+      make_float4(o2[0], o2[1], o2[2], o2[3]);
 }
 
 // ---------------------------------------------------------------------------
