@@ -74,6 +74,49 @@ struct DevBuf {
 };
 
 std::mutex g_table_mutex;
+
+// The contexts' wait-timeout flags: words of one page of pinned host memory
+// that the kernels write and the host reads without a copy. Pinning the first
+// page of a process takes 2 to 5 ms, as much as the rest of a context, and so
+// does the next after the last was freed: the page is shared by the contexts
+// (portable: on every device) and kept for the process. A context beyond its
+// words pins its own.
+struct FlagPage {
+  static constexpr int kWords = 1024;
+  std::mutex mutex;
+  int* words = nullptr;
+  bool used[kWords] = {};
+
+  // A flag set to 0, or NULL if no memory can be pinned.
+  int* Take() {
+    std::lock_guard<std::mutex> lock(mutex);
+    if (!words && !Pin(kWords, &words)) return nullptr;
+    for (int i = 0; i < kWords; ++i) {
+      if (used[i]) continue;
+      used[i] = true;
+      words[i] = 0;
+      return words + i;
+    }
+    int* own = nullptr;
+    if (!Pin(1, &own)) return nullptr;
+    *own = 0;
+    return own;
+  }
+  void Give(int* flag) {
+    std::lock_guard<std::mutex> lock(mutex);
+    if (words && flag >= words && flag < words + kWords) {
+      used[flag - words] = false;
+    } else {
+      cudaFreeHost(flag);
+    }
+  }
+  static bool Pin(int n, int** out) {
+    return cudaHostAlloc(out, n * sizeof(int),
+                         cudaHostAllocMapped | cudaHostAllocPortable) ==
+           cudaSuccess;
+  }
+};
+FlagPage g_flags;
 bool g_tables_uploaded[64] = {};
 
 // Persistent tensor-core transform CTAs per SM (default): 4 x 128
@@ -1096,10 +1139,8 @@ int pikgpu_ctx_create(int device, pikgpu_ctx** out) {
   }
   cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount,
                          device);
-  if (cudaHostAlloc(&ctx->tc_err, sizeof(int), cudaHostAllocMapped) ==
-      cudaSuccess) {
-    *ctx->tc_err = 0;
-  } else {
+  ctx->tc_err = g_flags.Take();
+  if (!ctx->tc_err) {
     pikgpu_ctx_destroy(ctx);
     return PIKGPU_ERR_NO_MEMORY;
   }
@@ -1137,7 +1178,7 @@ int pikgpu_ctx_destroy(pikgpu_ctx* ctx) {
   for (auto& b : ctx->active) FreeBuf(&b);
   FreeBuf(&ctx->counters);
   DropFrameGraph(ctx);
-  if (ctx->tc_err) cudaFreeHost(ctx->tc_err);
+  if (ctx->tc_err) g_flags.Give(ctx->tc_err);
   for (auto& e : ctx->ev) {
     if (e) cudaEventDestroy(e);
   }
