@@ -54,8 +54,8 @@ PATH_BYTES_PER_PX = 18.28
 # profiles/k_epf_box_c2_4k.md) and the DRAM bytes (dram__bytes_read.sum +
 # dram__bytes_write.sum) of all the frame's 17 launches, run one after
 # another with the caches kept between them (profiles/traffic_c2_4k.md).
-EPF_WARP_INSTR_4K = 175.5e6
-PATH_TRAFFIC_4K = 835.2e6
+EPF_WARP_INSTR_4K = 132.6e6
+PATH_TRAFFIC_4K = 730.2e6
 # Algorithmic bytes per pixel of each kernel group (PIKGPU_OPT_PROFILE
 # groups), with 4-byte floats.
 GROUP_BYTES = {
@@ -963,7 +963,7 @@ def main():
     # DRAM bytes per launch of the 4K workload measured with ncu
     # (dram__bytes_read.sum + dram__bytes_write.sum, one cold launch each).
     ncu_traffic_4k = {
-        "epf": 100.38e6 + 63.28e6,
+        "epf": 58.53e6 + 15.34e6,
         "gaborish1_minmax": 99.54e6 + 64.64e6,
         "gaborish2_opsin_srgb": 99.55e6 + 63.85e6,
     }
