@@ -484,8 +484,13 @@ int UploadTables(pikgpu_ctx* ctx) {
     CUDA_TRY(ctx, e);
   }
   CUDA_TRY(ctx, cudaFuncSetAttribute(
-                    k_lf_tile, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                    int(kLfSmemBytes)));
+                    k_lf_tile<LfTile16>,
+                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                    int(LfTile16::kSmemBytes)));
+  CUDA_TRY(ctx, cudaFuncSetAttribute(
+                    k_lf_tile<LfTile32>,
+                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                    int(LfTile32::kSmemBytes)));
   CUDA_TRY(ctx, cudaFuncSetAttribute(
                     k_square_ar_tc<16, 2>,
                     cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -802,11 +807,21 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
   Mark(ctx, kTLf);
   // Per-group LF prediction and the LF update of every block's dequantised
   // coefficients, with its pred2x2 (after DC and the dequantisation): one
-  // CTA per tile of 32 x 32 cells of a group and channel.
+  // CTA per tile of a group and channel.
   const int ng = g.Gx * g.Gy;
-  constexpr int kTilesPerGroup = (64 + kLfTile - 1) / kLfTile;
-  k_lf_tile<<<dim3(kTilesPerGroup * kTilesPerGroup, ng, 3), kLfThreads,
-              kLfSmemBytes, st>>>(g, f, s.predict_lf, s.predict_hf);
+  auto lf_tiles = [&](auto win) {
+    using W = decltype(win);
+    const int tiles = W::kTilesPerGroup * W::kTilesPerGroup;
+    k_lf_tile<W><<<dim3(tiles, ng, 3), W::kThreads, W::kSmemBytes, st>>>(
+        g, f, s.predict_lf, s.predict_hf);
+  };
+  // The larger tiles where they fill four waves of two CTAs per SM.
+  constexpr int kTiles32 = LfTile32::kTilesPerGroup * LfTile32::kTilesPerGroup;
+  if (3 * kTiles32 * ng >= 4 * 2 * ctx->num_sms) {
+    lf_tiles(LfTile32());
+  } else {
+    lf_tiles(LfTile16());
+  }
   ++ctx->launches;
   Mark(ctx, kTIdct);
   br.Fork(1, 1);

@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(256)
 // pik/compressed_dc.cc:530-556). The 2x2 image of the group is
 // 2 (gxs + 2) x 2 (gys + 2), mirrored at its edges by the blur.
 //
-// A CTA (k_lf_tile) takes one channel of a tile of kLfTile x kLfTile cells
+// A CTA (k_lf_tile) takes one channel of a tile of 16 x 16 or 32 x 32 cells
 // of a group and keeps the images it needs in shared memory: the DC, LLF and
 // 2x2 images of every block that reaches the tile's blurred range (one
 // cell beyond the tile, and the ring where the tile touches it), so its
@@ -585,40 +585,50 @@ struct LfGroup {
   }
 };
 
-constexpr int kLfTile = 16;           // cells per tile side
-constexpr int kLfWin = kLfTile + 12;  // shared-memory window, cells
-constexpr int kLfWin2 = 2 * kLfWin;   // the 2x2 images' window, pixels
-constexpr int kLfThreads = 256;
-// Shared memory of k_lf_tile: the DC and LLF images, the 2x2 image before
-// and after LFPredictionBlur, over the window, and the list of the window's
-// first cells (by block size: 8x8-class blocks, then 16x16, then 32x32).
-constexpr int kLfList1 = kLfWin * kLfWin;
-constexpr int kLfList2 = (kLfWin / 2 + 1) * (kLfWin / 2 + 1);
-constexpr int kLfList4 = (kLfWin / 4 + 1) * (kLfWin / 4 + 1);
-constexpr size_t kLfSmemBytes =
-    4 * (2 * size_t(kLfWin) * kLfWin + 2 * size_t(kLfWin2) * kLfWin2 +
-         kLfList1 + kLfList2 + kLfList4);
-
-// The window of a tile: cell (X, Y) of the group is at (X - ex, Y - ey).
+// The window of a tile of TILE x TILE cells: cell (X, Y) of the group is at
+// (X - ex, Y - ey).
+template <int TILE, int THREADS>
 struct LfWin {
+  static constexpr int kTile = TILE;          // cells per tile side
+  static constexpr int kThreads = THREADS;    // of the tile's CTA
+  static constexpr int kWin = TILE + 12;      // shared-memory window, cells
+  static constexpr int kWin2 = 2 * kWin;      // the 2x2 images' window, pixels
+  static constexpr int kTilesPerGroup = (64 + TILE - 1) / TILE;  // per side
+  // Shared memory of k_lf_tile: the DC and LLF images, the 2x2 image before
+  // and after LFPredictionBlur, over the window, and the list of the window's
+  // first cells (by block size: 8x8-class blocks, then 16x16, then 32x32).
+  static constexpr int kList1 = kWin * kWin;
+  static constexpr int kList2 = (kWin / 2 + 1) * (kWin / 2 + 1);
+  static constexpr int kList4 = (kWin / 4 + 1) * (kWin / 4 + 1);
+  static constexpr size_t kSmemBytes =
+      4 * (2 * size_t(kWin) * kWin + 2 * size_t(kWin2) * kWin2 + kList1 +
+           kList2 + kList4);
+
   int ex, ey;
-  float* dc;   // kLfWin x kLfWin
-  float* llf;  // kLfWin x kLfWin
-  float* tmp;  // kLfWin2 x kLfWin2
-  float* lf;   // kLfWin2 x kLfWin2
+  float* dc;   // kWin x kWin
+  float* llf;  // kWin x kWin
+  float* tmp;  // kWin2 x kWin2
+  float* lf;   // kWin2 x kWin2
   __device__ float* Dc(int X, int Y) const {
-    return dc + (Y - ey) * kLfWin + (X - ex);
+    return dc + (Y - ey) * kWin + (X - ex);
   }
   __device__ float* Llf(int X, int Y) const {
-    return llf + (Y - ey) * kLfWin + (X - ex);
+    return llf + (Y - ey) * kWin + (X - ex);
   }
   __device__ float* Tmp(int X2, int Y2) const {
-    return tmp + (Y2 - 2 * ey) * kLfWin2 + (X2 - 2 * ex);
+    return tmp + (Y2 - 2 * ey) * kWin2 + (X2 - 2 * ex);
   }
   __device__ float* Lf(int X2, int Y2) const {
-    return lf + (Y2 - 2 * ey) * kLfWin2 + (X2 - 2 * ex);
+    return lf + (Y2 - 2 * ey) * kWin2 + (X2 - 2 * ex);
   }
 };
+// Tiles of 16 cells, or of 32 in large frames: the larger tile loads
+// 1.9 cells per cell of its own instead of 3.1 and forms 1.3 instead of 1.7
+// times the blocks, but leaves 4K frames one and a half waves of CTAs and
+// small frames a few CTAs: 272 instead of 334 us at 8192x8192, 42.5 instead of
+// 41.3 at 3840x2160, 18 instead of 11 at 256x256.
+using LfTile16 = LfWin<16, 256>;
+using LfTile32 = LfWin<32, 512>;
 
 // The per-block LF steps, on a unit of kLanes lanes per block: one lane for
 // the 8x8 classes, a lane per row of the 2 COV x 2 COV low frequencies for
@@ -655,7 +665,8 @@ struct LfUnit {
 
   // ComputeLlf (LowestFrequenciesFromDC) and, with `up`, the block's 2x2
   // cells from the LLF (DC2x2FromLowestFrequencies).
-  static __device__ __forceinline__ void Llf(const LfWin& w, bool on, int r,
+  template <typename W>
+  static __device__ __forceinline__ void Llf(const W& w, bool on, int r,
                                              int type, int X, int Y, bool up) {
     const float* dc = w.Dc(X, Y);
     if constexpr (COV == 1) {
@@ -671,11 +682,11 @@ struct LfUnit {
         const float t0 = 0.f + v * a[0], t1 = 0.f + v * a[2];
         *reinterpret_cast<float2*>(d) =
             make_float2(0.f + a[0] * t0, 0.f + a[2] * t0);
-        *reinterpret_cast<float2*>(d + kLfWin2) =
+        *reinterpret_cast<float2*>(d + W::kWin2) =
             make_float2(0.f + a[0] * t1, 0.f + a[2] * t1);
       } else {
         *reinterpret_cast<float2*>(d) = make_float2(v, v);
-        *reinterpret_cast<float2*>(d + kLfWin2) = make_float2(v, v);
+        *reinterpret_cast<float2*>(d + W::kWin2) = make_float2(v, v);
       }
     } else {
       // ReinterpDct<D, COV> of the block's DC: the lane takes coefficient
@@ -692,7 +703,7 @@ struct LfUnit {
       for (int y = 0; y < COV; ++y) {
         float sum = 0.f;
 #pragma unroll
-        for (int x = 0; x < COV; ++x) sum += b[x] * dc[y * kLfWin + x];
+        for (int x = 0; x < COV; ++x) sum += b[x] * dc[y * W::kWin + x];
         q[y] = sum;
       }
       constexpr float scale = 1.0f / float(COV * COV);
@@ -724,7 +735,7 @@ struct LfUnit {
         float sum = 0.f;
 #pragma unroll
         for (int l = 0; l < COV; ++l) {
-          const float v = in[kk * kLfWin + l] *
+          const float v = in[kk * W::kWin + l] *
                           c_t.inv_total_scale[sn][kk][l] *
                           c_t.total_scale[sd][kk][l];
           sum += v * a[l];
@@ -751,14 +762,15 @@ struct LfUnit {
 
   // LowFrequenciesFromDC2x2 of the block's cells of the blurred 2x2 image,
   // in place.
-  static __device__ __forceinline__ void Forward(const LfWin& w, bool on,
+  template <typename W>
+  static __device__ __forceinline__ void Forward(const W& w, bool on,
                                                  int r, int type, int X,
                                                  int Y) {
     float* base = w.Lf(2 * X, 2 * Y);
     if constexpr (COV == 1) {
       if (!on) return;
       const float2 p0 = *reinterpret_cast<const float2*>(base);
-      const float2 p1 = *reinterpret_cast<const float2*>(base + kLfWin2);
+      const float2 p1 = *reinterpret_cast<const float2*>(base + W::kWin2);
       const float in[4] = {p0.x, p0.y, p1.x, p1.y};
       float o[4];
       if (DctLike(type)) {
@@ -770,7 +782,7 @@ struct LfUnit {
         o[3] = (in[0] - in[1] - in[2] + in[3]) * 0.25f;
       }
       *reinterpret_cast<float2*>(base) = make_float2(o[0], o[1]);
-      *reinterpret_cast<float2*>(base + kLfWin2) = make_float2(o[2], o[3]);
+      *reinterpret_cast<float2*>(base + W::kWin2) = make_float2(o[2], o[3]);
     } else {
       float q[N];
       if constexpr (COV == 2) {
@@ -784,13 +796,13 @@ struct LfUnit {
         for (int y = 0; y < N; ++y) {
           float sum = 0.f;
 #pragma unroll
-          for (int x = 0; x < N; ++x) sum += b[x] * base[y * kLfWin2 + x];
+          for (int x = 0; x < N; ++x) sum += b[x] * base[y * W::kWin2 + x];
           q[y] = sum;
         }
       } else {
         // First pass on the lane's row, transposed through the window.
         float p[N], t[N];
-        LoadRow(base + r * kLfWin2, p);
+        LoadRow(base + r * W::kWin2, p);
 #pragma unroll
         for (int k = 0; k < N; ++k) {
           float sum = 0.f;
@@ -803,10 +815,10 @@ struct LfUnit {
         __syncwarp();
         if (on) {
 #pragma unroll
-          for (int k = 0; k < N; ++k) base[k * kLfWin2 + r] = t[k];
+          for (int k = 0; k < N; ++k) base[k * W::kWin2 + r] = t[k];
         }
         __syncwarp();
-        LoadRow(base + r * kLfWin2, q);
+        LoadRow(base + r * W::kWin2, q);
       }
       float ts[N], its[N], o[N];
       ScaleRow<N>(g_t.total_scale[sn], r, ts);
@@ -822,7 +834,7 @@ struct LfUnit {
         o[l] = sum * scale * ts[l] * its[l];
       }
       __syncwarp();
-      if (on) StoreRow(base + r * kLfWin2, o);
+      if (on) StoreRow(base + r * W::kWin2, o);
       __syncwarp();
     }
   }
@@ -831,8 +843,9 @@ struct LfUnit {
   // the block's corner, the LF prediction added to the LF coefficients, and
   // the block's pred2x2 cells from the updated corner. The corner's rows are
   // contiguous in the frame layout's first cell row.
+  template <typename W>
   static __device__ __forceinline__ void Update(
-      const Geo& g, const DevFrame& f, const LfGroup& q, const LfWin& w,
+      const Geo& g, const DevFrame& f, const LfGroup& q, const W& w,
       bool on, int r, int type, int X, int Y, int predict_lf,
       int predict_hf) {
     float* base = f.ac + size_t(q.c) * g.ac_stride * g.By +
@@ -848,7 +861,7 @@ struct LfUnit {
       b[0] = *w.Llf(X, Y), b[1] = a0.y, b[2] = a1.x, b[3] = a1.y;
       if (predict_lf) {
         const float* l = w.Lf(2 * X, 2 * Y);
-        b[1] += l[1], b[2] += l[kLfWin2], b[3] += l[kLfWin2 + 1];
+        b[1] += l[1], b[2] += l[W::kWin2], b[3] += l[W::kWin2 + 1];
       }
       *reinterpret_cast<float2*>(base) = make_float2(b[0], b[1]);
       *reinterpret_cast<float2*>(base + 8) = make_float2(b[2], b[3]);
@@ -913,7 +926,7 @@ struct LfUnit {
       __syncwarp();
       const float* col = w.Lf(2 * X + r, 2 * Y);
 #pragma unroll
-      for (int k = 0; k < N; ++k) t[k] = col[k * kLfWin2];
+      for (int k = 0; k < N; ++k) t[k] = col[k * W::kWin2];
 #pragma unroll
       for (int u = 0; u < N; ++u) {
         float sum = 0.f;
@@ -949,7 +962,8 @@ struct LfUnit {
 // mirrored at the image's edges) for the run of up to 8 pixels x0 ..
 // x0 + n - 1 of row y: the 3 x (n + 2) inputs are loaded once, and each
 // output keeps Symmetric3's operation order.
-__device__ void LfBlurRun(const LfGroup& q, const LfWin& w, int x0, int y,
+template <typename W>
+__device__ void LfBlurRun(const LfGroup& q, const W& w, int x0, int y,
                           int n) {
   const int w2 = 2 * (q.gxs + 2), h2 = 2 * (q.gys + 2);
   const int yr[3] = {MirrorIdx(y - 1, h2), y, MirrorIdx(y + 1, h2)};
@@ -980,8 +994,9 @@ __device__ void LfBlurRun(const LfGroup& q, const LfWin& w, int x0, int y,
 }
 
 // Ring cell (x, y) of pred2x2 (pik/compressed_image.cc:978-1039).
+template <typename W>
 __device__ void PredBorderCell(const DevFrame& f, const LfGroup& q,
-                               const LfWin& w, int x, int y,
+                               const W& w, int x, int y,
                                int predict_lf) {
   float* pred = f.pred2x2_g + q.gi * kG2GroupFloats + q.c * kG2 * kG2;
   float* d = pred + 2 * y * kG2 + 2 * x;
@@ -998,11 +1013,11 @@ __device__ void PredBorderCell(const DevFrame& f, const LfGroup& q,
 // blocks first, whose steps are the longest), warp by warp: a warp step
 // takes 32 / LfUnit<cov>::kLanes blocks of one size. Entries past own[k]
 // stand at the list's back.
-template <typename Fn>
+template <typename W, typename Fn>
 __device__ __forceinline__ void ForLfUnits(int* const* lists, const int* own,
                                            const int* n, Fn&& fn) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr int kWarps = kLfThreads / 32;
+  constexpr int kWarps = W::kThreads / 32;
   const int w4 = (n[2] + 3) / 4, w2 = w4 + (n[1] + 7) / 8,
             w1 = w2 + (n[0] + 31) / 32;
   auto entry = [&](int k, int cap, bool on, int u) {
@@ -1014,16 +1029,16 @@ __device__ __forceinline__ void ForLfUnits(int* const* lists, const int* own,
       const int u = 4 * i + lane / 8;
       const bool on = u < n[2];
       fn(std::integral_constant<int, 4>(), on, lane % 8,
-         entry(2, kLfList4, on, u));
+         entry(2, W::kList4, on, u));
     } else if (i < w2) {
       const int u = 8 * (i - w4) + lane / 4;
       const bool on = u < n[1];
       fn(std::integral_constant<int, 2>(), on, lane % 4,
-         entry(1, kLfList2, on, u));
+         entry(1, W::kList2, on, u));
     } else {
       const int u = 32 * (i - w2) + lane;
       const bool on = u < n[0];
-      fn(std::integral_constant<int, 1>(), on, 0, entry(0, kLfList1, on, u));
+      fn(std::integral_constant<int, 1>(), on, 0, entry(0, W::kList1, on, u));
     }
   }
 }
@@ -1034,31 +1049,32 @@ __device__ __forceinline__ void ForLfUnits(int* const* lists, const int* own,
 // cell is in [lo - 4, hi + 1) (the blur reads cells lo - 1 .. hi), then the
 // blur and LowFrequenciesFromDC2x2 over [lo, hi) -- the tile plus the ring
 // cells beside it -- then the ring's pred2x2 and the update of the tile's
-// blocks. Bound by the latency of the phases' chains: four CTAs per SM (64
-// registers, some spills) took 334 us at 8192x8192, three (80 registers) 340
-// and two 382.
-__global__ void __launch_bounds__(kLfThreads, 4)
+// blocks. Bound by the latency of the phases' chains: with tiles of 16 cells
+// four CTAs per SM (64 registers, some spills) took 334 us at 8192x8192, three
+// (80 registers) 340 and two 382; tiles of 32 cells take 272.
+template <typename W>
+__global__ void __launch_bounds__(W::kThreads, 1024 / W::kThreads)
     k_lf_tile(Geo g, DevFrame f, int predict_lf, int predict_hf) {
   extern __shared__ __align__(16) float lf_smem[];
   LfGroup q;
   q.gi = blockIdx.y;
   q.c = blockIdx.z;
   GroupDims(g, q.gi, &q.x0, &q.y0, &q.gxs, &q.gys);
-  const int ntx = (q.gxs + kLfTile - 1) / kLfTile;
+  const int ntx = (q.gxs + W::kTile - 1) / W::kTile;
   const int tx = blockIdx.x % ntx, ty = blockIdx.x / ntx;
-  if (ty * kLfTile >= q.gys) return;
+  if (ty * W::kTile >= q.gys) return;
   // The tile's cells [X0, X1) x [Y0, Y1); the LF range adds the ring.
-  const int X0 = 1 + tx * kLfTile, X1 = min(X0 + kLfTile, q.gxs + 1);
-  const int Y0 = 1 + ty * kLfTile, Y1 = min(Y0 + kLfTile, q.gys + 1);
+  const int X0 = 1 + tx * W::kTile, X1 = min(X0 + W::kTile, q.gxs + 1);
+  const int Y0 = 1 + ty * W::kTile, Y1 = min(Y0 + W::kTile, q.gys + 1);
   const int lx = X0 == 1 ? 0 : X0, hx = X1 == q.gxs + 1 ? q.gxs + 2 : X1;
   const int ly = Y0 == 1 ? 0 : Y0, hy = Y1 == q.gys + 1 ? q.gys + 2 : Y1;
-  LfWin w;
+  W w;
   w.ex = lx - 4;
   w.ey = ly - 4;
   w.tmp = lf_smem;
-  w.lf = w.tmp + kLfWin2 * kLfWin2;
-  w.llf = w.lf + kLfWin2 * kLfWin2;
-  w.dc = w.llf + kLfWin * kLfWin;
+  w.lf = w.tmp + W::kWin2 * W::kWin2;
+  w.llf = w.lf + W::kWin2 * W::kWin2;
+  w.dc = w.llf + W::kWin * W::kWin;
   // The first cells of the blocks reaching cells lx - 1 .. hx (clipped to
   // the group's ring), listed as X | Y << 10 | strategy byte << 20, one list
   // per block size, so that the per-block phases give every lane work of
@@ -1066,14 +1082,14 @@ __global__ void __launch_bounds__(kLfThreads, 4)
   // update) from its front and the others from its back.
   __shared__ int s_own[3], s_far[3];
   int* const lists[3] = {
-      reinterpret_cast<int*>(w.dc + kLfWin * kLfWin),
-      reinterpret_cast<int*>(w.dc + kLfWin * kLfWin) + kLfList1,
-      reinterpret_cast<int*>(w.dc + kLfWin * kLfWin) + kLfList1 + kLfList2};
+      reinterpret_cast<int*>(w.dc + W::kWin * W::kWin),
+      reinterpret_cast<int*>(w.dc + W::kWin * W::kWin) + W::kList1,
+      reinterpret_cast<int*>(w.dc + W::kWin * W::kWin) + W::kList1 + W::kList2};
   if (threadIdx.x < 3) s_own[threadIdx.x] = s_far[threadIdx.x] = 0;
   __syncthreads();
   const float* dc = f.dc + size_t(q.c) * g.By * g.Bx;
-  for (int i = threadIdx.x; i < kLfWin * kLfWin; i += kLfThreads) {
-    const int X = w.ex + i % kLfWin, Y = w.ey + i / kLfWin;
+  for (int i = threadIdx.x; i < W::kWin * W::kWin; i += W::kThreads) {
+    const int X = w.ex + i % W::kWin, Y = w.ey + i / W::kWin;
     if (X < 0 || Y < 0 || X > q.gxs + 1 || Y > q.gys + 1) continue;
     w.dc[i] = dc[size_t(MirrorIdx(q.y0 + Y - 1, g.By)) * g.Bx +
                  MirrorIdx(q.x0 + X - 1, g.Bx)];
@@ -1082,7 +1098,7 @@ __global__ void __launch_bounds__(kLfThreads, 4)
     if (a & 0xF) continue;
     const int cov = Covered(a >> 4), k = cov == 1 ? 0 : cov == 2 ? 1 : 2;
     const int e = X | (Y << 10) | (a << 20);
-    const int cap = k == 0 ? kLfList1 : k == 1 ? kLfList2 : kLfList4;
+    const int cap = k == 0 ? W::kList1 : k == 1 ? W::kList2 : W::kList4;
     if (X >= X0 && X < X1 && Y >= Y0 && Y < Y1) {
       lists[k][atomicAdd(&s_own[k], 1)] = e;
       // The update's lines of the dequantised AC, two phases ahead.
@@ -1100,7 +1116,7 @@ __global__ void __launch_bounds__(kLfThreads, 4)
   int own[3], all[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) own[k] = s_own[k], all[k] = own[k] + s_far[k];
-  ForLfUnits(lists, own, all, [&](auto cov, bool on, int r, int e) {
+  ForLfUnits<W>(lists, own, all, [&](auto cov, bool on, int r, int e) {
     LfUnit<cov.value>::Llf(w, on, r, e >> 24, e & 1023, (e >> 10) & 1023,
                            predict_lf);
   });
@@ -1109,12 +1125,12 @@ __global__ void __launch_bounds__(kLfThreads, 4)
     // Runs of 8 pixels of the blurred range's rows.
     const int w2 = 2 * (hx - lx), runs = (w2 + 7) / 8;
     const int n2 = runs * 2 * (hy - ly);
-    for (int i = threadIdx.x; i < n2; i += kLfThreads) {
+    for (int i = threadIdx.x; i < n2; i += W::kThreads) {
       const int r = i % runs, y = 2 * ly + i / runs;
       LfBlurRun(q, w, 2 * lx + 8 * r, y, min(8, w2 - 8 * r));
     }
     __syncthreads();
-    ForLfUnits(lists, own, all, [&](auto cov, bool on, int r, int e) {
+    ForLfUnits<W>(lists, own, all, [&](auto cov, bool on, int r, int e) {
       const int X = e & 1023, Y = (e >> 10) & 1023;
       on = on && X >= lx && X < hx && Y >= ly && Y < hy;
       LfUnit<cov.value>::Forward(w, on, r, e >> 24, X, Y);
@@ -1124,7 +1140,7 @@ __global__ void __launch_bounds__(kLfThreads, 4)
   if (predict_hf) {
     // Ring cells beside the tile: left/right columns, then top/bottom rows.
     const int rows = hy - ly, cols = hx - lx;
-    for (int i = threadIdx.x; i < 2 * rows + 2 * cols; i += kLfThreads) {
+    for (int i = threadIdx.x; i < 2 * rows + 2 * cols; i += W::kThreads) {
       int X, Y;
       if (i < 2 * rows) {
         X = (i & 1) ? q.gxs + 1 : 0;
@@ -1141,7 +1157,7 @@ __global__ void __launch_bounds__(kLfThreads, 4)
       PredBorderCell(f, q, w, X, Y, predict_lf);
     }
   }
-  ForLfUnits(lists, own, own, [&](auto cov, bool on, int r, int e) {
+  ForLfUnits<W>(lists, own, own, [&](auto cov, bool on, int r, int e) {
     LfUnit<cov.value>::Update(g, f, q, w, on, r, e >> 24, e & 1023,
                               (e >> 10) & 1023, predict_lf, predict_hf);
   });
