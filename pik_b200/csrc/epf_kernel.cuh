@@ -12,9 +12,9 @@
 // loads of 32 consecutive offsets hit 32 consecutive words, free of bank
 // conflicts), and the sum of absolute differences against the centre
 // pixel's patch row is one __vsadu4. For every displacement (cy, cx) of the
-// 7 x 8 neighbourhood and every channel, a lane forms ROWS + 2 patch-row SADs of its column and
-// sums them vertically into the 3 x 4 patch SADs of its rows; the SAD is
-// the maximum over the channels. The SADs are exact integers; the weights
+// 7 x 8 neighbourhood and every channel, a lane forms ROWS + 2 patch-row SADs
+// of its column and sums them vertically into the 3 x 4 patch SADs of its
+// rows; the SAD is the maximum over the channels. The SADs are exact integers; the weights
 // (WeightFast's bit construction) and the weighted sums follow the
 // reference's neighbour order (cy = -3..3, cx = -3..4) with separately
 // rounded products and sums, so the output equals the per-pixel formulation
@@ -586,7 +586,8 @@ __device__ __forceinline__ void EpfFilterTile(
 // bounded, so that no copy is in flight when the CTA exits. Border tiles,
 // and all tiles without a tensor map, are staged with cp.async (EpfStage).
 template <bool kFma, int TH, int ROWS, bool kList>
-__global__ void __launch_bounds__(EpfThreads<TH, ROWS>(), ROWS < 8 ? 2 : kFma ? 3 : 4)
+__global__ void __launch_bounds__(EpfThreads<TH, ROWS>(),
+                                  ROWS < 8 ? 2 : kFma ? 3 : 4)
     k_epf_box(const float* in, const uint8_t* guide_ovr, int gab, int w, int h,
               const uint32_t* mm, EpfWork work, float* out, EpfDc dco,
               const __grid_constant__ CUtensorMap tmap, int use_tma,
