@@ -1656,6 +1656,8 @@ int pikgpu_get_stage(pikgpu_ctx* ctx, int stage, float* const planes[3],
   if (!ctx) return PIKGPU_ERR_INVALID_ARG;
   PIKGPU_NOT_PENDING(ctx);
   if (!ctx->have_result) return Fail(ctx, PIKGPU_ERR_STATE, "no result");
+  // Two of the stages are completed by kernels on the context's stream.
+  CUDA_TRY(ctx, cudaSetDevice(ctx->device));
   const Geo& g = ctx->g;
   const float* src = nullptr;
   size_t w = 0, h = 0;
@@ -1680,13 +1682,6 @@ int pikgpu_get_stage(pikgpu_ctx* ctx, int stage, float* const planes[3],
       break;
     case PIKGPU_STAGE_AR:
       src = P<float>(ctx->filt), w = g.PW, h = g.PH;
-      if (ctx->s.have_ar) {
-        k_fill_regions<<<Blocks(3 * w * h, 4 * 256), 256, 0, ctx->stream>>>(
-            P<float>(ctx->idct), P<uint32_t>(ctx->region), g.PW, g.PH,
-            P<float>(ctx->filt));
-        CUDA_TRY(ctx, cudaGetLastError());
-        CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-      }
       break;
     case PIKGPU_STAGE_PRE_OPSIN:
       src = P<float>(ctx->dbg_pre), w = g.W, h = g.H;
@@ -1709,6 +1704,13 @@ int pikgpu_get_stage(pikgpu_ctx* ctx, int stage, float* const planes[3],
     return Fail(ctx, PIKGPU_ERR_INVALID_ARG,
                 "stage %d is %zux%zu (got %zux%zu, stride %zu)", stage, w, h,
                 xsize, ysize, stride);
+  }
+  if (stage == PIKGPU_STAGE_AR && ctx->s.have_ar) {
+    k_fill_regions<<<Blocks(3 * w * h, 4 * 256), 256, 0, ctx->stream>>>(
+        P<float>(ctx->idct), P<uint32_t>(ctx->region), g.PW, g.PH,
+        P<float>(ctx->filt));
+    CUDA_TRY(ctx, cudaGetLastError());
+    CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   }
   for (int c = 0; c < 3; ++c) {
     CUDA_TRY(ctx, cudaMemcpy2D(planes[c], 4 * stride, src + c * w * h, 4 * w,
@@ -1757,6 +1759,7 @@ int pikgpu_get_epf_decisions(pikgpu_ctx* ctx, uint8_t* guide,
   if (!ctx->have_result || !ctx->s.have_ar) {
     return Fail(ctx, PIKGPU_ERR_STATE, "no EPF result");
   }
+  CUDA_TRY(ctx, cudaSetDevice(ctx->device));
   const Geo& g = ctx->g;
   if (sigma) {
     CUDA_TRY(ctx, cudaMemcpy(sigma, ctx->sigma.p, 4 * size_t(g.Bx) * g.By,
