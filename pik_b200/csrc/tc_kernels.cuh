@@ -612,7 +612,9 @@ __global__ void __launch_bounds__(tc::kArThreads, tc::ArCtasPerSm<N>())
     ChannelSync(c);  // the operand may be written again
     batch = next;
   }
-  if (!ok && t == 0) tc::ReportTimeout(err, 1);
+  // After the last batch's inverse passes `ok` is each thread's own: any one
+  // whose wait ran out has left its stores out.
+  if (!ok) tc::ReportTimeout(err, 1);
   FenceBefore();
   __syncthreads();
   if (threadIdx.x < 32) {
