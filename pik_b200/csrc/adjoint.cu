@@ -48,24 +48,19 @@
 namespace pikgpu {
 namespace {
 
-constexpr int kJTypes = 5;  // DCT8, IDENTITY, DCT2X2, DCT4X4, LINES
+constexpr int kJTypes = 4;  // IDENTITY, DCT2X2, DCT4X4, LINES
 
 __host__ __device__ inline int JIndex(int type) {
   switch (type) {
-    case kDCT:
-    case kDCT_NOHF:
-      return 0;
-    case kIDENTITY:
-      return 1;
     case kDCT2X2:
-      return 2;
+      return 1;
     case kDCT4X4:
     case kDCT4X4_NOHF:
-      return 3;
+      return 2;
     case kLINES:
-      return 4;
+      return 3;
   }
-  return -1;
+  return 0;  // kIDENTITY
 }
 
 struct AdjJac {
@@ -75,12 +70,10 @@ struct AdjJac {
   float j2[9][64][64];         // DC2x2 of the LF corner, [cell][LF input]
 };
 
-// TransformToPixels of an 8x8 type (AcStrategy::TransformToPixels,
+// TransformToPixels of one of the kJTypes (AcStrategy::TransformToPixels,
 // pik/ac_strategy.cc:741-849): coefficients and pixels 8x8 row-major.
 __device__ void ToPixels8(int type, const float* co, float* px) {
-  if (type == kDCT || type == kDCT_NOHF) {
-    TsIdct1(8, co, 8, px, 8);
-  } else if (type == kDCT4X4 || type == kDCT4X4_NOHF) {
+  if (type == kDCT4X4 || type == kDCT4X4_NOHF) {
     const float b00 = co[0], b01 = co[1], b10 = co[8], b11 = co[9];
     const float d[4] = {b00 + b01 + b10 + b11, b00 + b01 - b10 - b11,
                         b00 - b01 + b10 - b11, b00 - b01 - b10 + b11};
@@ -103,11 +96,9 @@ __device__ void ToPixels8(int type, const float* co, float* px) {
   }
 }
 
-// TransformFromPixels of an 8x8 type (pik/ac_strategy.cc:531-663).
+// TransformFromPixels of one of the kJTypes (pik/ac_strategy.cc:531-663).
 __device__ void FromPixels8(int type, const float* px, float* co) {
-  if (type == kDCT || type == kDCT_NOHF) {
-    TsDct1(8, px, 8, co, 8);
-  } else if (type == kDCT4X4 || type == kDCT4X4_NOHF) {
+  if (type == kDCT4X4 || type == kDCT4X4_NOHF) {
     for (int sy = 0; sy < 2; ++sy) {
       for (int sx = 0; sx < 2; ++sx) {
         float in4[16], r4[16];
@@ -133,7 +124,7 @@ __device__ void FromPixels8(int type, const float* px, float* co) {
 // Block 2 kJTypes + 9 CTAs of 64 threads; thread j builds column j.
 __global__ void k_adj_build_jac(AdjJac* J) {
   const int which = blockIdx.x, j = threadIdx.x;
-  const int kTypes[kJTypes] = {kDCT, kIDENTITY, kDCT2X2, kDCT4X4, kLINES};
+  const int kTypes[kJTypes] = {kIDENTITY, kDCT2X2, kDCT4X4, kLINES};
   float in[64], out[64];
   for (int i = 0; i < 64; ++i) {
     in[i] = i == j ? 1.0f : 0.0f;
@@ -316,7 +307,7 @@ struct Adj8Lists {
   }
 };
 
-// Clamp backward of 8x8 blocks (all cov = 1 types) from the dense
+// Clamp backward of 8x8 blocks of the types in Adj8Lists from the dense
 // Jacobians. Blocks the EPF left unfiltered have EPF output == IDCT output,
 // a zero correction and ratio 0: the gradient passes to the IDCT output.
 __global__ void __launch_bounds__(kAdjThreads)
@@ -882,8 +873,8 @@ __global__ void __launch_bounds__(64 * kAdjBand, 4)
   }
 }
 
-// TransformToPixels transposed for 8x8 blocks; for HF-predicting types the
-// masked coefficient gradient (all but 0, 1, 8, 9) through
+// TransformToPixels transposed for the same blocks; for HF-predicting types
+// the masked coefficient gradient (all but 0, 1, 8, 9) through
 // TransformFromPixels transposed into the upsampled-prediction gradient.
 __global__ void __launch_bounds__(kAdjThreads)
     k_adj_topix8(Geo g, DevFrame f, const AdjJac* J, Adj8Lists lists,
