@@ -28,11 +28,11 @@ __device__ __forceinline__ const float* DctMat(int n) {
 }
 
 // ---------------------------------------------------------------------------
-// Single-thread transforms used by the small LF kernels (n <= 8).
+// Single-thread transforms (n <= 8) of the adjoint's matrices
+// (k_adj_build_jac).
 
 // tsIDCT (pik/dct.h:441-507): out = A C^T A^T (C row = horizontal freq).
-// Runtime size n <= 8: compact loops (these run once per block in the LF
-// kernels, where code size and registers matter more than unrolling).
+// Compact loops of a runtime size: they run once per context.
 __device__ void TsIdct1(int n, const float* in, int is, float* out, int os) {
   const float* a = IdctMat(n);
   float tmp[64];
@@ -138,11 +138,7 @@ __device__ void ReinterpDct(const float* in, int is, float* out, int os) {
 #pragma unroll
     for (int x = 0; x < N; ++x) block[y * N + x] = in[y * is + x];
   }
-  if constexpr (N <= 4) {
-    TsDctSmall<N>(block, N, res, N);
-  } else {
-    TsDct1(N, block, N, res, N);
-  }
+  TsDctSmall<N>(block, N, res, N);
   constexpr int sn = SizeIndex(N), sd = SizeIndex(DCTN);
 #pragma unroll
   for (int y = 0; y < N; ++y) {
@@ -1213,23 +1209,10 @@ __device__ void CoopTsDctT(int n, int nb, const float* bT, const float* in,
   __syncthreads();
 }
 
-// Upsampled-blurred HF prediction pixel (UpSample4x4BlurDCT,
-// pik/ac_predictions.cc:263-374) at group-local pixel (X, Y).
-__device__ __forceinline__ float Upsample(const float* pred, int X, int Y) {
-  const int r = Y >> 2, q = X >> 2, ix = X & 3, iy = Y & 3;
-  float bx[3];
-  for (int j = 0; j < 3; ++j) {
-    const float* row = pred + (r + j + 1) * kG2;
-    const float v0 = row[q + 1], v1 = row[q + 2], v2 = row[q + 3];
-    bx[j] = v0 * c_t.ub4[0][ix] + v1 * c_t.ub4[1][ix] + v2 * c_t.ub4[2][ix];
-  }
-  return bx[0] * c_t.ub4[0][iy] + bx[1] * c_t.ub4[1][iy] +
-         bx[2] * c_t.ub4[2][iy];
-}
-
-// Upsample for the N pixels X0 .. X0 + N - 1 of row Y (X0 a multiple of 4):
-// the same arithmetic as Upsample, with the 3 x (N / 4 + 2) source values
-// loaded once.
+// Upsampled-blurred HF prediction (UpSample4x4BlurDCT,
+// pik/ac_predictions.cc:263-374) at the group-local pixels X0 .. X0 + N - 1 of
+// row Y (X0 a multiple of 4), with the 3 x (N / 4 + 2) source values loaded
+// once.
 template <int N>
 __device__ __forceinline__ void UpsampleRow(const float* pred, int X0, int Y,
                                             float* out) {
