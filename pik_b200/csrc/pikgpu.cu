@@ -514,7 +514,7 @@ inline size_t NumRegions(const Geo& g) {
 
 
 // Writes the smoothed frame (gaborish #1 of the IDCT output) for the stage
-// and guide exports; the reconstruction itself never stores it.
+// export; the reconstruction itself never stores it.
 int EnsureSmoothed(pikgpu_ctx* ctx) {
   if (ctx->smoothed_valid || !ctx->s.gaborish) return PIKGPU_OK;
   const Geo& g = ctx->g;
@@ -523,7 +523,7 @@ int EnsureSmoothed(pikgpu_ctx* ctx) {
   dim3 gr(Blocks(g.PW, kTileW), Blocks(g.PH, kGabTileH), 3);
   k_gaborish_tile<<<gr, kTileThreads, 0, ctx->stream>>>(
       P<float>(ctx->idct), g.PW, g.PH, ctx->s.gaborish,
-      P<float>(ctx->smoothed), nullptr);
+      P<float>(ctx->smoothed));
   CUDA_TRY(ctx, cudaGetLastError());
   CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   ctx->smoothed_valid = true;

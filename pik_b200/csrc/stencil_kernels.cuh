@@ -1,19 +1,18 @@
-// Shared-memory tile forms of the two full-frame 3x3 stencil passes:
-//  * k_gaborish_tile: ConvolveGaborish (pik/gaborish.cc:137-159) of one
-//    plane into `out` (skipped when `out` is null: the EPF recomputes the
-//    smoothed values it needs), plus the plane's min/max (MinMax,
-//    pik/epf_target.cc:980-1006) for the EPF guide (skipped when `mm` is
-//    null);
-//  * k_gaborish_minmax: the same min/max without staging (the frame path);
+// The full-frame 3x3 stencil passes:
+//  * k_gaborish_tile: ConvolveGaborish (pik/gaborish.cc:137-159) of the
+//    planes, for the stage export (the EPF recomputes the smoothed values
+//    that it needs);
+//  * k_gaborish_minmax: the min/max of its output (MinMax,
+//    pik/epf_target.cc:980-1006), for the EPF guide, without storing it;
 //  * k_final_direct: gaborish #2 (or a copy), ShrinkTo(xsize, ysize),
 //    XybToRgb (pik/opsin_inverse.cc:38-123) and optional sRGB-8
 //    (pik/color_management.cc:323-345, pik/external_image.cc:1205).
 //
-// k_gaborish_tile stages a 128 x TH output tile with its 1-pixel halo (rows y0 - 1 ..
-// y0 + TH, columns x0 - 4 .. x0 + 131, widened to 16-byte boundaries) in
-// shared memory: interior tiles with independent 128-bit loads (many in
-// flight per thread), border tiles with mirrored scalar loads. Each thread
-// then computes 4 adjacent columns of TH / 8 rows, reading 128-bit row
+// k_gaborish_tile stages a 128 x TH output tile with its 1-pixel halo (rows
+// y0 - 1 .. y0 + TH, columns x0 - 4 .. x0 + 131, widened to 16-byte
+// boundaries) in shared memory: interior tiles with independent 128-bit loads
+// (many in flight per thread), border tiles with mirrored scalar loads. Each
+// thread then computes 4 adjacent columns of TH / 8 rows, reading 128-bit row
 // segments and taking the left/right neighbours from the adjacent lanes.
 // The arithmetic of each output is Sym3's, in the same order, so results are
 // bit-identical to it. The padded plane width must be a multiple of 4 (it is
@@ -25,7 +24,7 @@ namespace pikgpu {
 
 constexpr int kTileW = 128, kTileThreads = 256;
 constexpr int kTileSW = kTileW + 8;  // staged columns x0 - 4 .. x0 + 131
-constexpr int kGabTileH = 64;        // rows per CTA, min/max pass
+constexpr int kGabTileH = 64;        // rows per CTA
 
 // Symmetric 3x3 stencil of output column i (0..3) from three 6-value rows
 // (columns x - 1 .. x + 4), in Sym3's operation order.
@@ -103,11 +102,9 @@ __device__ __forceinline__ void TileRow6(const float (*t)[kTileSW], int r,
 }
 
 __global__ void __launch_bounds__(kTileThreads)
-    k_gaborish_tile(const float* in, int w, int h, int strength, float* out,
-                    uint32_t* mm) {
+    k_gaborish_tile(const float* in, int w, int h, int strength, float* out) {
   constexpr int TH = kGabTileH, R = TH / 8;
   __shared__ __align__(16) float t[TH + 2][kTileSW];
-  __shared__ uint32_t s_lo[kTileThreads / 32], s_hi[kTileThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.z;
   const size_t plane = size_t(w) * h;
@@ -118,7 +115,6 @@ __global__ void __launch_bounds__(kTileThreads)
   const float* wt = c_t.gaborish[strength];
   const float w0 = wt[0], w1 = wt[1], w2 = wt[2];
   const int x = x0 + 4 * lane;
-  uint32_t lo = 0xFFFFFFFFu, hi = 0u;
   float a[6], m[6], b[6];
   TileRow6(t, R * warp, lane, a);
   TileRow6(t, R * warp + 1, lane, m);
@@ -129,41 +125,14 @@ __global__ void __launch_bounds__(kTileThreads)
     if (x < w && y < h) {
       float r[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        r[i] = Sym3Rows(a, m, b, i, w0, w1, w2);
-        const uint32_t ob = OrderedBits(r[i]);
-        lo = min(lo, ob);
-        hi = max(hi, ob);
-      }
-      if (out) {
-        *reinterpret_cast<float4*>(out + c * plane + size_t(y) * w + x) =
-            make_float4(r[0], r[1], r[2], r[3]);
-      }
+      for (int i = 0; i < 4; ++i) r[i] = Sym3Rows(a, m, b, i, w0, w1, w2);
+      *reinterpret_cast<float4*>(out + c * plane + size_t(y) * w + x) =
+          make_float4(r[0], r[1], r[2], r[3]);
     }
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
       a[i] = m[i];
       m[i] = b[i];
-    }
-  }
-  if (!mm) return;
-  for (int off = 16; off; off >>= 1) {
-    lo = min(lo, __shfl_xor_sync(0xFFFFFFFFu, lo, off));
-    hi = max(hi, __shfl_xor_sync(0xFFFFFFFFu, hi, off));
-  }
-  if (lane == 0) {
-    s_lo[warp] = lo;
-    s_hi[warp] = hi;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int i = 1; i < kTileThreads / 32; ++i) {
-      lo = min(lo, s_lo[i]);
-      hi = max(hi, s_hi[i]);
-    }
-    if (lo <= hi) {
-      atomicMin(&mm[c], lo);
-      atomicMax(&mm[3 + c], hi);
     }
   }
 }
