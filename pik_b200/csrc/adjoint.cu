@@ -491,8 +491,8 @@ __device__ __forceinline__ void MatRow(const float (&v)[N], float (&o)[N]) {
 // The same for 8x8 DCT blocks, by rows in registers: a warp per channel of
 // four blocks, the element-wise step on the three channels' coefficients in
 // shared memory. With the dense Jacobians of k_adj_ar8 the 8x8 DCT blocks of
-// a 1024x1024 frame took 17 us, now 9. (16x16 blocks by the same split: 44 us
-// against 41 for k_adj_ar_sq, which has more warps per block.)
+// a 1024x1024 frame took 17 us, now 9. (16x16 blocks by the same split, at that size:
+// 44 us against 41 for k_adj_ar_sq, which has more warps per block.)
 __global__ void __launch_bounds__(kSquareArThreads)
     k_adj_ar_dct8(Geo g, DevFrame f, FrameScalars s, const uint32_t* list,
                int count, const int32_t* sigma, const uint8_t* tape,
@@ -621,8 +621,10 @@ __global__ void __launch_bounds__(kSquareArThreads)
 // as a SAD threshold, here of the sender's block: a lane's senders at one cx
 // lie in two block rows. The sums and their normaliser recomputed from the
 // guide in a pass of their own, and the offsets one by one, took 53 + 101 us
-// at 1024x1024; this takes 52, and
-// 59 with eight rows per lane, which leaves the last wave of CTAs empty.
+// at 1024x1024; this takes 53. Eight rows per lane, as the forward has, halve
+// the warps of an SM and put a lane's senders in three block rows: 60 us there,
+// 23 instead of 20 at 512x512, 139 instead of 115 at 1536x1536, 240 instead of
+// 195 at 2048x2048.
 constexpr int kAdjEpfH = 16, kAdjEpfThreads = 16 * kAdjEpfH;
 constexpr int kAdjEpfGH = kAdjEpfH + 8;   // guide rows y0 - 4 .. y0 + 19
 constexpr int kAdjEpfGPlane = kAdjEpfGH * kEpfGRow;
@@ -817,7 +819,7 @@ __global__ void __launch_bounds__(kAdjEpfThreads, 3)
 // turn: 79 us at 1024x1024, now 9).
 constexpr int kAdjBand = 4;  // pixels per CTA
 __host__ __device__ inline size_t AdjBandPixels(int w, int h) {
-  // (an 8-row frame has its two bands of rows, an 8-column one all columns)
+  // (an 8-row frame has two rows between its bands, an 8-column one a column)
   return size_t(6) * w + size_t(7) * (h - 6);
 }
 __global__ void __launch_bounds__(64 * kAdjBand, 4)

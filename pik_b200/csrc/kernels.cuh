@@ -66,11 +66,11 @@ struct PdlTail {
     asm volatile("griddepcontrol.wait;" ::: "memory");
   }
 };
-// On the main stream, kernels that read their predecessor's output (the
-// EPF reads the guide range of the min/max pass, the active-block pass the
-// EPF's sigma) may also be launched that way: they call PdlWait before the
-// first such read, and what comes before it (staging the frame's tile, say)
-// overlaps the predecessor's last CTAs.
+// On the main stream, min/max pass -> plan -> EPF are launched that way too.
+// Each calls PdlWait before it first reads its predecessor's output: the plan
+// (k_epf_plan) reads the side information before it waits for the guide's
+// range, the EPF (k_epf_box) waits first thing, since its tiles are the plan's
+// output, so that little more than its launch overlaps.
 __device__ __forceinline__ void PdlWait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }

@@ -815,7 +815,8 @@ int LaunchAll(pikgpu_ctx* ctx, float* lin, size_t lin_stride, uint8_t* rgb8,
     k_lf_tile<W><<<dim3(tiles, ng, 3), W::kThreads, W::kSmemBytes, st>>>(
         g, f, s.predict_lf, s.predict_hf);
   };
-  // The larger tiles where they fill four waves of two CTAs per SM.
+  // The larger tiles where they fill four waves of two CTAs per SM (times on
+  // both sides of the line: LfTile32).
   constexpr int kTiles32 = LfTile32::kTilesPerGroup * LfTile32::kTilesPerGroup;
   if (3 * kTiles32 * ng >= 4 * 2 * ctx->num_sms) {
     lf_tiles(LfTile32());

@@ -243,7 +243,7 @@ __global__ void k_frame_init(uint32_t* mm, int* counters, int n,
 
 __global__ void __launch_bounds__(256)
     k_minmax(const float* planes, size_t n, uint32_t* mm) {
-  PdlLaunchDependents();  // the EPF may start on free SMs
+  PdlLaunchDependents();  // the plan may start on free SMs
   __shared__ uint32_t s_lo[8], s_hi[8];
   const int c = blockIdx.y;
   const float* p = planes + size_t(c) * n;
@@ -458,7 +458,10 @@ __global__ void k_encode_pnm(const float* lin, size_t stride, int w, int h,
 // at 8192x8192), most of them the biased value's division and branches: the
 // CTA tabulates it for magnitudes below kDequantTable (it is odd in q, and
 // nearly all coefficients are small), and a thread with a larger one takes its
-// coefficients again in full. 36 -> 31 us at 4K, 260 -> 221 at 8192x8192.
+// coefficients again in full. 36 -> 31 us at 4K, 260 -> 221 at 8192x8192. With
+// 0.2% of the coefficients beyond the table, at random places, the two are
+// even (41 and 40 us at 4K, by events around the launch); with 5% or more this
+// takes 51 instead of 42.
 constexpr int kDequantCoefs = 4;
 constexpr int kDequantCells = 256 / (64 / kDequantCoefs);
 constexpr int kDequantTable = 64;  // a power of two
@@ -622,7 +625,11 @@ struct LfWin {
 // 1.9 cells per cell of its own instead of 3.1 and forms 1.3 instead of 1.7
 // times the blocks, but leaves 4K frames one and a half waves of CTAs and
 // small frames a few CTAs: 272 instead of 334 us at 8192x8192, 42.5 instead of
-// 41.3 at 3840x2160, 18 instead of 11 at 256x256.
+// 41.3 at 3840x2160, 18 instead of 11 at 256x256. By the number of 512x512
+// groups, over four transform mixes, as a share of a frame without the EPF: 1
+// to 2% slower at 25, 0 to 2% at 36, even at 40, then faster, 2 to 3% at 48, 1
+// to 3% at 63 to 100, 2 to 4% at 121 to 196. They are taken from 99 on, where
+// they fill four waves.
 using LfTile16 = LfWin<16, 256>;
 using LfTile32 = LfWin<32, 512>;
 
