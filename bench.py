@@ -961,11 +961,13 @@ def main():
     peak, peak_kind = load_peaks()
     top = max(acc, key=acc.get)
     # DRAM bytes per launch of the 4K workload measured with ncu
-    # (dram__bytes_read.sum + dram__bytes_write.sum, one cold launch each).
+    # (dram__bytes_read.sum + dram__bytes_write.sum, each launch replayed alone
+    # with cold caches; profiles/kernels_c2_4k.md). Writes that stay in the L2
+    # at a kernel's end are not in it.
     ncu_traffic_4k = {
-        "epf": 58.53e6 + 15.34e6,
-        "gaborish1_minmax": 99.54e6 + 64.64e6,
-        "gaborish2_opsin_srgb": 99.55e6 + 63.85e6,
+        "epf": 58.65e6 + 14.64e6,
+        "gaborish1_minmax": 99.56e6 + 3.99e6,
+        "gaborish2_opsin_srgb": 99.60e6 + 59.77e6,
     }
     traffic = ncu_traffic_4k.get(top) if px == 3840 * 2160 else None
     top_bytes = GROUP_BYTES.get(top, 12) * px
