@@ -962,8 +962,8 @@ def main():
     top = max(acc, key=acc.get)
     # DRAM bytes per launch of the 4K workload measured with ncu
     # (dram__bytes_read.sum + dram__bytes_write.sum, each launch replayed alone
-    # with cold caches; profiles/kernels_c2_4k.md). Writes that stay in the L2
-    # at a kernel's end are not in it.
+    # with cold caches). Writes that stay in the L2 at a kernel's end are not in
+    # it.
     ncu_traffic_4k = {
         "epf": 58.65e6 + 14.64e6,
         "gaborish1_minmax": 99.56e6 + 3.99e6,
